@@ -242,8 +242,7 @@ gem_status lane_create(gem_ctx *root, uint64_t budget, gem_ctx **out) {
   ctx->loaded = true;
   ctx->borrowed_graph = true;
   ctx->g = root->g;
-  ctx->vnh_off = root->vnh_off;
-  ctx->vnh_slots = root->vnh_slots;
+  ctx->vnh_buckets = root->vnh_buckets;
   ctx->label_freq = root->label_freq;
   ctx->label_arcs = root->label_arcs;
   ctx->label_pair_arcs = root->label_pair_arcs;
@@ -299,8 +298,7 @@ static void free_graph(gem_ctx *ctx) {
   }
   ctx->vnh_mem = nullptr;
   ctx->vnh_bytes = 0;
-  ctx->vnh_off = nullptr;
-  ctx->vnh_slots = nullptr;
+  ctx->vnh_buckets = nullptr;
   ctx->graph_mem = nullptr;
   ctx->graph_bytes = 0;
   ctx->g = DevGraph();
@@ -527,29 +525,16 @@ extern "C" gem_status gem_ctx_load_graph(gem_ctx *ctx, const gem_hgraph *hg) {
   // it is built from the mapped adjacency (one read over the host link) and
   // lives on the device like the tables the join reads.
   if (na) {
-    std::vector<uint64_t> hoff(nv + 1);
-    uint64_t n_slots = 0;
-    for (uint32_t v = 0; v < nv; ++v) {
-      hoff[v] = n_slots;
-      const uint64_t d = hg->off[v + 1] - hg->off[v];
-      if (d) {
-        uint64_t size = 2;
-        while (size < 2 * d) size <<= 1;
-        n_slots += size;
-      }
-    }
-    hoff[nv] = n_slots;
-    const uint64_t b_hoff = al(8ull * (nv + 1)), b_slots = al(4ull * n_slots);
+    // the build's scratch bits sit behind the buckets and are given back with them
+    const uint64_t b_bkt = al(sizeof(uint2) * vnh_base(na)), b_vnh = b_bkt + al(4 * vnh_moved_words(na));
     const uint64_t left = ctx->budget > ctx->device_bytes ? ctx->budget - ctx->device_bytes : 0;
     char *hp = nullptr;
-    if (b_hoff + b_slots <= left - left / 4 && cudaMalloc(&hp, b_hoff + b_slots) == cudaSuccess) {
+    if (b_vnh <= left - left / 4 && cudaMalloc(&hp, b_vnh) == cudaSuccess) {
       ctx->vnh_mem = hp;
-      ctx->vnh_bytes = b_hoff + b_slots;
+      ctx->vnh_bytes = b_vnh;
       ctx->device_bytes += ctx->vnh_bytes;
-      ctx->vnh_off = (const uint64_t *)hp;
-      ctx->vnh_slots = (const uint32_t *)(hp + b_hoff);
-      CU(cudaMemcpyAsync(hp, hoff.data(), 8ull * (nv + 1), cudaMemcpyHostToDevice, ctx->s));
-      launch_vnh_build(g, (const uint64_t *)hp, (uint32_t *)(hp + b_hoff), n_slots, ctx->s);
+      ctx->vnh_buckets = (const uint2 *)hp;
+      launch_vnh_build(g, (uint2 *)hp, (uint32_t *)(hp + b_bkt), ctx->s);
       CU(cudaGetLastError());
       CU(cudaStreamSynchronize(ctx->s));
     } else {
@@ -835,7 +820,7 @@ static uint32_t flat_code(const Plan &p, int mode) {
 // enumerated prefix of a root and one neighbour level, a closed-form suffix
 // eligible for balanced counting, and the neighbourhood hash.
 static bool pair_pool(const gem_ctx *ctx, const Plan &p, int mode) {
-  return ctx->vnh_off && mode == GEM_MODE_COUNT && p.n_enum == 2 && p.n >= 3 && flat_code(p, mode) != 0;
+  return ctx->vnh_buckets && mode == GEM_MODE_COUNT && p.n_enum == 2 && p.n >= 3 && flat_code(p, mode) != 0;
 }
 
 // A slice of the pinned staging buffer for one copy of the current wave, or
@@ -1531,8 +1516,8 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   a.lane_scan_max = tu.lane_scan_max ? tu.lane_scan_max : 48;
   a.flat_donate_blocks = tu.split_blocks ? tu.split_blocks : 32;
   a.nv = ctx->g.nv;
-  a.vnh_off = ctx->vnh_off;
-  a.vnh_slots = ctx->vnh_slots;
+  a.vnh_off = ctx->g.off;
+  a.vnh_buckets = ctx->vnh_buckets;
   a.n_values = w.table_values;
   a.n_backs = (uint32_t)jb.size();
   a.n_terms = (uint32_t)terms.size();

@@ -135,8 +135,7 @@ struct gem_ctx {
   char *graph_mem = nullptr;
   char *vnh_mem = nullptr;           // neighbourhood hash (in-core graphs that fit)
   uint64_t vnh_bytes = 0;
-  const uint64_t *vnh_off = nullptr;
-  const uint32_t *vnh_slots = nullptr;
+  const uint2 *vnh_buckets = nullptr;
   void *pinned_nbr = nullptr;        // out-of-core: mapped pinned adjacency (owned)
   void *host_nbr = nullptr;          // the same, as the host-side source of partition copies (lanes borrow it)
   // out-of-core partition streaming: vertex ranges of at most ooc_part_kib

@@ -64,41 +64,57 @@ void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s
   nlc_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.lab, g.nv, g.nlabels, nlc, stride);
 }
 
-// ---------------------------------------------------------------------------
-// Exclusive scan: 2048 items per block (256 threads x 8 consecutive items).
-// ---------------------------------------------------------------------------
-// One warp per vertex inserts its neighbours into the vertex's table.
+// One warp per vertex inserts its neighbours into the vertex's table; the
+// buckets that some neighbour had to move on from are marked in `moved`.
 __global__ void __launch_bounds__(256) vnh_build_kernel(const uint64_t *__restrict__ off,
                                                         const uint32_t *__restrict__ nbr, uint32_t nv,
-                                                        const uint64_t *__restrict__ hoff, uint32_t *slots) {
+                                                        uint32_t *slots, uint32_t *moved) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
   for (uint64_t u = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < nv; u += nw) {
-    const uint64_t b = hoff[u], size = hoff[u + 1] - b;
-    if (!size) continue;
-    const uint32_t lg = 63 - __clzll(size);
-    for (uint64_t i = off[u] + lane; i < off[u + 1]; i += 32) {
+    const uint64_t a0 = off[u], a1 = off[u + 1], b0 = vnh_base(a0);
+    const uint32_t nb = (uint32_t)(vnh_base(a1) - b0);
+    for (uint64_t i = a0 + lane; i < a1; i += 32) {
       const uint32_t v = nbr[i];
-      uint64_t pos = (v * VNH_MULT) >> (64 - lg);
-      for (uint64_t k = 0; k < size; ++k) {  // size >= 2 deg: a free slot exists
-        const uint32_t prev = atomicCAS(slots + b + pos, VNH_EMPTY, v);
+      uint32_t b = vnh_bucket(v, nb);
+      for (uint32_t k = 0; k < nb; ++k) {  // at least 2 deg slots: a free one exists
+        uint32_t *t = slots + 2 * (b0 + b);
+        uint32_t prev = atomicCAS(t, VNH_EMPTY, v);
+        if (prev != VNH_EMPTY && prev != v) prev = atomicCAS(t + 1, VNH_EMPTY, v);
         if (prev == VNH_EMPTY || prev == v) break;
-        pos = (pos + 1) & (size - 1);
+        atomicOr(moved + ((b0 + b) >> 5), 1u << ((b0 + b) & 31u));
+        if (++b == nb) b = 0;
       }
     }
   }
 }
 
-void launch_vnh_build(const DevGraph &g, const uint64_t *hoff, uint32_t *slots, uint64_t n_slots,
-                      cudaStream_t s) {
-  if (!g.nv || !n_slots) return;
-  cudaMemsetAsync(slots, 0xFF, n_slots * 4, s);
-  uint64_t blocks = ((uint64_t)g.nv + 7) / 8;
-  if (blocks > 148ull * 32) blocks = 148ull * 32;
-  count_launch();
-  vnh_build_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.nv, hoff, slots);
+// Orders every bucket's slots by whether a neighbour moved on from it.
+__global__ void __launch_bounds__(256) vnh_order_kernel(uint2 *buckets, uint64_t n, const uint32_t *__restrict__ moved) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint2 x = buckets[i];
+    const bool mv = (__ldg(moved + (i >> 5)) >> (i & 31u)) & 1u;
+    if (mv != (x.x > x.y)) buckets[i] = make_uint2(x.y, x.x);
+  }
 }
 
+void launch_vnh_build(const DevGraph &g, uint2 *buckets, uint32_t *moved, cudaStream_t s) {
+  if (!g.nv || !g.narcs) return;
+  const uint64_t n = vnh_base(g.narcs);
+  cudaMemsetAsync(buckets, 0xFF, n * sizeof(uint2), s);
+  cudaMemsetAsync(moved, 0, 4 * vnh_moved_words(g.narcs), s);
+  uint64_t blocks = ((uint64_t)g.nv + 7) / 8;
+  if (blocks > 148ull * 32) blocks = 148ull * 32;
+  count_launch(2);
+  vnh_build_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.nv, reinterpret_cast<uint32_t *>(buckets), moved);
+  blocks = (n + 255) / 256;
+  if (blocks > 148ull * 32) blocks = 148ull * 32;
+  vnh_order_kernel<<<(uint32_t)blocks, 256, 0, s>>>(buckets, n, moved);
+}
+
+// ---------------------------------------------------------------------------
+// Exclusive scan: 2048 items per block (256 threads x 8 consecutive items).
+// ---------------------------------------------------------------------------
 constexpr uint32_t SCAN_T = 256, SCAN_I = 8, SCAN_B = SCAN_T * SCAN_I;
 
 template <ScanInput K>

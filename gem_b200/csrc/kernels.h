@@ -37,16 +37,29 @@ struct DevGraph {
 void launch_degrees(const DevGraph &g, uint32_t *deg, cudaStream_t s);
 void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s);
 
-// Neighbourhood hash: per vertex u an open-addressed table of its neighbours
-// (u32, empty = VNH_EMPTY) of a power of two >= 2 deg(u) slots, at
-// [hoff[u], hoff[u+1]) of `slots`; a neighbour v starts probing at the top
-// log2(size) bits of v * VNH_MULT and moves to the next slot (mod size).
-// It answers "is (u, v) an arc" in about one load, where a binary search of
-// a hub's sorted adjacency takes a dozen dependent loads.
+// Neighbourhood hash: per vertex u a table of its neighbours (u32, empty =
+// VNH_EMPTY) in 8-byte buckets of two slots, three buckets for two arcs: u's
+// are [vnh_base(off[u]), vnh_base(off[u+1])), off the adjacency's own
+// offsets.  A neighbour goes to its bucket's first empty slot, or to the next
+// bucket (mod the table) that has one.  The order of a bucket's slots tells
+// whether a neighbour had to move on from it: first <= second, none has (an
+// empty slot counts as the largest value); first > second, some has.  So a
+// search ends at its first bucket 97% of the time (two thirds of a neighbour
+// per bucket on average: 3% of the buckets overflow), and "is (u, v) an arc"
+// is one 8-byte load, where a binary search of a hub's sorted adjacency takes
+// a dozen dependent loads.
 constexpr uint32_t VNH_EMPTY = 0xFFFFFFFFu;
-constexpr uint64_t VNH_MULT = 0x9E3779B97F4A7C15ull;
-void launch_vnh_build(const DevGraph &g, const uint64_t *hoff, uint32_t *slots, uint64_t n_slots,
-                      cudaStream_t s);
+constexpr uint32_t VNH_MULT = 0x9E3779B1u;  // 2^32 / golden ratio (multiplicative hashing)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint64_t vnh_base(uint64_t arc) { return arc + (arc >> 1); }
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t vnh_bucket(uint32_t v, uint32_t nb) { return __umulhi(v * VNH_MULT, nb); }
+#endif
+// buckets: vnh_base(narcs) of them; moved: a scratch bit per bucket.
+inline uint64_t vnh_moved_words(uint64_t narcs) { return vnh_base(narcs) / 32 + 1; }
+void launch_vnh_build(const DevGraph &g, uint2 *buckets, uint32_t *moved, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // Generic exclusive scan (u64 results, n + 1 entries: out[n] = total)
@@ -247,7 +260,7 @@ constexpr uint32_t JOIN_WARPS_PER_BLOCK = 8;
 // (one per subset of a prefix match) shared out in blocks of 8 entries.
 constexpr uint32_t FLAT_MAX_VALUES = 4;  // subset values per prefix match
 constexpr uint32_t FLAT_MAX_JOBS = 96;
-constexpr uint32_t FLAT_JOB_BYTES = 40;
+constexpr uint32_t FLAT_JOB_BYTES = 48;
 constexpr uint32_t FLAT_WARP_BYTES = FLAT_MAX_JOBS * (FLAT_JOB_BYTES + 8) + 16;
 // Ranges of the suffix lists keyed by prefix levels, per warp: 32 {lo, hi}
 // pairs and a header (the first suffix back entry).
@@ -361,8 +374,8 @@ struct JoinArgs {
   uint32_t lp2_nq;
   const uint64_t *lp2_prefix; // lp2_nq + 1 chunk-padded pair offsets (written by the prepare kernel)
   const uint32_t *vkey;       // per value of the pool queries' root tables: its key's position
-  const uint64_t *vnh_off;   // neighbourhood hash offsets (nv + 1), or null: binary search
-  const uint32_t *vnh_slots;
+  const uint64_t *vnh_off;   // the adjacency offsets: first bucket of each vertex
+  const uint2 *vnh_buckets;  // neighbourhood hash, or null: binary search
   uint64_t n_values;         // entries of `values`
   uint32_t n_backs;          // entries of `backs`
   uint32_t n_terms;          // entries of `terms`
