@@ -883,77 +883,98 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
     }
   }
   const uint32_t rows = (uint32_t)row_sig.size();
-  // descriptors: runs of up to QV rows whose neighbour labels number at most QV
-  std::vector<FilterDesc> fd;
-  for (uint32_t r = 0; r < rows;) {
-    FilterDesc d;
-    std::memset(&d, 0, sizeof d);
-    d.threshold = threshold;
-    d.row_base = r;
-    while (r < rows && d.nq < QV) {
-      const std::vector<uint32_t> &sg = row_sig[r];
-      uint32_t extra = 0;
-      for (size_t i = 2; i < sg.size(); ++i) {
-        bool seen = false;
-        for (uint32_t k = 0; k < d.nql && !seen; ++k) seen = d.ql[k] == sg[i];
-        for (size_t j = 2; j < i && !seen; ++j) seen = sg[j] == sg[i];
-        extra += seen ? 0u : 1u;
-      }
-      if (d.nq && d.nql + extra > QV) break;
-      d.lab[d.nq] = sg[0];
-      d.deg[d.nq] = sg[1];
-      for (size_t i = 2; i < sg.size(); ++i) {
-        uint32_t k = 0;
-        while (k < d.nql && d.ql[k] != sg[i]) ++k;
-        if (k == d.nql) d.ql[d.nql++] = sg[i];
-        d.nlc[d.nq][k]++;
-      }
-      ++d.nq;
-      ++r;
-    }
-    fd.push_back(d);
-  }
   w.nrows = rows;
-  FilterDesc *d_fd;
-  ST(aalloc(ctx, fd.size(), &d_fd));
-  CU(h2d(ctx, d_fd, fd.data(), fd.size() * sizeof(FilterDesc)));
+  // the label counts the rows need: the graph's own table, or (above
+  // NLC_MAX_LABELS labels) one of the wave's neighbour labels alone
+  const uint8_t *nlc = ctx->g.nlc;
+  uint32_t stride = ctx->g.nlc_stride;
+  std::vector<uint32_t> wl;
+  if (!stride) {
+    for (const auto &sg : row_sig)
+      for (size_t i = 2; i < sg.size(); ++i)
+        if (sg[i] < ctx->g.nlabels) wl.push_back(sg[i]);
+    std::sort(wl.begin(), wl.end());
+    wl.erase(std::unique(wl.begin(), wl.end()), wl.end());
+  }
+  // rows in order of their label (a warp tests rows of one label together)
+  std::vector<uint32_t> ord(rows);
+  for (uint32_t r = 0; r < rows; ++r) ord[r] = r;
+  std::stable_sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) { return row_sig[x][0] < row_sig[y][0]; });
+  std::vector<FilterRow> fr(rows);
+  std::vector<uint32_t> more;
+  for (uint32_t k = 0; k < rows; ++k) {
+    const std::vector<uint32_t> &sg = row_sig[ord[k]];
+    FilterRow &f = fr[k];
+    std::memset(&f, 0, sizeof f);
+    f.lab = sg[0];
+    f.row = ord[k];
+    if (f.lab >= ctx->g.nlabels) f.need = UINT32_MAX;  // no vertex has the label
+    f.more = (uint32_t)more.size();
+    uint32_t n = 0;
+    for (size_t i = 2, j; i < sg.size(); i = j) {  // runs of one neighbour label
+      for (j = i; j < sg.size() && sg[j] == sg[i];) ++j;
+      const uint32_t want = (uint32_t)(j - i);
+      if (sg[i] >= ctx->g.nlabels) {
+        if (f.need != UINT32_MAX) f.need += want;
+        continue;
+      }
+      const uint32_t col =
+          stride ? sg[i] : (uint32_t)(std::lower_bound(wl.begin(), wl.end(), sg[i]) - wl.begin());
+      if (n < FILTER_NEEDS) f.needs[n++] = col << 8 | want;
+      else more.push_back(col << 8 | want);
+    }
+    f.n_more = (uint32_t)more.size() - f.more;
+  }
+  if (!stride && !wl.empty()) {
+    stride = (uint32_t)((wl.size() + 15) / 16) * 16;
+    uint32_t *d_wl;
+    uint8_t *d_nlc;
+    ST(aalloc(ctx, wl.size(), &d_wl));
+    CU(h2d(ctx, d_wl, wl.data(), 4 * wl.size()));
+    ST(aalloc(ctx, (uint64_t)ctx->g.nv * stride, &d_nlc));
+    launch_nlc_labels(ctx->g, d_wl, (uint32_t)wl.size(), d_nlc, stride, ctx->s);
+    nlc = d_nlc;
+  }
+  FilterRow *d_fr;
+  uint32_t *d_more;
+  ST(aalloc(ctx, rows ? rows : 1, &d_fr));
+  CU(h2d(ctx, d_fr, fr.data(), rows * sizeof(FilterRow)));
+  ST(aalloc(ctx, more.empty() ? 1 : more.size(), &d_more));
+  CU(h2d(ctx, d_more, more.data(), 4 * more.size()));
   const uint64_t nbits = (uint64_t)rows * nwords;
+  const uint32_t ts = filter_set_tiles(rows, nwords), nsets = (nwords + ts - 1) / ts;
+  const uint64_t nsc = (uint64_t)rows * nsets;
   ST(aalloc(ctx, nbits, &w.d_rb));
+  ST(aalloc(ctx, nbits, &w.d_bits));
+  uint32_t *d_cnt;
   uint64_t *d_ex, *d_tmp, *d_rows;
-  ST(aalloc(ctx, nbits + 1, &d_ex));
-  ST(aalloc(ctx, scan_tmp_words(nbits), &d_tmp));
+  ST(aalloc(ctx, nsc, &d_cnt));
+  ST(aalloc(ctx, nsc + 1, &d_ex));
+  ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
-  launch_filter(ctx->g, d_fd, (uint32_t)fd.size(), w.d_rb, nwords, ctx->s);
-  launch_scan(w.d_rb, SCAN_POPC_U64LO, nbits, d_ex, d_tmp, ctx->s);
-  launch_gather_strided(d_ex, nwords, rows + 1, d_rows, ctx->s);
+  launch_filter(ctx->g, nlc, stride, d_fr, d_more, rows, threshold, w.d_bits, d_cnt, nwords, ctx->s);
+  launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
+  launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
   std::vector<uint64_t> rs(rows + 1);
   CU(d2h_sync(ctx, rs.data(), d_rows, 8ull * (rows + 1)));
   CU(cudaGetLastError());
   w.cnt.resize(rows);
   w.c_base.resize(rows + 1);
   for (uint32_t r = 0; r < rows; ++r) w.cnt[r] = (uint32_t)(rs[r + 1] - rs[r]);
-  for (uint32_t r = 0; r <= rows; ++r) w.c_base[r] = rs[r] - rs[0];
+  for (uint32_t r = 0; r <= rows; ++r) w.c_base[r] = rs[r];
   const uint64_t total = w.c_base[rows];
-  uint64_t *d_cbase;
-  ST(aalloc(ctx, rows + 1, &d_cbase));
-  CU(h2d(ctx, d_cbase, w.c_base.data(), 8ull * (rows + 1)));
   ST(aalloc(ctx, total ? total : 1, &w.d_cand));
-  ST(aalloc(ctx, nbits, &w.d_bits));
-  launch_compact(w.d_rb, d_ex, rows, nwords, d_cbase, w.d_cand, ctx->s, w.d_bits);
+  launch_rank_rows(w.d_bits, rows, nwords, d_ex, w.d_rb, w.d_cand, ctx->s);
   CU(cudaGetLastError());
   w.cand_total = total;
-  // algorithmic bytes, per descriptor: labels + degrees of every vertex, the
-  // label-count rows of vertices whose label occurs in its rows' neighbour
-  // labels, its bit rows (write, scan, rank rewrite); then the candidate lists.
-  uint64_t b = 0;
-  for (const FilterDesc &d : fd) {
-    uint64_t lb = 8ull * ctx->g.nv;
-    for (uint32_t k = 0; k < d.nql; ++k)
-      if (d.ql[k] < ctx->label_freq.size()) lb += (uint64_t)ctx->g.nlc_stride * ctx->label_freq[d.ql[k]];
-    lb += 8ull * nwords * d.nq * 4;
-    b += lb;
-  }
-  w.bytes_filter = b + 4 * total;
+  // algorithmic bytes: the labels of every vertex, the label counts of the
+  // vertices of every label that some row has, the rows' words (written,
+  // read and rewritten as rank words), the candidate lists
+  uint64_t b = 4ull * ctx->g.nv + 16 * nbits + 4 * total;
+  for (uint32_t k = 0; k < rows; ++k)
+    if ((k == 0 || fr[k].lab != fr[k - 1].lab) && fr[k].lab < ctx->label_freq.size())
+      b += (uint64_t)stride * ctx->label_freq[fr[k].lab];
+  w.bytes_filter = b;
   return GEM_OK;
 }
 

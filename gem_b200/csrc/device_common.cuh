@@ -73,5 +73,20 @@ __device__ __forceinline__ bool rank_member(const uint64_t *__restrict__ rb, uin
   return (uint32_t)__ldg(rb + (v >> 5)) & (1u << (v & 31u));
 }
 
+// Position of the (r + 1)-th set bit of m (r < popc(m)).
+__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t r) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t w = 16; w >= 1; w >>= 1) {
+    const uint32_t low = __popc(m & ((1u << w) - 1u));
+    if (r >= low) {
+      r -= low;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
+}
+
 }  // namespace dev
 }  // namespace gem

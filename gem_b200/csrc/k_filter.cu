@@ -4,104 +4,185 @@
 // (in-core/lib/filter/src/filter_kernel.cu:122-283) and the CPU filterSSM
 // (out-of-core/lib/filter/src/filter.cu:160-240): label equality, query degree
 // <= data degree + T, and a neighbour-label-count deficit <= T over the labels
-// that occur in the query.  Layout differences: one warp covers 32
-// consecutive data vertices (one per lane, coalesced label/degree loads), the
-// per-vertex label counts come from the table built at graph load, every
-// query of a wave is evaluated against a tile while it is in registers, and
-// each (query vertex, tile) result is one ballot word.  The compaction turns
-// the bit rows into sorted candidate lists and leaves a per-word rank in the
-// high half of each word, so the same row answers "is v in C(u)" and "where
-// is v in C(u)" with one 8-byte load.
+// that occur in the query.  The degree test follows from the deficit (a
+// query vertex's needs sum to its degree, so a deficit <= T leaves at least
+// degree - T neighbours) and is not made apart.  Each (row, 32 data vertices)
+// result is one word; the compaction turns the words into sorted candidate
+// lists and rank words, so that the same row answers "is v in C(u)" and
+// "where is v in C(u)" with one 8-byte load.
 #include "device_common.cuh"
 #include "kernels.h"
 
 namespace gem {
 
-__global__ void __launch_bounds__(256) filter_kernel(DevGraph g, const FilterDesc *__restrict__ descs,
-                                                     uint32_t nquery, uint64_t *__restrict__ rb,
-                                                     uint32_t nwords) {
-  const uint32_t lane = dev::lane_id();
-  const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t t = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); t < nwords; t += nwarps) {
-    const uint64_t v = t * 32 + lane;
-    const bool valid = v < g.nv;
-    const uint32_t l = valid ? __ldg(g.lab + v) : 0u;
-    const uint32_t d = valid ? __ldg(g.deg + v) : 0u;
-    const uint8_t *row = (g.nlc_stride && valid) ? g.nlc + v * g.nlc_stride : nullptr;
-    // this block's group of queries (blockIdx.y): small graphs have too few
-    // tiles to fill the GPU with whole waves of queries per warp
-    const uint32_t qper = (nquery + gridDim.y - 1) / gridDim.y;
-    const uint32_t q0 = blockIdx.y * qper, q1 = q0 + qper < nquery ? q0 + qper : nquery;
-    for (uint32_t qi = q0; qi < q1; ++qi) {
-      const FilterDesc *q = descs + qi;
-      const uint32_t nq = q->nq, T = q->threshold, nql = q->nql;
-      uint32_t pmask = 0;
-      if (valid)
-        for (uint32_t u = 0; u < nq; ++u)
-          if (l == q->lab[u] && q->deg[u] <= d + T) pmask |= 1u << u;
-      if (__ballot_sync(dev::FULL, pmask != 0)) {
-        if (pmask) {
-          uint32_t cnt[QV];
-          if (row) {
-            for (uint32_t k = 0; k < nql; ++k) {
-              uint32_t lk = q->ql[k];
-              cnt[k] = lk < g.nlabels ? (uint32_t)__ldg(row + lk) : 0u;
-            }
-          } else {
-            for (uint32_t k = 0; k < nql; ++k) cnt[k] = 0;
-            for (uint64_t i = g.off[v], e = g.off[v + 1]; i < e; ++i) {
-              uint32_t ln = __ldg(g.lab + __ldg(g.nbr + i));
-              for (uint32_t k = 0; k < nql; ++k)
-                if (q->ql[k] == ln) { cnt[k]++; break; }
-            }
-          }
-          uint32_t m = pmask;
-          while (m) {
-            uint32_t u = __ffs(m) - 1;
-            m &= m - 1;
-            uint32_t diff = 0;
-            for (uint32_t k = 0; k < nql; ++k) {
-              uint32_t qc = q->nlc[u][k];
-              if (qc > cnt[k]) diff += qc - cnt[k];
-            }
-            if (diff > T) pmask &= ~(1u << u);
-          }
+// One warp per (set of TS tiles of 32 vertices, group of R rows): a lane per
+// row (and per tile, 32 / R of them side by side when the wave has few rows).
+// Only a tile's vertices of the row's own label can be its candidates, a few
+// of the 32: the warp finds them with one ballot per distinct label of the
+// group (rows come sorted by label, so mostly one), and each lane tests its
+// row's needs (label, count) on those vertices alone.  The words are turned
+// in shared memory so that a row's TS words leave in one coalesced store.
+//
+// What bounds it is instruction issue, then the words written.  A lane per
+// vertex instead, every row tested on all 32 of them against a descriptor of
+// up to 32 labels (the counts copied to local memory), took 6.0 ms for
+// the 2,880 query vertices of 180 mixed-size queries on 1,048,576 vertices
+// with 32 labels; this form 0.2 ms.
+template <uint32_t TS>
+__global__ void __launch_bounds__(256) filter_kernel(const uint32_t *__restrict__ lab, uint32_t nv,
+                                                     const uint8_t *__restrict__ nlc, uint32_t stride,
+                                                     const FilterRow *__restrict__ rows,
+                                                     const uint32_t *__restrict__ more, uint32_t nrows, uint32_t R,
+                                                     uint32_t T, uint32_t nwords, uint32_t *__restrict__ bits,
+                                                     uint32_t *__restrict__ cnt) {
+  __shared__ uint32_t turn[8][32][TS + 1];
+  const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t ngroups = (nrows + R - 1) / R, nsets = (nwords + TS - 1) / TS;
+  const uint32_t rl = lane & (R - 1), sub = lane / R, nsub = 32 / R;
+  const uint64_t items = (uint64_t)ngroups * nsets;
+  for (uint64_t it = blockIdx.x * 8ull + warp; it < items; it += gridDim.x * 8ull) {
+    const uint32_t set = (uint32_t)(it / ngroups), ri = (uint32_t)(it % ngroups) * R + rl;
+    const bool have = ri < nrows;
+    FilterRow row = {};
+    if (have) row = rows[ri];
+    const bool live = have && row.need <= T;
+    // one lane per distinct label of the group
+    const uint32_t same = __match_any_sync(dev::FULL, live ? row.lab : 0xFFFFFFFFu);
+    const uint32_t leaders = __ballot_sync(dev::FULL, live && lane == (uint32_t)__ffs(same) - 1);
+    uint32_t n = 0;
+    for (uint32_t t0 = 0; t0 < TS; t0 += nsub) {
+      uint32_t m = 0;
+      for (uint32_t j = 0; j < nsub; ++j) {
+        const uint64_t v = ((uint64_t)set * TS + t0 + j) * 32 + lane;
+        const bool valid = v < nv;
+        const uint32_t l = valid ? __ldg(lab + v) : 0u;
+        for (uint32_t x = leaders; x; x &= x - 1) {
+          const uint32_t ll = __shfl_sync(dev::FULL, row.lab, __ffs(x) - 1);
+          const uint32_t b = __ballot_sync(dev::FULL, valid && l == ll);
+          if (live && sub == j && row.lab == ll) m = b;
         }
       }
+      const uint64_t vb = ((uint64_t)set * TS + t0 + sub) * 32;
       uint32_t word = 0;
-      for (uint32_t u = 0; u < nq; ++u) {
-        uint32_t b = __ballot_sync(dev::FULL, (pmask >> u) & 1u);
-        if (lane == u) word = b;
+      while (m) {  // two vertices a step: their loads overlap
+        const uint32_t b0 = __ffs(m) - 1;
+        m &= m - 1;
+        const uint32_t b1 = m ? __ffs(m) - 1 : b0;
+        m &= m - 1;
+        const uint8_t *r0 = nlc + (vb + b0) * stride, *r1 = nlc + (vb + b1) * stride;
+        uint32_t d0 = row.need, d1 = row.need;
+#pragma unroll
+        for (uint32_t i = 0; i < FILTER_NEEDS; ++i) {
+          const uint32_t k = row.needs[i] >> 8, q = row.needs[i] & 0xFFu;  // unused entries need 0
+          const uint32_t c0 = q ? __ldg(r0 + k) : 0u, c1 = q ? __ldg(r1 + k) : 0u;
+          d0 += q > c0 ? q - c0 : 0u;
+          d1 += q > c1 ? q - c1 : 0u;
+        }
+        for (uint32_t i = 0; i < row.n_more; ++i) {
+          const uint32_t e = __ldg(more + row.more + i), k = e >> 8, q = e & 0xFFu;
+          const uint32_t c0 = __ldg(r0 + k), c1 = __ldg(r1 + k);
+          d0 += q > c0 ? q - c0 : 0u;
+          d1 += q > c1 ? q - c1 : 0u;
+        }
+        word |= (d0 <= T ? 1u << b0 : 0u) | (d1 <= T ? 1u << b1 : 0u);
       }
-      if (lane < nq) rb[(uint64_t)(q->row_base + lane) * nwords + t] = (uint64_t)word;
+      n += __popc(word);
+      turn[warp][rl][t0 + sub] = word;
+    }
+    for (uint32_t o = R; o < 32; o <<= 1) n += __shfl_xor_sync(dev::FULL, n, o);
+    if (have && sub == 0) cnt[(uint64_t)row.row * nsets + set] = n;
+    __syncwarp();
+    for (uint32_t r = lane / TS; r < ((R + 32 / TS - 1) / (32 / TS)) * (32 / TS); r += 32 / TS) {
+      const uint32_t rr = __shfl_sync(dev::FULL, row.row, r & 31u);
+      const bool ok = __shfl_sync(dev::FULL, (int)have, r & 31u) && r < R;
+      const uint32_t w = set * TS + lane % TS;
+      if (ok && w < nwords) bits[(uint64_t)rr * nwords + w] = turn[warp][r][lane % TS];
+    }
+    __syncwarp();  // the words are read before the next item's are written
+  }
+}
+
+uint32_t filter_set_tiles(uint32_t nrows, uint32_t nwords) {
+  // sets of 32 tiles (128-byte stores) once they make two warps per
+  // scheduler, else sets of 8, so that a small graph's rows still spread
+  return (uint64_t)((nrows + 31) / 32) * ((nwords + 31) / 32) >= 148 * 8 ? 32u : 8u;
+}
+
+void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const FilterRow *rows,
+                   const uint32_t *more, uint32_t nrows, uint32_t threshold, uint32_t *bits, uint32_t *cnt,
+                   uint32_t nwords, cudaStream_t s) {
+  if (nwords == 0 || nrows == 0) return;
+  const uint32_t TS = filter_set_tiles(nrows, nwords);
+  uint32_t R = 1;  // rows per group: the wave's, rounded up to a power of two, at least the tiles side by side
+  while (R < 32 && (R < nrows || 32 / R > TS)) R <<= 1;
+  const uint64_t items = (uint64_t)((nrows + R - 1) / R) * ((nwords + TS - 1) / TS);
+  uint64_t blocks = (items + 7) / 8;
+  if (blocks > 148ull * 48) blocks = 148ull * 48;
+  count_launch();
+  if (TS == 32)
+    filter_kernel<32><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, nrows, R, threshold,
+                                                       nwords, bits, cnt);
+  else
+    filter_kernel<8><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, nrows, R, threshold,
+                                                      nwords, bits, cnt);
+}
+
+// One warp per 32 words of a row: their ranks into the rank words, their
+// candidates to the row's list.  ex: exclusive scan of the filter's counts
+// (all rows' sets of TS words in order), which is where a set's candidates
+// start in the lists laid back to back.
+__global__ void __launch_bounds__(256) rank_rows_kernel(const uint32_t *__restrict__ bits, uint32_t nrows,
+                                                        uint32_t nwords, const uint64_t *__restrict__ ex,
+                                                        uint32_t TS, uint64_t *__restrict__ rb,
+                                                        uint32_t *__restrict__ cand) {
+  const uint32_t lane = dev::lane_id();
+  const uint32_t G = (nwords + 31) / 32, nsets = (nwords + TS - 1) / TS;
+  const uint64_t items = (uint64_t)nrows * G;
+  for (uint64_t it = blockIdx.x * 8ull + (threadIdx.x >> 5); it < items; it += gridDim.x * 8ull) {
+    const uint32_t r = (uint32_t)(it / G), w0 = (uint32_t)(it % G) * 32, w = w0 + lane;
+    const uint64_t at = __ldg(ex + (uint64_t)r * nsets + w0 / TS), row0 = __ldg(ex + (uint64_t)r * nsets);
+    const uint64_t i = (uint64_t)r * nwords + w;
+    const uint32_t word = w < nwords ? __ldg(bits + i) : 0u, c = __popc(word);
+    uint32_t incl = c;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(dev::FULL, incl, d);
+      if (lane >= d) incl += y;
+    }
+    if (w < nwords) rb[i] = ((at - row0 + incl - c) << 32) | word;
+    const uint32_t total = __shfl_sync(dev::FULL, incl, 31);
+    for (uint32_t b = 0; b < total; b += 32) {  // a candidate per lane: the first word whose count passes it
+      const uint32_t q = b + lane;
+      uint32_t j = 0;
+#pragma unroll
+      for (uint32_t step = 16; step >= 1; step >>= 1)
+        if (__shfl_sync(dev::FULL, incl, j + step - 1) <= q) j += step;
+      const uint32_t wj = __shfl_sync(dev::FULL, word, j), before = __shfl_sync(dev::FULL, incl - c, j);
+      if (q < total) cand[at + q] = (w0 + j) * 32u + dev::nth_set_bit(wj, q - before);
     }
   }
 }
 
-void launch_filter(const DevGraph &g, const FilterDesc *d_desc, uint32_t nquery, uint64_t *rb, uint32_t nwords,
-                   cudaStream_t s) {
-  if (nwords == 0 || nquery == 0) return;
-  uint64_t blocks = (nwords + 7) / 8;
-  if (blocks > 148ull * 16) blocks = 148ull * 16;
-  // split the wave's queries over grid.y until about 148 x 48 warps run
-  uint64_t groups = (148ull * 48 + nwords - 1) / nwords;
-  if (groups > nquery) groups = nquery;
-  if (groups > 65535) groups = 65535;
-  if (groups == 0) groups = 1;
+void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint64_t *rb,
+                      uint32_t *cand, cudaStream_t s) {
+  const uint64_t items = (uint64_t)nrows * ((nwords + 31) / 32);
+  if (items == 0) return;
+  uint64_t blocks = (items + 7) / 8;
+  if (blocks > 148ull * 64) blocks = 148ull * 64;
   count_launch();
-  filter_kernel<<<dim3((uint32_t)blocks, (uint32_t)groups), 256, 0, s>>>(g, d_desc, nquery, rb, nwords);
+  rank_rows_kernel<<<(uint32_t)blocks, 256, 0, s>>>(bits, nrows, nwords, ex, filter_set_tiles(nrows, nwords), rb, cand);
 }
 
+// Compaction of bit rows kept in the low halves of rank words
+// (gem_filter_static, whose scratch is fixed).
 __global__ void compact_kernel(uint64_t *__restrict__ rb, const uint64_t *__restrict__ ex, uint32_t nrows,
-                               uint32_t nwords, const uint64_t *__restrict__ c_base, uint32_t *__restrict__ cand,
-                               uint32_t *__restrict__ bit_rows) {
+                               uint32_t nwords, const uint64_t *__restrict__ c_base, uint32_t *__restrict__ cand) {
   const uint64_t n = (uint64_t)nrows * nwords;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t r = (uint32_t)(i / nwords), w = (uint32_t)(i % nwords);
     const uint32_t bits = (uint32_t)rb[i];
     const uint64_t rank = ex[i] - ex[(uint64_t)r * nwords];
     rb[i] = (rank << 32) | bits;
-    if (bit_rows) bit_rows[i] = bits;
     uint32_t m = bits, j = 0;
     uint32_t *dst = cand + c_base[r] + rank;
     while (m) {
@@ -113,13 +194,13 @@ __global__ void compact_kernel(uint64_t *__restrict__ rb, const uint64_t *__rest
 }
 
 void launch_compact(uint64_t *rb, const uint64_t *ex, uint32_t nrows, uint32_t nwords, const uint64_t *c_base,
-                    uint32_t *cand, cudaStream_t s, uint32_t *bit_rows) {
+                    uint32_t *cand, cudaStream_t s) {
   uint64_t n = (uint64_t)nrows * nwords;
   if (n == 0) return;
   uint64_t blocks = (n + 255) / 256;
   if (blocks > 148ull * 32) blocks = 148ull * 32;
   count_launch();
-  compact_kernel<<<(uint32_t)blocks, 256, 0, s>>>(rb, ex, nrows, nwords, c_base, cand, bit_rows);
+  compact_kernel<<<(uint32_t)blocks, 256, 0, s>>>(rb, ex, nrows, nwords, c_base, cand);
 }
 
 }  // namespace gem

@@ -64,6 +64,53 @@ void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s
   nlc_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.lab, g.nv, g.nlabels, nlc, stride);
 }
 
+// As nlc_kernel for n chosen labels, found by binary search (at most
+// NLC_MAX_LABELS of them per launch, columns c0 .. c0 + n - 1).
+__global__ void __launch_bounds__(256) nlc_labels_kernel(const uint64_t *__restrict__ off,
+                                                         const uint32_t *__restrict__ nbr,
+                                                         const uint32_t *__restrict__ lab, uint32_t nv,
+                                                         const uint32_t *__restrict__ labels, uint32_t n,
+                                                         uint8_t *__restrict__ nlc, uint32_t stride) {
+  __shared__ uint32_t hist[8][NLC_MAX_LABELS];
+  __shared__ uint32_t want[NLC_MAX_LABELS];
+  const uint32_t lane = dev::lane_id(), w = threadIdx.x >> 5;
+  if (threadIdx.x < n) want[threadIdx.x] = labels[threadIdx.x];
+  __syncthreads();
+  const uint64_t nwarps = (uint64_t)gridDim.x * 8;
+  for (uint64_t v = blockIdx.x * 8ull + w; v < nv; v += nwarps) {
+    for (uint32_t l = lane; l < n; l += 32) hist[w][l] = 0;
+    __syncwarp();
+    for (uint64_t i = off[v] + lane, e = off[v + 1]; i < e; i += 32) {
+      const uint32_t l = __ldg(lab + __ldg(nbr + i));
+      uint32_t lo = 0, hi = n;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (want[mid] < l) lo = mid + 1; else hi = mid;
+      }
+      if (lo < n && want[lo] == l) atomicAdd(&hist[w][lo], 1u);
+    }
+    __syncwarp();
+    for (uint32_t l = lane; l < n; l += 32) {
+      const uint32_t c = hist[w][l];
+      nlc[v * stride + l] = (uint8_t)(c > 255u ? 255u : c);
+    }
+    __syncwarp();
+  }
+}
+
+void launch_nlc_labels(const DevGraph &g, const uint32_t *labels, uint32_t n, uint8_t *nlc, uint32_t stride,
+                       cudaStream_t s) {
+  if (g.nv == 0) return;
+  uint64_t blocks = ((uint64_t)g.nv + 7) / 8;
+  if (blocks > 148ull * 64) blocks = 148ull * 64;
+  for (uint32_t c = 0; c < n; c += NLC_MAX_LABELS) {
+    count_launch();
+    nlc_labels_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.lab, g.nv, labels + c,
+                                                       n - c < NLC_MAX_LABELS ? n - c : NLC_MAX_LABELS, nlc + c,
+                                                       stride);
+  }
+}
+
 // One warp per vertex inserts its neighbours into the vertex's table; the
 // buckets that some neighbour had to move on from are marked in `moved`.
 __global__ void __launch_bounds__(256) vnh_build_kernel(const uint64_t *__restrict__ off,
@@ -263,6 +310,50 @@ __global__ void __launch_bounds__(SCAN_T) scan_final_kernel(const void *in, uint
   }
 }
 
+// Short inputs in one block and one launch: a plain query's scans are a few
+// thousand items, where three launches cost more than the work (SCAN_SMALL
+// items take two steps of the block).
+constexpr uint64_t SCAN_SMALL = 16384;
+
+template <ScanInput K>
+__global__ void __launch_bounds__(1024) scan_small_kernel(const void *in, uint64_t n, uint64_t *out) {
+  __shared__ uint64_t wsum[2][32];
+  const uint32_t lane = dev::lane_id(), w = threadIdx.x >> 5;
+  uint64_t carry = 0;
+  uint32_t step = 0;
+  for (uint64_t b0 = 0; b0 < n; b0 += 1024 * SCAN_I, step ^= 1u) {
+    const uint64_t base = b0 + (uint64_t)threadIdx.x * SCAN_I;
+    uint32_t v[SCAN_I];
+    scan_items<K>(in, n, base, v);
+    uint64_t x = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < SCAN_I; ++j) x += v[j];
+    uint64_t inc = x;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t y = __shfl_up_sync(dev::FULL, inc, d);
+      if (lane >= (uint32_t)d) inc += y;
+    }
+    if (lane == 31) wsum[step][w] = inc;
+    __syncthreads();
+    // every warp scans the 32 warp sums for itself (two buffers: one barrier a step)
+    uint64_t s = wsum[step][lane], si = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t y = __shfl_up_sync(dev::FULL, si, d);
+      if (lane >= (uint32_t)d) si += y;
+    }
+    uint64_t ex = carry + __shfl_sync(dev::FULL, si - s, w) + inc - x;
+    carry += __shfl_sync(dev::FULL, si, 31);
+#pragma unroll
+    for (uint32_t j = 0; j < SCAN_I; ++j) {
+      if (base + j < n) out[base + j] = ex;
+      ex += v[j];
+    }
+  }
+  if (threadIdx.x == 0) out[n] = carry;
+}
+
 __global__ void gather_strided_kernel(const uint64_t *__restrict__ in, uint64_t stride, uint32_t n,
                                       uint64_t *__restrict__ out) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = in[i * stride];
@@ -285,6 +376,19 @@ void launch_set_deadline(unsigned long long *deadline, uint64_t cap_ns, cudaStre
 
 uint64_t scan_tmp_words(uint64_t n) { return (n + SCAN_B - 1) / SCAN_B + 2; }
 
+template <ScanInput K>
+static void scan_kind(const void *in, uint64_t n, uint64_t nb, uint64_t *out, uint64_t *tmp, cudaStream_t s) {
+  if (n <= SCAN_SMALL) {
+    count_launch();
+    scan_small_kernel<K><<<1, 1024, 0, s>>>(in, n, out);
+    return;
+  }
+  count_launch(3);
+  scan_partial_kernel<K><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp);
+  scan_top_kernel<<<1, 1024, 0, s>>>(tmp, nb, out, n);
+  scan_final_kernel<K><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp, out);
+}
+
 void launch_scan(const void *in, ScanInput kind, uint64_t n, uint64_t *out, uint64_t *tmp, cudaStream_t s) {
   const uint64_t nb = (n + SCAN_B - 1) / SCAN_B;
   if (n == 0) {
@@ -292,30 +396,9 @@ void launch_scan(const void *in, ScanInput kind, uint64_t n, uint64_t *out, uint
     return;
   }
   switch (kind) {
-    case SCAN_POPC_U64LO:
-      count_launch();
-      scan_partial_kernel<SCAN_POPC_U64LO><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp);
-      count_launch();
-      scan_top_kernel<<<1, 1024, 0, s>>>(tmp, nb, out, n);
-      count_launch();
-      scan_final_kernel<SCAN_POPC_U64LO><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp, out);
-      break;
-    case SCAN_POPC_U32:
-      count_launch();
-      scan_partial_kernel<SCAN_POPC_U32><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp);
-      count_launch();
-      scan_top_kernel<<<1, 1024, 0, s>>>(tmp, nb, out, n);
-      count_launch();
-      scan_final_kernel<SCAN_POPC_U32><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp, out);
-      break;
-    default:
-      count_launch();
-      scan_partial_kernel<SCAN_U32><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp);
-      count_launch();
-      scan_top_kernel<<<1, 1024, 0, s>>>(tmp, nb, out, n);
-      count_launch();
-      scan_final_kernel<SCAN_U32><<<(uint32_t)nb, SCAN_T, 0, s>>>(in, n, tmp, out);
-      break;
+    case SCAN_POPC_U64LO: scan_kind<SCAN_POPC_U64LO>(in, n, nb, out, tmp, s); break;
+    case SCAN_POPC_U32: scan_kind<SCAN_POPC_U32>(in, n, nb, out, tmp, s); break;
+    default: scan_kind<SCAN_U32>(in, n, nb, out, tmp, s); break;
   }
 }
 

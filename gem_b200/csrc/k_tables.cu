@@ -153,21 +153,6 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Position of the (r + 1)-th set bit of m (r < popc(m)).
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t r) {
-  uint32_t pos = 0;
-#pragma unroll
-  for (uint32_t w = 16; w >= 1; w >>= 1) {
-    const uint32_t low = __popc(m & ((1u << w) - 1u));
-    if (r >= low) {
-      r -= low;
-      m >>= w;
-      pos += w;
-    }
-  }
-  return pos;
-}
-
 // The table passes over vertex tiles.  One warp per tile (32 arcs of one
 // vertex v): the arcs are read once for every source whose candidates hold
 // v.  Those sources are the set bits of v's source column; the warp takes
@@ -270,7 +255,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
         uint32_t k = 0, e0 = 0, ne = 0;
         uint64_t lt = 0;
         if (q < total) {
-          const VSrc &src = P.vsrc[(wb + j) * 32u + nth_set_bit(wj, q - exj)];
+          const VSrc &src = P.vsrc[(wb + j) * 32u + dev::nth_set_bit(wj, q - exj)];
           const uint64_t rw = __ldg(src.rb + (v >> 5));
           k = (uint32_t)(rw >> 32) + __popc((uint32_t)rw & ((1u << (v & 31u)) - 1u));
           lt = __ldg(P.tp + src.key_base + k) - src.stb + c;

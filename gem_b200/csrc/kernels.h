@@ -36,6 +36,10 @@ struct DevGraph {
 // Per-graph derived data, built once at load time.
 void launch_degrees(const DevGraph &g, uint32_t *deg, cudaStream_t s);
 void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s);
+// Neighbour counts of `n` chosen labels (sorted ascending), stride bytes per
+// vertex: what a wave needs on a graph of more than NLC_MAX_LABELS labels.
+void launch_nlc_labels(const DevGraph &g, const uint32_t *labels, uint32_t n, uint8_t *nlc, uint32_t stride,
+                       cudaStream_t s);
 
 // Neighbourhood hash: per vertex u a table of its neighbours (u32, empty =
 // VNH_EMPTY) in 8-byte buckets of two slots, three buckets for two arcs: u's
@@ -81,28 +85,46 @@ void launch_scan(const void *in, ScanInput kind, uint64_t n, uint64_t *out, uint
 // ---------------------------------------------------------------------------
 // Filter
 // ---------------------------------------------------------------------------
-struct FilterDesc {          // one query of a wave
+struct FilterDesc {          // one query (gem_filter_static)
   uint32_t nq;               // query vertices
   uint32_t nql;              // distinct labels in the query
   uint32_t threshold;
-  uint32_t row_base;         // first rank-bitmap row of this query
+  uint32_t row_base;
   uint32_t ql[QV];           // distinct labels
   uint32_t lab[QV];          // label of each query vertex
   uint32_t deg[QV];          // query degree of each vertex
   uint8_t nlc[QV][QV];       // nlc[u][k]: neighbours of u with label ql[k]
 };
 
-// Writes the candidate bit of every (query vertex, data vertex) pair into the
-// low halves of rb (rows of nwords u64, row = row_base + u).
-void launch_filter(const DevGraph &g, const FilterDesc *d_desc, uint32_t nquery, uint64_t *rb,
+// A row of a wave's filter: candidates have label `lab` and, over the needs
+// (label-count column << 8 | neighbours wanted, 0 = unused), a deficit of at
+// most the threshold; `need` is the deficit that no vertex can make up
+// (neighbour labels that the graph lacks; above the threshold: no candidates).
+constexpr uint32_t FILTER_NEEDS = 4;
+struct FilterRow {
+  uint32_t lab;
+  uint32_t row;              // row index of the outputs
+  uint32_t need;
+  uint32_t more, n_more;     // the needs after the first FILTER_NEEDS, in the wave's list of them
+  uint32_t needs[FILTER_NEEDS];
+};
+// Vertex tiles per filter item (the granularity of its counts).
+uint32_t filter_set_tiles(uint32_t nrows, uint32_t nwords);
+// Candidate words of every row, bits[row * nwords + word], and the
+// candidates of every set of filter_set_tiles words, cnt[row * sets + set].
+// rows sorted by label; nlc: label counts of every vertex, stride bytes each.
+void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const FilterRow *rows,
+                   const uint32_t *more, uint32_t nrows, uint32_t threshold, uint32_t *bits, uint32_t *cnt,
                    uint32_t nwords, cudaStream_t s);
+// Rank words (members before the word << 32 | the word) and the sorted
+// candidate lists back to back, given ex = exclusive scan of cnt.
+void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint64_t *rb,
+                      uint32_t *cand, cudaStream_t s);
 // Given ex = exclusive scan of popcounts over all rows, writes the per-word
 // ranks into the high halves of rb and the sorted candidate lists
 // cand[c_base[row] ...].
-// bit_rows (optional, nrows x nwords u32): the membership bits alone, half
-// the bytes of rb for tests that need no rank.
 void launch_compact(uint64_t *rb, const uint64_t *ex, uint32_t nrows, uint32_t nwords,
-                    const uint64_t *c_base, uint32_t *cand, cudaStream_t s, uint32_t *bit_rows = nullptr);
+                    const uint64_t *c_base, uint32_t *cand, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // Edge-candidate tables
