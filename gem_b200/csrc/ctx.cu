@@ -1268,15 +1268,25 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // single query whose tables do not fit the device budget keeps them in
   // mapped pinned host memory, which the write pass and the join reach over
   // the host link; a batch wave that does not fit is split instead.
+  // Key positions that only spread the ordinary pool's items (pair 2) are left
+  // out when they do not fit.
   w.d_vkey = nullptr;
   const uint64_t nv_alloc = nvals ? nvals : 1;
+  const bool map_needed = key_map && std::find(w.pair.begin(), w.pair.end(), PAIR_POOL) != w.pair.end();
   gem_status vst = aalloc(ctx, nv_alloc, &w.d_values);
-  if (vst == GEM_OK && key_map) vst = aalloc(ctx, nv_alloc, &w.d_vkey);
+  if (vst == GEM_OK && key_map) {
+    vst = aalloc(ctx, nv_alloc, &w.d_vkey);
+    if (vst == GEM_ERR_OOM && !map_needed) {
+      ctx->err.clear();
+      w.d_vkey = nullptr;
+      vst = GEM_OK;
+    }
+  }
   if (vst == GEM_ERR_OOM && ctx->opts.ooc && w.q.size() == 1) {
-    const uint64_t need = 4 * nv_alloc * (key_map ? 2 : 1);
+    const uint64_t need = 4 * nv_alloc * (map_needed ? 2 : 1);
     ST(spill_buffer(ctx, need));
     w.d_values = static_cast<uint32_t *>(ctx->spill_dev);
-    w.d_vkey = key_map ? w.d_values + nv_alloc : nullptr;
+    w.d_vkey = map_needed ? w.d_values + nv_alloc : nullptr;
     ctx->err.clear();
     ctx->ooc.waves_spilled += 1;
     ctx->ooc.bytes_spilled += need;
@@ -1299,7 +1309,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // value its id (and key position); the offsets; per key its tile count
   // and scan.
   w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * WS) + vtiles * 32ull * 4 * WT + 2 * src_tiles * 16 +
-                   tiles * (4 + 4 + 8) + nvals * (key_map ? 8 : 4) + offs * 8 + nkeys * (4 + 8 + 4);
+                   tiles * (4 + 4 + 8) + nvals * (w.d_vkey ? 8 : 4) + offs * 8 + nkeys * (4 + 8 + 4);
   return GEM_OK;
 }
 
@@ -1395,6 +1405,7 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   std::vector<uint64_t> rp, terms, lpp;
   std::vector<uint32_t> lpq, lp2q;
   uint64_t lp_roots = 0;
+  bool pair_items = false;
   w.jq_index.assign(w.q.size(), UINT32_MAX);
   uint64_t roots = 0;
   // Queries take the grid's warps in order of estimated work, cheapest
@@ -1459,14 +1470,19 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
       lp_roots += J.n_root;
       J.root_base = roots;
       rp.push_back(roots);
-    } else if (w.pair[qi] && w.d_vkey) {
+    } else if (w.pair[qi] == PAIR_POOL && w.d_vkey) {
       // (root, first level) pair pool; an empty range in the ordinary pool
       lp2q.push_back((uint32_t)jq.size());
       J.root_base = roots;
       rp.push_back(roots);
     } else {
+      // items of the ordinary pool: the entries of the root table (every
+      // root with each of its first-level vertices), so that a hub's many
+      // subtrees start on as many warps; else the roots
+      J.pairs = w.pair[qi] == PAIR_ITEMS && w.d_vkey;
+      pair_items |= J.pairs != 0;
       rp.push_back(roots);
-      roots += J.n_root;
+      roots += J.pairs ? w.edge_vals[w.edge_of[qi][1]] : J.n_root;
     }
     jq.push_back(J);
   }
@@ -1533,7 +1549,9 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   a.donate_max_level = tu.donate_max_level ? tu.donate_max_level : ctx->donate_max_level;
   a.donate_min_lane = tu.donate_min_lane ? tu.donate_min_lane : 32;
   a.donate_min_desc = tu.donate_min_desc ? tu.donate_min_desc : 1;
-  a.root_batch_max = tu.root_batch_max ? tu.root_batch_max : 1;
+  // pairs are ten to a hundred times as many as roots: a warp may take 32, one
+  // per lane to look up (fewer once a quarter of an even share is less)
+  a.root_batch_max = std::min(32u, tu.root_batch_max ? tu.root_batch_max : pair_items ? 32u : 1u);
   a.lane_scan_max = tu.lane_scan_max ? tu.lane_scan_max : 48;
   a.flat_donate_blocks = tu.split_blocks ? tu.split_blocks : 32;
   a.nv = ctx->g.nv;
@@ -1648,7 +1666,12 @@ gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_
     }
   }
   w.pair.assign(nq, 0);
-  for (size_t qi = 0; qi < nq; ++qi) w.pair[qi] = w.active[qi] && pair_pool(ctx, w.plan[qi], mode);
+  for (size_t qi = 0; qi < nq; ++qi)
+    if (w.active[qi])
+      // (out of core the key positions' memory is better left to the values)
+      w.pair[qi] = pair_pool(ctx, w.plan[qi], mode)                    ? PAIR_POOL
+                   : w.plan[qi].n_enum >= 3 && !ctx->opts.ooc ? PAIR_ITEMS
+                                                                       : 0;
   w.plan_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
   ST(wave_tables(ctx, w));
   ST(phase_sync("edge tables"));

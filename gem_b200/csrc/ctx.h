@@ -58,6 +58,8 @@ struct Plan {
 // count_suffix: choose a closed-form suffix (count mode only).
 void make_plan(const gem::HostQuery &q, const uint32_t *cnt, bool count_suffix, Plan &p);
 
+constexpr uint8_t PAIR_POOL = 1, PAIR_ITEMS = 2;
+
 // One wave: a set of queries processed by shared launches.
 struct Wave {
   std::vector<gem::HostQuery> q;
@@ -74,7 +76,8 @@ struct Wave {
   std::vector<std::vector<uint32_t>> idx_kind;  // per query, per level
   std::vector<std::vector<const gem::CuckooTable *>> ck_of;
   std::vector<std::vector<uint32_t>> edge_of;   // per query: [j*QV+k] -> edge index
-  std::vector<uint8_t> pair;        // query counted through the (root, first level) pair pool
+  std::vector<uint8_t> pair;        // PAIR_POOL: counted through the (root, first level) pair pool;
+                                    // PAIR_ITEMS: its items of the ordinary pool are such pairs
   uint32_t *d_vkey = nullptr;       // key positions of the pool queries' root-table values
   uint32_t nrows = 0, nwords = 0, nsrc = 0;
   uint64_t *d_rb = nullptr;       // rank bitmaps, nrows x nwords

@@ -1338,6 +1338,35 @@ __device__ void abandon(const JoinArgs &a, uint32_t q) {
     for (uint32_t k = find_query(a.root_prefix, a.nquery, r0); k < a.nquery; ++k) atomicOr(&a.out[k].pad[0], 1ull);
 }
 
+// Item r of the ordinary pool: a root of its query, or (JQuery::pairs) an
+// entry of the query's root table, which is a root and a first-level vertex.
+// k0 = 0xFFFFFFFF: a bounds check failed.
+template <uint32_t MODE>
+__device__ __forceinline__ void root_item(const JoinArgs &a, uint64_t r, uint32_t &q, uint32_t &f0, uint32_t &k0,
+                                          uint32_t &f1, uint32_t &k1) {
+  q = find_query(a.root_prefix, a.nquery, r);
+  const JQuery *Q = a.queries + q;
+  const uint64_t rl = r - Q->root_base;
+  f0 = f1 = k1 = 0;
+  k0 = 0xFFFFFFFFu;
+  if (!Q->pairs) {
+    if (!inb(a, SITE_ROOT, rl, Q->n_root)) return;
+    k0 = (uint32_t)rl;
+    f0 = __ldg(Q->root_cand + k0);
+    return;
+  }
+  const JLevel *L1 = &Q->lv[1];
+  if (!inb(a, SITE_BACK, L1->back_base, a.n_backs)) return;
+  const uint64_t p = __ldg(a.backs[L1->back_base].off) + rl;
+  if (!inb(a, SITE_RANGE, p, a.n_values)) return;
+  const uint32_t kr = __ldg(a.vkey + p);
+  if (!inb(a, SITE_ROOT, kr, Q->n_root)) return;
+  f1 = __ldg(a.values + p);
+  f0 = __ldg(Q->root_cand + kr);
+  k1 = index_of(a, L1, f1);
+  k0 = kr;
+}
+
 template <uint32_t MODE>
 __device__ __forceinline__ void emit_last(const JoinArgs &a, const JQuery *__restrict__ Q, uint32_t lvl, uint32_t m,
                                           uint32_t w, const LaneState &c, uint64_t &lane_cnt, uint64_t &lane_hash) {
@@ -1601,14 +1630,18 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
     }
   }
 
+  // Lane i's item of the batch held (rb_first + i): its query, and the matched
+  // vertices and positions of its prefix (a root, or a root and a first level).
+  uint64_t rb_first = 0;
+  uint32_t iq = 0, if0 = 0, ik0 = 0, if1 = 0, ik1 = 0;
+  uint32_t iter = 0;  // chunks evaluated: the time cap is looked at every fourth
   for (;;) {
     // ------------------------------------------------------------ acquire
     uint32_t q = 0, base_lvl = 0, lvl = 0;
     bool have = false, from_root = false;
-    uint64_t r = 0;
     if (!idle_registered) {
       if (rb_cur >= rb_end) {
-        // guided batches: a quarter of the remaining roots per warp, 1..16
+        // guided batches: a quarter of the remaining items per warp, 1..root_batch_max
         unsigned long long rr = 0, cnt = 1;
         if (lane == 0) {
           const unsigned long long seen = ld_vol(&ctl->root_next);
@@ -1623,27 +1656,26 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
         rb_cur = __shfl_sync(FULL, rr, 0);
         cnt = __shfl_sync(FULL, cnt, 0);
         rb_end = rb_cur < a.n_roots ? (rb_cur + cnt < a.n_roots ? rb_cur + cnt : a.n_roots) : rb_cur;
-      }
-      r = rb_cur < rb_end ? rb_cur++ : a.n_roots;
-      // warp-uniform: lane 0 reads the error word for the whole warp
-      const int err_set = __shfl_sync(FULL, lane == 0 ? (int)(ld_vol(&ctl->err) != DERR_NONE) : 0, 0);
-      if (r < a.n_roots && err_set) {
-        // past the deadline: this root and the rest of the batch are not processed
-        if (lane == 0) {
-          const uint32_t q0 = find_query(a.root_prefix, a.nquery, r);
-          const uint32_t q1 = find_query(a.root_prefix, a.nquery, rb_end - 1);
-          for (uint32_t k = q0; k <= q1; ++k) atomicOr(&a.out[k].pad[0], 1ull);
-          abandon(a, q0);
-          if (pushed) __threadfence();
-          atomicSub(&ctl->busy, 1u);
+        rb_first = rb_cur;
+        if (rb_cur < rb_end && err_set(a)) {
+          // past the deadline: the batch is not processed
+          if (lane == 0) {
+            const uint32_t q0 = find_query(a.root_prefix, a.nquery, rb_cur);
+            const uint32_t q1 = find_query(a.root_prefix, a.nquery, rb_end - 1);
+            for (uint32_t k = q0; k <= q1; ++k) atomicOr(&a.out[k].pad[0], 1ull);
+            abandon(a, q0);
+            if (pushed) __threadfence();
+            atomicSub(&ctl->busy, 1u);
+          }
+          pushed = false;
+          rb_cur = rb_end;
         }
-        pushed = false;
-        rb_cur = rb_end;
-        r = a.n_roots;
+        if (rb_cur + lane < rb_end) root_item<MODE>(a, rb_cur + lane, iq, if0, ik0, if1, ik1);
       }
-      if (r < a.n_roots) {
+      if (rb_cur < rb_end) {
         have = true;
         from_root = true;
+        q = __shfl_sync(FULL, iq, (uint32_t)(rb_cur - rb_first));
       } else {
         idle_registered = true;
         if (lane == 0) atomicAdd(&ctl->idle, 1u);
@@ -1707,44 +1739,50 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
       }
     }
 
-    // ------------------------------------------------------------ set up
     ++epoch;
     uint64_t lane_cnt = 0, lane_hash = 0;
     const JQuery *__restrict__ Q = a.queries + q;
+    const uint32_t n = Q->n;
+    bool abort = false;
+    for (;;) {  // the items of the batch that belong to q, or one donated task
+    // ------------------------------------------------------------ set up
     if (from_root) {
-      q = find_query(a.root_prefix, a.nquery, r);
-      Q = a.queries + q;
-      const uint64_t rl = r - Q->root_base;
+      const uint32_t il = (uint32_t)(rb_cur++ - rb_first);
+      const uint32_t f0 = __shfl_sync(FULL, if0, il), k0 = __shfl_sync(FULL, ik0, il);
+      const uint32_t f1 = __shfl_sync(FULL, if1, il), k1 = __shfl_sync(FULL, ik1, il);
       lvl = 0;
       base_lvl = 1;
-      if (inb(a, SITE_ROOT, rl, Q->n_root)) {
-        const uint32_t w0 = __ldg(Q->root_cand + rl);
-        const uint64_t h0 = MODE == MODE_COUNT ? 0ull : emb_term(Q->root_u, w0);
+      ++epoch;
+      if (k0 != 0xFFFFFFFFu) {  // not a failed bounds check
+        const uint64_t h0 = MODE == MODE_COUNT ? 0ull : emb_term(Q->root_u, f0);
         if (lane == 0) {
-          c.f = w0;
-          c.idx = (uint32_t)rl;
+          c.f = f0;
+          c.idx = k0;
           c.hs = h0;
         }
+        if (Q->pairs && lane == 1) {
+          c.f = f1;
+          c.idx = k1;
+          if (MODE != MODE_COUNT) c.hs = h0 + emb_term(Q->lv[1].u, f1);
+        }
         st.nodes += lane == 0;
-        if (Q->n >= 2) {
+        const uint32_t first = Q->pairs ? 2u : 1u;
+        if (n > first) {
           uint32_t nb, src;
           uint64_t lo, hi, s_lo, s_hi;
-          level_lists(a, &Q->lv[1], c, nb, lo, hi, src, s_lo, s_hi);
-          if (lane == 1) {
+          level_lists(a, &Q->lv[first], c, nb, lo, hi, src, s_lo, s_hi);
+          if (lane == first) {
             c.src = src;
             c.pos = s_lo;
             c.end = s_hi;
             c.mask = 0;
           }
-          lvl = base_lvl = 1;
+          lvl = base_lvl = first;
         }
       }
     }
 
     // ------------------------------------------------------------ DFS
-    const uint32_t n = Q->n;
-    uint32_t iter = 0;
-    bool abort = false;
     while (lvl >= base_lvl && lvl != 0) {
       const JLevel *__restrict__ L = &Q->lv[lvl & 31u];
       const uint32_t mask = __shfl_sync(FULL, c.mask, lvl);
@@ -1949,6 +1987,8 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
         c.mask = 0;
       }
       lvl = nxt;
+    }
+    if (abort || !from_root || rb_cur >= rb_end || __shfl_sync(FULL, iq, (uint32_t)(rb_cur - rb_first)) != q) break;
     }
 
     // ------------------------------------------------------------ retire

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
             // the value position.  A key's tiles are consecutive in its
             // source's tile order, so the unit's masks and positions are
             // consecutive words.
-            const uint32_t kf = have && (E.flags & TAB_KEY_MAP) ? pk : 0xFFFFFFFFu;
+            const uint32_t kf = have && P.vkey && (E.flags & TAB_KEY_MAP) ? pk : 0xFFFFFFFFu;
             const uint32_t below = (1u << lane) - 1u;
             uint32_t m[G];
             uint64_t vb[G];

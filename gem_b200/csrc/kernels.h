@@ -307,6 +307,8 @@ struct JQuery {
   uint32_t n_groups;         // label groups of the suffix
   uint32_t flat;             // balanced lane-level counting: subset values per prefix match
                              // (bits 0-7; 0 = not eligible) and those needing a scan (bits 8-15)
+  uint32_t pairs;            // items of the ordinary pool: (root, first level) pairs instead of roots
+  uint32_t pad;
   uint32_t grp_first[MAX_GROUPS];
   uint32_t grp_size[MAX_GROUPS];
   uint32_t term_base[MAX_GROUPS];
