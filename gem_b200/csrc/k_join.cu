@@ -278,17 +278,23 @@ __device__ __forceinline__ uint32_t index_of(const JoinArgs &a, const JLevel *__
 // of chains of dependent L2 loads.  A slot is tagged by the list's absolute
 // range in the values array, which identifies the list for the whole launch.
 // ---------------------------------------------------------------------------
-struct ListCache {
+template <bool CACHED>
+struct ListCacheT {
   uint32_t *buf;            // LIST_CACHE_SLOTS * LIST_CACHE_CAP entries
   unsigned long long *tag;  // {lo, hi} per slot
   unsigned long long *rng;  // {lo, hi} of suffix back entries b0 + i (lo ~0: not keyed by the prefix); rng[64] = b0
 };
 
-__device__ __forceinline__ int cache_slot(const ListCache &lc, uint64_t lo, uint64_t hi) {
-  if (hi <= lo) return -1;
+// CACHED = false: the counters of the lane-parallel pools, whose prefixes are
+// the lanes' own, so that nothing is shared and nothing is cached.
+using ListCache = ListCacheT<true>;
+
+template <bool C>
+__device__ __forceinline__ int cache_slot(const ListCacheT<C> &lc, uint64_t lo, uint64_t hi) {
+  if (C && hi > lo)
 #pragma unroll
-  for (int k = 0; k < (int)LIST_CACHE_SLOTS; ++k)
-    if (lc.tag[2 * k] == lo && lc.tag[2 * k + 1] == hi) return k;
+    for (int k = 0; k < (int)LIST_CACHE_SLOTS; ++k)
+      if (lc.tag[2 * k] == lo && lc.tag[2 * k + 1] == hi) return k;
   return -1;
 }
 
@@ -330,7 +336,8 @@ __device__ __forceinline__ uint32_t smem_member8(const uint32_t *b, uint32_t n, 
 // x in list [lo, hi): from the cache slot when there is one, else by binary
 // search of the values array from *cur (lists are probed in ascending x, so
 // the search start only moves forward).
-__device__ __forceinline__ bool list_member(const JoinArgs &a, const ListCache &lc, int slot, uint64_t lo,
+template <bool C>
+__device__ __forceinline__ bool list_member(const JoinArgs &a, const ListCacheT<C> &lc, int slot, uint64_t lo,
                                             uint64_t hi, uint64_t &cur, uint32_t x) {
   if (slot >= 0) return smem_contains(lc.buf + slot * LIST_CACHE_CAP, (uint32_t)(hi - lo), x);
   const uint64_t p = lower_bound_u32(a.values, cur, hi, x);
@@ -462,27 +469,31 @@ __device__ void cache_suffix_lists(const JoinArgs &a, const JQuery *__restrict__
 // warp's shared copy (sf, sidx).  Lists are addressed by index through the
 // members' backward entries, so no per-lane arrays are needed.
 // ---------------------------------------------------------------------------
+template <bool C>
 struct LaneCtx {
   const JQuery *Q;
   uint32_t L, w, widx;
   const uint32_t *sf, *sidx;
-  ListCache lc;
+  ListCacheT<C> lc;
   uint64_t deadline;  // device time cap (%globaltimer ns)
   // prefix level ownp (if < QV) is this lane's own, not the warp's shared prefix
   uint32_t ownp = 0xFFu, wp = 0, widxp = 0;
 };
 
 // Vertex and candidate position of prefix level j for this lane.
-__device__ __forceinline__ uint32_t lvl_vertex(const LaneCtx &x, uint32_t j) {
+template <bool C>
+__device__ __forceinline__ uint32_t lvl_vertex(const LaneCtx<C> &x, uint32_t j) {
   return j == x.L ? x.w : j == x.ownp ? x.wp : x.sf[j];
 }
-__device__ __forceinline__ uint32_t lvl_index(const LaneCtx &x, uint32_t j) {
+template <bool C>
+__device__ __forceinline__ uint32_t lvl_index(const LaneCtx<C> &x, uint32_t j) {
   return j == x.L ? x.widx : j == x.ownp ? x.widxp : x.sidx[j];
 }
 
 // List li of the subset `members` of a suffix group: its range, its key
 // vertex (f of the key level) and the level of the member it belongs to.
-__device__ __forceinline__ void lane_list(const JoinArgs &a, const LaneCtx &x, uint32_t first, uint32_t members,
+template <bool C>
+__device__ __forceinline__ void lane_list(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                           uint32_t li, uint64_t &lo, uint64_t &hi, uint32_t &kv, uint32_t &mlvl) {
   lo = hi = 0;
   kv = 0;
@@ -497,7 +508,7 @@ __device__ __forceinline__ void lane_list(const JoinArgs &a, const LaneCtx &x, u
       const uint32_t kl = b->lvl;
       if (!inb(a, SITE_KEYLVL, kl, (uint64_t)x.L + 1)) return;
       kv = lvl_vertex(x, kl);
-      if (kl < x.L && kl != x.ownp) {  // keyed by the shared prefix: the warp's range table has it
+      if (C && kl < x.L && kl != x.ownp) {  // keyed by the shared prefix: the warp's range table has it
         const uint32_t ti = M->back_base + li - (uint32_t)x.lc.rng[64];
         if (ti < 32 && x.lc.rng[2 * ti] != ~0ull) {
           lo = x.lc.rng[2 * ti];
@@ -526,7 +537,8 @@ __device__ __forceinline__ bool vnh_list_has(const JoinArgs &a, const JQuery *Q,
 // Lists of one subset, at most three: ranges computed once, cached lists read
 // from shared memory, the others probed through the neighbourhood hash (or
 // searched from a moving start without it).
-__device__ uint64_t lane_subset_count3(const JoinArgs &a, const LaneCtx &x, uint32_t first, uint32_t members,
+template <bool C>
+__device__ uint64_t lane_subset_count3(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                        uint32_t nl, uint32_t dup_mask, Stats &st, bool &heavy) {
   uint64_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0, lo2 = 0, hi2 = 0;
   uint32_t kv0 = 0, kv1 = 0, kv2 = 0, ml0 = 0, ml1 = 0, ml2 = 0;
@@ -630,7 +642,8 @@ __device__ uint64_t lane_subset_count3(const JoinArgs &a, const LaneCtx &x, uint
   return c;
 }
 
-__device__ uint64_t lane_subset_count(const JoinArgs &a, const LaneCtx &x, uint32_t first, uint32_t members,
+template <bool C>
+__device__ uint64_t lane_subset_count(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                       uint32_t dup_mask, Stats &st, bool &heavy) {
   uint32_t nl = 0;
   for (uint32_t m = members; m; m &= m - 1) nl += x.Q->lv[(first + __ffs(m) - 1) & 31u].nback;
@@ -721,11 +734,12 @@ __device__ __forceinline__ uint32_t flat_blocks(uint64_t s, uint32_t len) {
 // Keys among `want` that are in the probed list (word and nb from
 // flat_probe_word, slot1 = cache slot + 1 or 0); keys come from a list of
 // member level sml.
-__device__ __forceinline__ uint32_t flat_probe8(const JoinArgs &a, const JQuery *Q, const ListCache &lc,
+template <bool C>
+__device__ __forceinline__ uint32_t flat_probe8(const JoinArgs &a, const JQuery *Q, const ListCacheT<C> &lc,
                                                 uint32_t slot1, uint64_t word, uint32_t nb, uint32_t ml,
                                                 uint32_t sml, const uint32_t (&vv)[8], uint32_t want) {
   if (!want) return 0;
-  if (slot1) return smem_member8(lc.buf + (slot1 - 1) * LIST_CACHE_CAP, (uint32_t)word, vv, want);
+  if (C && slot1) return smem_member8(lc.buf + (slot1 - 1) * LIST_CACHE_CAP, (uint32_t)word, vv, want);
   const VnhRow r{a.vnh_buckets + word, nb};
   uint32_t f = vnh_has8(r, vv, want);
   if (ml != sml) {
@@ -748,7 +762,8 @@ struct FlatOrigin {
 
 // v (any vertex) in a list: its cache slot, the neighbourhood hash with a
 // candidate test, or a binary search.
-__device__ __forceinline__ bool list_has_vertex(const JoinArgs &a, const LaneCtx &x, int slot, uint64_t lo,
+template <bool C>
+__device__ __forceinline__ bool list_has_vertex(const JoinArgs &a, const LaneCtx<C> &x, int slot, uint64_t lo,
                                                 uint64_t hi, uint32_t kv, uint32_t ml, uint32_t v) {
   if (slot >= 0) return smem_contains(x.lc.buf + slot * LIST_CACHE_CAP, (uint32_t)(hi - lo), v);
   if (a.vnh_buckets) return vnh_list_has(a, x.Q, kv, ml, ~0u, v);
@@ -762,7 +777,8 @@ __device__ __forceinline__ bool list_has_vertex(const JoinArgs &a, const LaneCtx
 // upper half of its work go to the queue (the recipient evaluates them
 // again) and their lanes count nothing here.  Returns false, having done
 // nothing, when the chunk's jobs do not fit the job table.
-__device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx &x, uint32_t m, char *fbase,
+template <bool C>
+__device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx<C> &x, uint32_t m, char *fbase,
                                                 const FlatOrigin &org, const LaneState &c, bool &pushed,
                                                 Stats &st, uint64_t &my_cnt) {
   const uint32_t lane = lane_id();
@@ -909,7 +925,7 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
       }
       cur_j = lo;
       const FJob jb = jobs[lo];
-      const uint32_t ss1 = (jb.meta >> 1) & 3u, sa1 = (jb.meta >> 3) & 3u, sb1 = (jb.meta >> 5) & 3u;
+      const uint32_t ss1 = C ? (jb.meta >> 1) & 3u : 0u, sa1 = (jb.meta >> 3) & 3u, sb1 = (jb.meta >> 5) & 3u;
       const uint32_t sml = (jb.meta >> 7) & 31u, aml = (jb.meta >> 12) & 31u, bml = (jb.meta >> 17) & 31u;
       // the block's sector: two 16-byte loads (the values array is a whole
       // number of sectors), the entries outside the list masked
@@ -977,7 +993,8 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
 
 // Suffix completions of one lane's prefix match; sets `heavy` (and returns
 // 0) when an intersection is too long for one lane.
-__device__ uint64_t lane_suffix_count(const JoinArgs &a, const LaneCtx &x, Stats &st, bool &heavy) {
+template <bool C>
+__device__ uint64_t lane_suffix_count(const JoinArgs &a, const LaneCtx<C> &x, Stats &st, bool &heavy) {
   const JQuery *Q = x.Q;
   uint64_t total = 1;
   const uint32_t ng = Q->n_groups < MAX_GROUPS ? Q->n_groups : MAX_GROUPS;
@@ -1019,7 +1036,8 @@ __device__ uint64_t lane_suffix_count(const JoinArgs &a, const LaneCtx &x, Stats
 // Warp-cooperative form for one deferred (heavy) prefix match: every lane
 // receives the same context; lists are spread one per lane and the shortest
 // is scanned 32 entries at a time.
-__device__ uint64_t warp_subset_count(const JoinArgs &a, const LaneCtx &x, uint32_t first, uint32_t members,
+template <bool C>
+__device__ uint64_t warp_subset_count(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                       uint32_t dup_mask, Stats &st) {
   const uint32_t lane = lane_id();
   uint32_t nl = 0;
@@ -1132,7 +1150,8 @@ __device__ uint64_t warp_subset_count(const JoinArgs &a, const LaneCtx &x, uint3
   return cnt;
 }
 
-__device__ uint64_t warp_suffix_count(const JoinArgs &a, const LaneCtx &x, Stats &st) {
+template <bool C>
+__device__ uint64_t warp_suffix_count(const JoinArgs &a, const LaneCtx<C> &x, Stats &st) {
   const JQuery *Q = x.Q;
   uint64_t total = 1;
   const uint32_t ng = Q->n_groups < MAX_GROUPS ? Q->n_groups : MAX_GROUPS;
@@ -1392,12 +1411,21 @@ __device__ __forceinline__ void emit_last(const JoinArgs &a, const JQuery *__res
   }
 }
 
-// Dynamic shared memory of a join block: the list caches and job tables that
-// only counting uses.
-static uint32_t join_smem(uint32_t mode) { return mode == MODE_COUNT ? JOIN_DYN_SMEM : 0u; }
+// The join's two counting kernels.  PART_POOLS: the lane-parallel pools
+// (roots, and (root, first level) pairs), whose counters need neither a DFS
+// stack nor cached lists.  PART_DFS: the ordinary pool and the task queue.
+// The enumerating modes run both in one kernel (their pool holds the
+// single-vertex queries only).
+enum : uint32_t { PART_POOLS = 1, PART_DFS = 2 };
 
-template <uint32_t MODE>
-__global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
+// Dynamic shared memory of a join block: the list caches and job tables that
+// only counting uses, the job tables alone in the pools.
+static uint32_t join_smem(uint32_t mode, uint32_t part) {
+  return mode != MODE_COUNT ? 0u : part == PART_POOLS ? JOIN_WARPS_PER_BLOCK * FLAT_WARP_BYTES : JOIN_DYN_SMEM;
+}
+
+template <uint32_t MODE, uint32_t PART>
+__global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) join_kernel(JoinArgs a) {
   const uint32_t lane = lane_id();
   JControl *ctl = a.ctl;
   const uint64_t deadline = ctl->deadline_ns;
@@ -1408,10 +1436,12 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
   ListCache lc;
   // per warp: the list cache, then the balanced-counting job table
   lc.buf = s_lcache + (threadIdx.x >> 5) * (JOIN_WARP_SMEM / 4);
-  char *fbuf = reinterpret_cast<char *>(lc.buf + LIST_CACHE_SLOTS * LIST_CACHE_CAP);
+  char *fbuf = PART == PART_POOLS ? reinterpret_cast<char *>(s_lcache) + (threadIdx.x >> 5) * FLAT_WARP_BYTES
+                                  : reinterpret_cast<char *>(lc.buf + LIST_CACHE_SLOTS * LIST_CACHE_CAP);
   lc.rng = reinterpret_cast<unsigned long long *>(fbuf + FLAT_WARP_BYTES);
   lc.tag = s_ctag[threadIdx.x >> 5];
-  if (MODE == MODE_COUNT) {
+  const ListCacheT<false> nolc{};
+  if (MODE == MODE_COUNT && (PART & PART_DFS)) {
     lc.rng[2 * lane] = ~0ull;
     if (lane == 0) lc.rng[64] = 0;
     if (lane < 2 * LIST_CACHE_SLOTS) lc.tag[lane] = 0ull;  // empty: no list has lo == hi == 0 and hi > lo
@@ -1432,7 +1462,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
 
   // ---------------------------------------------------------------- lane-parallel roots
   // Queries whose only enumerated level is the root: one root per lane.
-  if (a.lp_roots) {
+  if ((PART & PART_POOLS) && a.lp_roots) {
     uint32_t it = 0;
     for (;;) {
       unsigned long long base = 0;
@@ -1477,14 +1507,14 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
                 if (s < a.emb_cap) a.emb[s] = w0;
               }
             } else if (MODE == MODE_COUNT) {  // a suffix: count mode's plans only
-              LaneCtx x;
+              LaneCtx<false> x;
               x.Q = Q;
               x.L = 0;
               x.w = w0;
               x.widx = (uint32_t)rl;
               x.sf = sf;
               x.sidx = sidx;
-              x.lc = lc;
+              x.lc = nolc;
               x.deadline = deadline;
               cnt = lane_suffix_count(a, x, st, heavy);
               hq = q;
@@ -1500,14 +1530,14 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
       for (uint32_t hm = MODE == MODE_COUNT ? __ballot_sync(FULL, heavy) : 0u; hm; hm &= hm - 1) {
         const uint32_t hl = __ffs(hm) - 1;
         const uint32_t qh = __shfl_sync(FULL, hq, hl);
-        LaneCtx x;
+        LaneCtx<false> x;
         x.Q = a.queries + qh;
         x.L = 0;
         x.w = __shfl_sync(FULL, hw, hl);
         x.widx = __shfl_sync(FULL, hidx, hl);
         x.sf = sf;
         x.sidx = sidx;
-        x.lc = lc;
+        x.lc = nolc;
         x.deadline = deadline;
         const uint64_t k = warp_suffix_count(a, x, st);
         if (lane == 0 && k) atomicAdd(&a.out[qh].count, (unsigned long long)k);
@@ -1532,7 +1562,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
   // prefix matches are the entries of the root's edge table, taken 32 at a
   // time (each query's range padded to whole chunks), one match per lane with
   // its own root, so short neighbour lists still fill the warp.
-  if (MODE == MODE_COUNT && a.lp2_nq) {
+  if (MODE == MODE_COUNT && (PART & PART_POOLS) && a.lp2_nq) {
     const uint64_t total = a.lp2_prefix[a.lp2_nq];
     uint32_t it = 0;
     for (;;) {
@@ -1579,14 +1609,14 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
         }
       }
       const uint32_t m = __ballot_sync(FULL, valid);
-      LaneCtx x;
+      LaneCtx<false> x;
       x.Q = Q;
       x.L = 1;
       x.w = f1;
       x.widx = i1;
       x.sf = sf;
       x.sidx = sidx;
-      x.lc = lc;
+      x.lc = nolc;
       x.deadline = deadline;
       x.ownp = 0;
       x.wp = f0;
@@ -1601,7 +1631,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
         cnt = valid ? lane_suffix_count(a, x, st, heavy) : 0;
         for (uint32_t hm = __ballot_sync(FULL, heavy); hm; hm &= hm - 1) {
           const uint32_t hl = __ffs(hm) - 1;
-          LaneCtx y = x;
+          LaneCtx<false> y = x;
           y.w = __shfl_sync(FULL, f1, hl);
           y.widx = __shfl_sync(FULL, i1, hl);
           y.wp = __shfl_sync(FULL, f0, hl);
@@ -1635,7 +1665,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
   uint64_t rb_first = 0;
   uint32_t iq = 0, if0 = 0, ik0 = 0, if1 = 0, ik1 = 0;
   uint32_t iter = 0;  // chunks evaluated: the time cap is looked at every fourth
-  for (;;) {
+  for (; PART & PART_DFS;) {
     // ------------------------------------------------------------ acquire
     uint32_t q = 0, base_lvl = 0, lvl = 0;
     bool have = false, from_root = false;
@@ -1855,7 +1885,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
           }
           bool flat_done = false;
           if (Q->flat && a.vnh_buckets) {
-            LaneCtx x;
+            LaneCtx<true> x;
             x.Q = Q;
             x.L = lvl;
             x.w = w;
@@ -1877,7 +1907,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
           uint32_t widx = 0;
           uint64_t my_cnt = 0;
           if (!flat_done && ((m >> lane) & 1u)) {
-            LaneCtx x;
+            LaneCtx<true> x;
             x.Q = Q;
             x.L = lvl;
             x.w = w;
@@ -1910,7 +1940,7 @@ __global__ void __launch_bounds__(256, 2) join_kernel(JoinArgs a) {
           lane_cnt += my_cnt;
           for (; hm; hm &= hm - 1) {
             const uint32_t hl = __ffs(hm) - 1;
-            LaneCtx x;
+            LaneCtx<true> x;
             x.Q = Q;
             x.L = lvl;
             x.w = __shfl_sync(FULL, w, hl);
@@ -2088,26 +2118,32 @@ __global__ void join_prepare_kernel(JControl *ctl, JOut *out, uint32_t nquery, J
   }
 }
 
-static void *join_fn(uint32_t mode) {
-  if (mode == MODE_COUNT) return (void *)join_kernel<MODE_COUNT>;
-  if (mode == MODE_HASH) return (void *)join_kernel<MODE_HASH>;
-  return (void *)join_kernel<MODE_ENUM>;
+static void *join_fn(uint32_t mode, uint32_t part) {
+  if (mode == MODE_COUNT)
+    return part == PART_POOLS ? (void *)join_kernel<MODE_COUNT, PART_POOLS> : (void *)join_kernel<MODE_COUNT, PART_DFS>;
+  return mode == MODE_HASH ? (void *)join_kernel<MODE_HASH, PART_POOLS | PART_DFS>
+                           : (void *)join_kernel<MODE_ENUM, PART_POOLS | PART_DFS>;
 }
 
 // The list cache takes JOIN_DYN_SMEM of dynamic shared memory per block,
-// above the default 48 KiB limit: the counting instance opts in once.
+// above the default 48 KiB limit: the counting instances opt in once.
 static cudaError_t join_smem_optin() {
   static cudaError_t done = [] {
-    return cudaFuncSetAttribute(join_fn(MODE_COUNT), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JOIN_DYN_SMEM);
+    for (uint32_t part : {PART_POOLS, PART_DFS}) {
+      const cudaError_t e = cudaFuncSetAttribute(join_fn(MODE_COUNT, part), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)join_smem(MODE_COUNT, part));
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }();
   return done;
 }
 
-int join_blocks_per_sm(uint32_t mode) {
+static int blocks_per_sm(uint32_t mode, uint32_t part) {
   int n = 0;
   if (join_smem_optin() != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, join_fn(mode), JOIN_WARPS_PER_BLOCK * 32, join_smem(mode)) !=
-          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, join_fn(mode, part), JOIN_WARPS_PER_BLOCK * 32,
+                                                    join_smem(mode, part)) != cudaSuccess ||
       n <= 0) {
     cudaGetLastError();
     n = 1;
@@ -2115,13 +2151,19 @@ int join_blocks_per_sm(uint32_t mode) {
   return n;
 }
 
+int join_blocks_per_sm(uint32_t mode) { return blocks_per_sm(mode, PART_DFS); }
+int join_pool_blocks_per_sm() { return blocks_per_sm(MODE_COUNT, PART_POOLS); }
+
 void destroy_join_graph(JoinGraph &jg) {
-  if (jg.exec) cudaGraphExecDestroy(jg.exec);
-  if (jg.graph) cudaGraphDestroy(jg.graph);
-  jg = JoinGraph();
+  for (JoinGraph::Shape &g : jg.shape) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (g.graph) cudaGraphDestroy(g.graph);
+    g = JoinGraph::Shape();
+  }
 }
 
-cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns, uint32_t grid, cudaStream_t s) {
+cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns, uint32_t grid, uint32_t pool_grid,
+                              cudaStream_t s) {
   JoinArgs args = a;
   JControl *ctl = a.ctl;
   JOut *out = a.out;
@@ -2136,33 +2178,38 @@ cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns,
   uint64_t *lp2_prefix = const_cast<uint64_t *>(a.lp2_prefix);
   void *prep_params[] = {&ctl, &out, &nq, &cells, &qends, &cap, &queries, &backs, &lp2q, &lp2_nq, &lp2_prefix};
   void *join_params[] = {&args};
-  cudaKernelNodeParams pp = {};
-  pp.func = (void *)join_prepare_kernel;
-  pp.gridDim = dim3(32);
-  pp.blockDim = dim3(256);
-  pp.kernelParams = prep_params;
-  cudaKernelNodeParams jp = {};
-  jp.func = join_fn(a.mode);
-  jp.gridDim = dim3(grid);
-  jp.blockDim = dim3(JOIN_WARPS_PER_BLOCK * 32);
-  jp.sharedMemBytes = join_smem(a.mode);
-  jp.kernelParams = join_params;
+  // the kernels this wave needs, in order
+  const bool split = a.mode == MODE_COUNT;
+  const bool pools = split && (a.lp_roots || a.lp2_nq), dfs = !split || a.n_roots;
+  cudaKernelNodeParams kp[3] = {};
+  uint32_t nk = 0;
+  auto node = [&](void *fn, uint32_t blocks, uint32_t smem, void **params) {
+    kp[nk].func = fn;
+    kp[nk].gridDim = dim3(blocks);
+    kp[nk].blockDim = dim3(JOIN_WARPS_PER_BLOCK * 32);
+    kp[nk].sharedMemBytes = smem;
+    kp[nk].kernelParams = params;
+    ++nk;
+  };
+  node((void *)join_prepare_kernel, 32, 0, prep_params);
+  if (pools) node(join_fn(a.mode, PART_POOLS), pool_grid, join_smem(a.mode, PART_POOLS), join_params);
+  if (dfs) node(join_fn(a.mode, PART_DFS), grid, join_smem(a.mode, PART_DFS), join_params);
   cudaError_t e;
   if ((e = join_smem_optin()) != cudaSuccess) return e;
-  if (!jg.exec || jg.mode != a.mode || jg.grid != grid) {
-    destroy_join_graph(jg);
-    if ((e = cudaGraphCreate(&jg.graph, 0)) != cudaSuccess) return e;
-    if ((e = cudaGraphAddKernelNode(&jg.prep, jg.graph, nullptr, 0, &pp)) != cudaSuccess) return e;
-    if ((e = cudaGraphAddKernelNode(&jg.join, jg.graph, &jg.prep, 1, &jp)) != cudaSuccess) return e;
-    if ((e = cudaGraphInstantiate(&jg.exec, jg.graph, 0)) != cudaSuccess) return e;
-    jg.mode = a.mode;
-    jg.grid = grid;
+  JoinGraph::Shape &g = jg.shape[a.mode == MODE_COUNT ? (pools ? 1 : 0) + (dfs ? 2 : 0) : 3 + a.mode];
+  if (!g.exec) {
+    if ((e = cudaGraphCreate(&g.graph, 0)) != cudaSuccess) return e;
+    for (uint32_t i = 0; i < nk; ++i)
+      if ((e = cudaGraphAddKernelNode(&g.node[i], g.graph, i ? &g.node[i - 1] : nullptr, i ? 1 : 0, &kp[i])) !=
+          cudaSuccess)
+        return e;
+    if ((e = cudaGraphInstantiate(&g.exec, g.graph, 0)) != cudaSuccess) return e;
   } else {
-    if ((e = cudaGraphExecKernelNodeSetParams(jg.exec, jg.prep, &pp)) != cudaSuccess) return e;
-    if ((e = cudaGraphExecKernelNodeSetParams(jg.exec, jg.join, &jp)) != cudaSuccess) return e;
+    for (uint32_t i = 0; i < nk; ++i)
+      if ((e = cudaGraphExecKernelNodeSetParams(g.exec, g.node[i], &kp[i])) != cudaSuccess) return e;
   }
-  count_launch(2);
-  return cudaGraphLaunch(jg.exec, s);
+  count_launch(nk);
+  return cudaGraphLaunch(g.exec, s);
 }
 
 }  // namespace gem

@@ -406,17 +406,23 @@ struct JoinArgs {
 };
 // The join of a wave as a CUDA graph: a prepare kernel (zero the control
 // block and the per-query outputs, reset the task queue, set the device
-// deadline) followed by the persistent join.  One executable graph is built
-// per (mode, grid) and reused; each wave only updates the two kernel nodes'
-// parameters before cudaGraphLaunch.
+// deadline), then the persistent join: for counting, the lane-parallel pools
+// and the depth-first part as kernels of their own, each only when the wave
+// has work for it.  One executable graph per such shape is built and reused;
+// each wave only updates the kernel nodes' parameters.
 struct JoinGraph {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t prep = nullptr, join = nullptr;
-  uint32_t mode = 0, grid = 0;
+  struct Shape {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    cudaGraphNode_t node[3] = {nullptr, nullptr, nullptr};
+  };
+  Shape shape[6];  // counting: pools | depth-first part << 1; then the hash and enumerate modes
 };
-cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns, uint32_t grid, cudaStream_t s);
+constexpr int POOL_BLOCKS = 3;  // blocks per SM of the pools' kernel
+cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns, uint32_t grid, uint32_t pool_grid,
+                              cudaStream_t s);
 void destroy_join_graph(JoinGraph &jg);
 int join_blocks_per_sm(uint32_t mode);
+int join_pool_blocks_per_sm();
 
 }  // namespace gem
