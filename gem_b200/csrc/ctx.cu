@@ -854,7 +854,8 @@ static cudaError_t d2h_sync(gem_ctx *ctx, void *dst, const void *src, size_t byt
   return e;
 }
 
-static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
+// columns: also the membership columns the table passes read.
+static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool columns) {
   const uint32_t nwords = (ctx->g.nv + 31) / 32;
   w.nwords = nwords;
   // Rows.  The filter predicate of a query vertex depends only on its label,
@@ -908,9 +909,8 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
     const std::vector<uint32_t> &sg = row_sig[ord[k]];
     FilterRow &f = fr[k];
     std::memset(&f, 0, sizeof f);
-    f.lab = sg[0];
     f.row = ord[k];
-    if (f.lab >= ctx->g.nlabels) f.need = UINT32_MAX;  // no vertex has the label
+    if (sg[0] >= ctx->g.nlabels) f.need = UINT32_MAX;  // no vertex has the label
     f.more = (uint32_t)more.size();
     uint32_t n = 0;
     for (size_t i = 2, j; i < sg.size(); i = j) {  // runs of one neighbour label
@@ -927,6 +927,31 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
     }
     f.n_more = (uint32_t)more.size() - f.more;
   }
+  // groups of up to 32 rows of one label; a label's rows are consecutive bit
+  // positions from a multiple of 32 on (waves of at most 32 rows: all rows
+  // share one column word, and no label list is needed to find their bits)
+  std::vector<FilterGroup> groups;
+  const bool one = rows <= 32;
+  w.labels.clear();
+  w.row_pos.assign(rows, 0);
+  w.row_lab.resize(rows);
+  w.pos_words = one ? 1 : 0;
+  uint32_t widest = 1;  // column words of a label
+  for (uint32_t k = 0, e; k < rows; k = e) {
+    const uint32_t lab = row_sig[ord[k]][0];
+    for (e = k; e < rows && row_sig[ord[e]][0] == lab; ++e) {
+      w.row_pos[ord[e]] = one ? e : 32 * w.pos_words + (e - k);
+      w.row_lab[ord[e]] = lab;
+    }
+    const uint32_t words = (e - k + 31) / 32;
+    for (uint32_t c = 0; c < words; ++c)
+      groups.push_back(FilterGroup{lab, k + 32 * c, std::min(32u, e - k - 32 * c), c, one ? k : 0u});
+    if (one) continue;
+    widest = std::max(widest, words);
+    w.labels.push_back(RowLabel{lab, w.pos_words, words, 0});
+    w.pos_words += words;
+  }
+  w.W = widest <= 2 ? widest : (widest + 3) / 4 * 4;
   if (!stride && !wl.empty()) {
     stride = (uint32_t)((wl.size() + 15) / 16) * 16;
     uint32_t *d_wl;
@@ -944,17 +969,27 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
   ST(aalloc(ctx, more.empty() ? 1 : more.size(), &d_more));
   CU(h2d(ctx, d_more, more.data(), 4 * more.size()));
   const uint64_t nbits = (uint64_t)rows * nwords;
-  const uint32_t ts = filter_set_tiles(rows, nwords), nsets = (nwords + ts - 1) / ts;
+  FilterGroup *d_groups;
+  ST(aalloc(ctx, groups.empty() ? 1 : groups.size(), &d_groups));
+  CU(h2d(ctx, d_groups, groups.data(), groups.size() * sizeof(FilterGroup)));
+  w.d_cols = nullptr;
+  if (columns) {
+    ST(aalloc(ctx, (uint64_t)ctx->g.nv * w.W, &w.d_cols));
+    if (one) CU(cudaMemsetAsync(w.d_cols, 0, 4ull * ctx->g.nv, ctx->s));
+  }
+  const uint32_t ts = filter_set_tiles((uint32_t)groups.size(), nwords), nsets = (nwords + ts - 1) / ts;
   const uint64_t nsc = (uint64_t)rows * nsets;
+  uint32_t *d_bits;
   ST(aalloc(ctx, nbits, &w.d_rb));
-  ST(aalloc(ctx, nbits, &w.d_bits));
+  ST(aalloc(ctx, nbits, &d_bits));
   uint32_t *d_cnt;
   uint64_t *d_ex, *d_tmp, *d_rows;
   ST(aalloc(ctx, nsc, &d_cnt));
   ST(aalloc(ctx, nsc + 1, &d_ex));
   ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
-  launch_filter(ctx->g, nlc, stride, d_fr, d_more, rows, threshold, w.d_bits, d_cnt, nwords, ctx->s);
+  launch_filter(ctx->g, nlc, stride, d_fr, d_more, d_groups, (uint32_t)groups.size(), ts, threshold, d_bits, d_cnt,
+                w.d_cols, w.W, nwords, ctx->s);
   launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
   launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
   std::vector<uint64_t> rs(rows + 1);
@@ -966,16 +1001,15 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold) {
   for (uint32_t r = 0; r <= rows; ++r) w.c_base[r] = rs[r];
   const uint64_t total = w.c_base[rows];
   ST(aalloc(ctx, total ? total : 1, &w.d_cand));
-  launch_rank_rows(w.d_bits, rows, nwords, d_ex, w.d_rb, w.d_cand, ctx->s);
+  launch_rank_rows(d_bits, rows, nwords, d_ex, ts, w.d_rb, w.d_cand, ctx->s);
   CU(cudaGetLastError());
   w.cand_total = total;
   // algorithmic bytes: the labels of every vertex, the label counts of the
   // vertices of every label that some row has, the rows' words (written,
   // read and rewritten as rank words), the candidate lists
   uint64_t b = 4ull * ctx->g.nv + 16 * nbits + 4 * total;
-  for (uint32_t k = 0; k < rows; ++k)
-    if ((k == 0 || fr[k].lab != fr[k - 1].lab) && fr[k].lab < ctx->label_freq.size())
-      b += (uint64_t)stride * ctx->label_freq[fr[k].lab];
+  for (const RowLabel &l : w.labels)
+    if (l.lab < ctx->label_freq.size()) b += (uint64_t)stride * ctx->label_freq[l.lab];
   w.bytes_filter = b;
   return GEM_OK;
 }
@@ -1047,20 +1081,23 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), nkeys, d_tiles, ctx->s);
   launch_scan(d_tiles, SCAN_U32, nkeys, d_tp, d_tmp, ctx->s);
   launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_stb, ctx->s);
-  // Vertex tiles: which sources hold each vertex (the source membership
-  // columns, WS words per vertex) and the 32-arc tiles of every vertex that
-  // some source holds; the table passes walk those tiles once for all sources.
+  // Vertex tiles: the 32-arc tiles of every vertex that some source holds
+  // (its membership column under the sources' bits); the table passes walk
+  // those tiles once for all sources.
   const uint32_t nv = ctx->g.nv;
-  const uint32_t WS = (uint32_t)((src.size() + 31) / 32);
-  uint32_t *d_srow, *d_S, *d_vtiles;
+  std::vector<uint32_t> smask(w.pos_words, 0);
+  for (uint32_t r : src_row) smask[w.row_pos[r] >> 5] |= 1u << (w.row_pos[r] & 31u);
+  RowLabel *d_labels;
+  uint32_t *d_smask, *d_vtiles;
   uint64_t *d_vtp, *d_tmp3;
-  ST(aalloc(ctx, src.size(), &d_srow));
-  CU(h2d(ctx, d_srow, src_row.data(), 4 * src_row.size()));
-  ST(aalloc(ctx, (uint64_t)nv * WS, &d_S));
+  ST(aalloc(ctx, w.labels.empty() ? 1 : w.labels.size(), &d_labels));
+  CU(h2d(ctx, d_labels, w.labels.data(), w.labels.size() * sizeof(RowLabel)));
+  ST(aalloc(ctx, smask.size(), &d_smask));
+  CU(h2d(ctx, d_smask, smask.data(), 4 * smask.size()));
   ST(aalloc(ctx, nv ? nv : 1, &d_vtiles));
   ST(aalloc(ctx, (uint64_t)nv + 1, &d_vtp));
   ST(aalloc(ctx, scan_tmp_words(nv), &d_tmp3));
-  launch_row_columns(w.d_bits, w.nwords, d_srow, (uint32_t)src.size(), WS, nv, d_S, d_vtiles, ctx->g.deg, ctx->s);
+  launch_vertex_tiles(ctx->g, d_labels, (uint32_t)w.labels.size(), w.d_cols, w.W, d_smask, d_vtiles, ctx->s);
   launch_scan(d_vtiles, SCAN_U32, nv, d_vtp, d_tmp3, ctx->s);
   // the write pass's units: up to TAB_WGROUP consecutive tiles of one vertex
   uint32_t *d_vunits;
@@ -1096,8 +1133,6 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // a table is keyed by its source row and filtered by its target row: queries
   // (or twin query vertices) that need the same pair share one table
   std::map<std::pair<uint32_t, uint32_t>, uint32_t> edge_by_rows;
-  std::vector<uint32_t> tgt_row;  // the target rows, one membership column bit each
-  std::vector<int> row_tcol(w.nrows, -1);
   for (const EdgeReq &rq : reqs) {
     const Plan &p = w.plan[rq.qi];
     const uint32_t tgt = w.row_of[rq.qi][p.order[rq.k]];
@@ -1113,12 +1148,11 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     TabEdge e;
     e.src = rq.s;
     e.flags = flags;
-    if (row_tcol[tgt] < 0) {
-      row_tcol[tgt] = (int)tgt_row.size();
-      tgt_row.push_back(tgt);
-    }
-    e.tcol = (uint32_t)row_tcol[tgt];
-    e.pad = 0;
+    e.tlab = w.row_lab[tgt];
+    e.tcol = w.row_pos[tgt];  // all rows in one column word, else the position within its label
+    if (!w.labels.empty())
+      e.tcol -= 32 * std::lower_bound(w.labels.begin(), w.labels.end(), e.tlab,
+                                      [](const RowLabel &x, uint32_t l) { return x.lab < l; })->word0;
     e.tile_base = tiles;
     e.ntiles = stb[rq.s + 1] - stb[rq.s];
     e.off_base = offs;
@@ -1142,30 +1176,25 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   ST(aalloc(ctx, tiles ? tiles : 1, &d_mask));
   ST(aalloc(ctx, tiles + 1, &d_vp));
   ST(aalloc(ctx, scan_tmp_words(tiles), &d_tmp2));
-  // the target membership columns, the tile -> vertex map, and the sources
-  // and tables as the passes read them
-  // target columns: whole 16-byte chunks per vertex (the count pass stages
-  // them with 16-byte asynchronous copies)
-  const uint32_t WT = (uint32_t)((tgt_row.size() + 127) / 128 * 4);
-  if (!table_vtx_fits(WT)) {
-    ctx->err = "too many edge-table target rows in one wave";
+  // the tile -> vertex map, and the sources (by row position) and tables as
+  // the passes read them
+  if (!table_vtx_fits(w.W)) {
+    ctx->err = "too many filter rows of one label in one wave";
     return GEM_ERR_LIMIT;
   }
-  uint32_t *d_trow, *d_B, *d_vt;
-  ST(aalloc(ctx, tgt_row.size(), &d_trow));
-  CU(h2d(ctx, d_trow, tgt_row.data(), 4 * tgt_row.size()));
-  ST(aalloc(ctx, (uint64_t)nv * WT, &d_B));
-  launch_row_columns(w.d_bits, w.nwords, d_trow, (uint32_t)tgt_row.size(), WT, nv, d_B, nullptr, nullptr, ctx->s);
+  uint32_t *d_vt;
   uint32_t *d_vg;
   ST(aalloc(ctx, vtiles ? vtiles : 1, &d_vt));
   launch_vertex_tile_map(d_vtp, nv, d_vt, ctx->s);
   ST(aalloc(ctx, vunits ? vunits : 1, &d_vg));
   launch_vertex_tile_map(d_vgp, nv, d_vg, ctx->s);
-  std::vector<VSrc> vs(src.size());
+  std::vector<VSrc> vs(32 * (size_t)w.pos_words);
   for (size_t i = 0; i < src.size(); ++i)
-    vs[i] = VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, stb[i], sedge[2 * i], sedge[2 * i + 1]};
+    vs[w.row_pos[src_row[i]]] =
+        VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, stb[i], sedge[2 * i], sedge[2 * i + 1]};
   std::vector<VEdge> ve(edge.size());
-  for (size_t i = 0; i < edge.size(); ++i) ve[i] = VEdge{edge[i].tile_base, edge[i].tcol, edge[i].flags};
+  for (size_t i = 0; i < edge.size(); ++i)
+    ve[i] = VEdge{edge[i].tile_base, edge[i].tlab, edge[i].tcol | (edge[i].flags & TAB_KEY_MAP) << 31};
   VSrc *d_vs;
   VEdge *d_ve;
   ST(aalloc(ctx, vs.size(), &d_vs));
@@ -1212,10 +1241,13 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.vtp = d_vtp;
     P.vg = d_vg;
     P.vgp = d_vgp;
-    P.S = d_S;
-    P.WS = WS;
-    P.WT = WT;
-    P.B = d_B;
+    P.lab = ctx->g.lab;
+    P.labels = d_labels;
+    P.nlab = (uint32_t)w.labels.size();
+    P.nlabels = ctx->g.nlabels;
+    P.W = w.W;
+    P.cols = w.d_cols;
+    P.smask = d_smask;
     P.vsrc = d_vs;
     P.vedge = d_ve;
     P.tp = d_tp;
@@ -1305,12 +1337,12 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   w.table_values = nvals;
   w.table_tiles = tiles;
   // algorithmic bytes of the two passes: per vertex tile (each pass) its
-  // offsets, 32 neighbour ids and source column, and (count) the 32 target
-  // columns; per tile of a source (each pass) the rank word and tile base;
+  // offsets, 32 neighbour ids and column, and (count) the 32 neighbours'
+  // columns and labels; per tile of a source (each pass) the rank word and tile base;
   // per table tile the mask written and read and the value position; per
   // value its id (and key position); the offsets; per key its tile count
   // and scan.
-  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * WS) + vtiles * 32ull * 4 * WT + 2 * src_tiles * 16 +
+  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * w.W) + vtiles * 32ull * 4 * (w.W + 1) + 2 * src_tiles * 16 +
                    tiles * (4 + 4 + 8) + nvals * (w.d_vkey ? 8 : 4) + offs * 8 + nkeys * (4 + 8 + 4);
   return GEM_OK;
 }
@@ -1647,7 +1679,7 @@ gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_
     return GEM_OK;
   };
   CU(cudaEventRecord(ctx->ev[0], ctx->s));
-  ST(wave_filter(ctx, w, threshold));
+  ST(wave_filter(ctx, w, threshold, true));
   ST(phase_sync("filter"));
   CU(cudaEventRecord(ctx->ev[1], ctx->s));
   auto h0 = std::chrono::steady_clock::now();
@@ -1983,7 +2015,7 @@ extern "C" gem_status gem_filter(gem_ctx *ctx, const gem_query *q, uint32_t thre
   ST(make_host_query(q, w.q[0], ctx->err));
   ctx->arena.reset();
   w.share_rows = false;  // rows in query-vertex order, one each
-  ST(wave_filter(ctx, w, threshold));
+  ST(wave_filter(ctx, w, threshold, false));
   CU(cudaStreamSynchronize(ctx->s));
   for (uint32_t u = 0; u < q->nv; ++u) counts[u] = w.cnt[u];
   if (w.cand_total > cand_cap) return GEM_ERR_OVERFLOW;
@@ -2005,7 +2037,7 @@ extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t 
   ctx->arena.reset();
   w.share_rows = false;  // rows in query-vertex order, one each
   w.active.assign(1, 1);
-  ST(wave_filter(ctx, w, 0));
+  ST(wave_filter(ctx, w, 0, true));
   // a two-level plan: u then w
   Plan p;
   p.n = 2;
@@ -2043,7 +2075,7 @@ extern "C" gem_status gem_index_probe(gem_ctx *ctx, const gem_query *q, uint32_t
   w.active.assign(1, 1);
   w.idx_kind.assign(1, std::vector<uint32_t>(QV, 0));
   w.ck_of.assign(1, std::vector<const CuckooTable *>(QV, nullptr));
-  ST(wave_filter(ctx, w, 0));
+  ST(wave_filter(ctx, w, 0, false));
   uint32_t *d_keys, *d_out;
   ST(aalloc(ctx, n_keys ? n_keys : 1, &d_keys));
   ST(aalloc(ctx, n_keys ? n_keys : 1, &d_out));

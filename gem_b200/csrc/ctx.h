@@ -81,7 +81,16 @@ struct Wave {
   uint32_t *d_vkey = nullptr;       // key positions of the pool queries' root-table values
   uint32_t nrows = 0, nwords = 0, nsrc = 0;
   uint64_t *d_rb = nullptr;       // rank bitmaps, nrows x nwords
-  uint32_t *d_bits = nullptr;     // their membership bits alone, nrows x nwords
+  // Membership columns: per data vertex W words, bit b of word c = the vertex
+  // is in the row at position 32 (word0 + c) + b, word0 of the vertex's label
+  // (rows of one label are consecutive positions); unset for vertices whose
+  // label no row has.
+  uint32_t *d_cols = nullptr;
+  uint32_t W = 1;
+  std::vector<gem::RowLabel> labels;  // the rows' labels, sorted
+  std::vector<uint32_t> row_pos;      // position per row
+  std::vector<uint32_t> row_lab;      // label per row
+  uint32_t pos_words = 0;             // positions / 32
   uint32_t *d_cand = nullptr;     // candidate lists back to back
   std::vector<uint32_t> cnt;      // |C| per row
   std::vector<uint64_t> c_base;   // list start per row

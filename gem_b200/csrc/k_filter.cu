@@ -15,76 +15,88 @@
 
 namespace gem {
 
-// One warp per (set of TS tiles of 32 vertices, group of R rows): a lane per
-// row (and per tile, 32 / R of them side by side when the wave has few rows).
-// Only a tile's vertices of the row's own label can be its candidates, a few
-// of the 32: the warp finds them with one ballot per distinct label of the
-// group (rows come sorted by label, so mostly one), and each lane tests its
-// row's needs (label, count) on those vertices alone.  The words are turned
-// in shared memory so that a row's TS words leave in one coalesced store.
+// One warp per (set of TS tiles of 32 vertices, group of up to 32 rows of one
+// label): a lane per row (and per tile, several side by side for a group of
+// few rows).  Only a tile's vertices of that label, a few of the
+// 32, can be the rows' candidates: one ballot finds them, and the lanes test
+// their rows' needs (label, count) on those vertices alone, all on the same
+// one, so that a ballot of the answers is the vertex's membership column.
+// The rows' words are turned in shared memory so that a row's TS words leave
+// in one coalesced store.
 //
 // What bounds it is instruction issue, then the words written.  A lane per
 // vertex instead, every row tested on all 32 of them against a descriptor of
-// up to 32 labels (the counts copied to local memory), took 6.0 ms for
-// the 2,880 query vertices of 180 mixed-size queries on 1,048,576 vertices
-// with 32 labels; this form 0.2 ms.
+// up to 32 labels (the counts copied to local memory), took 6 ms for the
+// 2,880 query vertices of 180 mixed-size queries on 1,048,576 vertices with
+// 32 labels, and transposing the columns out of the rows' words 2.2 ms; the
+// whole filter phase, host and compaction included, is 2.4 ms now (8.1).
 template <uint32_t TS>
 __global__ void __launch_bounds__(256) filter_kernel(const uint32_t *__restrict__ lab, uint32_t nv,
                                                      const uint8_t *__restrict__ nlc, uint32_t stride,
                                                      const FilterRow *__restrict__ rows,
-                                                     const uint32_t *__restrict__ more, uint32_t nrows, uint32_t R,
-                                                     uint32_t T, uint32_t nwords, uint32_t *__restrict__ bits,
-                                                     uint32_t *__restrict__ cnt) {
+                                                     const uint32_t *__restrict__ more,
+                                                     const FilterGroup *__restrict__ groups, uint32_t ngroups,
+                                                     uint32_t T, uint32_t nwords,
+                                                     uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt,
+                                                     uint32_t *__restrict__ cols, uint32_t W) {
   __shared__ uint32_t turn[8][32][TS + 1];
   const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t ngroups = (nrows + R - 1) / R, nsets = (nwords + TS - 1) / TS;
-  const uint32_t rl = lane & (R - 1), sub = lane / R, nsub = 32 / R;
+  const uint32_t nsets = (nwords + TS - 1) / TS;
   const uint64_t items = (uint64_t)ngroups * nsets;
   for (uint64_t it = blockIdx.x * 8ull + warp; it < items; it += gridDim.x * 8ull) {
-    const uint32_t set = (uint32_t)(it / ngroups), ri = (uint32_t)(it % ngroups) * R + rl;
-    const bool have = ri < nrows;
+    const uint32_t set = (uint32_t)(it / ngroups);
+    const FilterGroup g = groups[it % ngroups];
+    // lanes per tile: the group's rows rounded up to a power of two (no more
+    // tiles side by side than a set has)
+    uint32_t lg = g.n > 1 ? 32 - __clz(g.n - 1) : 0;
+    if (32u >> lg > TS) lg = 31 - __clz(32u / TS);
+    const uint32_t R = 1u << lg, rl = lane & (R - 1), sub = lane >> lg, nsub = 32u >> lg;
+    const uint32_t mine = R == 32 ? dev::FULL : (1u << R) - 1u;
+    const bool have = rl < g.n;
     FilterRow row = {};
-    if (have) row = rows[ri];
+    if (have) row = rows[g.row0 + rl];
     const bool live = have && row.need <= T;
-    // one lane per distinct label of the group
-    const uint32_t same = __match_any_sync(dev::FULL, live ? row.lab : 0xFFFFFFFFu);
-    const uint32_t leaders = __ballot_sync(dev::FULL, live && lane == (uint32_t)__ffs(same) - 1);
     uint32_t n = 0;
     for (uint32_t t0 = 0; t0 < TS; t0 += nsub) {
       uint32_t m = 0;
       for (uint32_t j = 0; j < nsub; ++j) {
         const uint64_t v = ((uint64_t)set * TS + t0 + j) * 32 + lane;
-        const bool valid = v < nv;
-        const uint32_t l = valid ? __ldg(lab + v) : 0u;
-        for (uint32_t x = leaders; x; x &= x - 1) {
-          const uint32_t ll = __shfl_sync(dev::FULL, row.lab, __ffs(x) - 1);
-          const uint32_t b = __ballot_sync(dev::FULL, valid && l == ll);
-          if (live && sub == j && row.lab == ll) m = b;
-        }
+        const uint32_t b = __ballot_sync(dev::FULL, v < nv && __ldg(lab + v) == g.lab);
+        if (sub == j) m = b;
       }
       const uint64_t vb = ((uint64_t)set * TS + t0 + sub) * 32;
       uint32_t word = 0;
-      while (m) {  // two vertices a step: their loads overlap
-        const uint32_t b0 = __ffs(m) - 1;
+      while (__ballot_sync(dev::FULL, m != 0)) {  // two vertices a step: their loads overlap
+        const bool a0 = m != 0;
+        const uint32_t b0 = a0 ? __ffs(m) - 1 : 0u;
+        m &= m - 1;  // 0 stays 0
+        const bool a1 = m != 0;
+        const uint32_t b1 = a1 ? __ffs(m) - 1 : b0;
         m &= m - 1;
-        const uint32_t b1 = m ? __ffs(m) - 1 : b0;
-        m &= m - 1;
-        const uint8_t *r0 = nlc + (vb + b0) * stride, *r1 = nlc + (vb + b1) * stride;
         uint32_t d0 = row.need, d1 = row.need;
+        if (live && a0) {
+          const uint8_t *r0 = nlc + (vb + b0) * stride, *r1 = nlc + (vb + b1) * stride;
 #pragma unroll
-        for (uint32_t i = 0; i < FILTER_NEEDS; ++i) {
-          const uint32_t k = row.needs[i] >> 8, q = row.needs[i] & 0xFFu;  // unused entries need 0
-          const uint32_t c0 = q ? __ldg(r0 + k) : 0u, c1 = q ? __ldg(r1 + k) : 0u;
-          d0 += q > c0 ? q - c0 : 0u;
-          d1 += q > c1 ? q - c1 : 0u;
+          for (uint32_t i = 0; i < FILTER_NEEDS; ++i) {
+            const uint32_t k = row.needs[i] >> 8, q = row.needs[i] & 0xFFu;  // unused entries need 0
+            const uint32_t c0 = q ? __ldg(r0 + k) : 0u, c1 = q ? __ldg(r1 + k) : 0u;
+            d0 += q > c0 ? q - c0 : 0u;
+            d1 += q > c1 ? q - c1 : 0u;
+          }
+          for (uint32_t i = 0; i < row.n_more; ++i) {
+            const uint32_t e = __ldg(more + row.more + i), k = e >> 8, q = e & 0xFFu;
+            const uint32_t c0 = __ldg(r0 + k), c1 = __ldg(r1 + k);
+            d0 += q > c0 ? q - c0 : 0u;
+            d1 += q > c1 ? q - c1 : 0u;
+          }
         }
-        for (uint32_t i = 0; i < row.n_more; ++i) {
-          const uint32_t e = __ldg(more + row.more + i), k = e >> 8, q = e & 0xFFu;
-          const uint32_t c0 = __ldg(r0 + k), c1 = __ldg(r1 + k);
-          d0 += q > c0 ? q - c0 : 0u;
-          d1 += q > c1 ? q - c1 : 0u;
+        const bool in0 = live && a0 && d0 <= T, in1 = live && a1 && d1 <= T;
+        word |= (in0 ? 1u << b0 : 0u) | (in1 ? 1u << b1 : 0u);
+        const uint32_t c0 = __ballot_sync(dev::FULL, in0), c1 = __ballot_sync(dev::FULL, in1);
+        if (cols && rl == 0) {
+          if (a0) cols[(vb + b0) * W + g.word] = ((c0 >> lane) & mine) << g.shift;
+          if (a1) cols[(vb + b1) * W + g.word] = ((c1 >> lane) & mine) << g.shift;
         }
-        word |= (d0 <= T ? 1u << b0 : 0u) | (d1 <= T ? 1u << b1 : 0u);
       }
       n += __popc(word);
       turn[warp][rl][t0 + sub] = word;
@@ -92,39 +104,37 @@ __global__ void __launch_bounds__(256) filter_kernel(const uint32_t *__restrict_
     for (uint32_t o = R; o < 32; o <<= 1) n += __shfl_xor_sync(dev::FULL, n, o);
     if (have && sub == 0) cnt[(uint64_t)row.row * nsets + set] = n;
     __syncwarp();
-    for (uint32_t r = lane / TS; r < ((R + 32 / TS - 1) / (32 / TS)) * (32 / TS); r += 32 / TS) {
+    constexpr uint32_t RP = 32 / TS;  // rows per store
+    for (uint32_t r0 = 0; r0 < g.n; r0 += RP) {
+      const uint32_t r = r0 + lane / TS, w = set * TS + lane % TS;
       const uint32_t rr = __shfl_sync(dev::FULL, row.row, r & 31u);
-      const bool ok = __shfl_sync(dev::FULL, (int)have, r & 31u) && r < R;
-      const uint32_t w = set * TS + lane % TS;
-      if (ok && w < nwords) bits[(uint64_t)rr * nwords + w] = turn[warp][r][lane % TS];
+      if (r < g.n && w < nwords) bits[(uint64_t)rr * nwords + w] = turn[warp][r][lane % TS];
     }
     __syncwarp();  // the words are read before the next item's are written
   }
 }
 
-uint32_t filter_set_tiles(uint32_t nrows, uint32_t nwords) {
+uint32_t filter_set_tiles(uint32_t ngroups, uint32_t nwords) {
   // sets of 32 tiles (128-byte stores) once they make two warps per
   // scheduler, else sets of 8, so that a small graph's rows still spread
-  return (uint64_t)((nrows + 31) / 32) * ((nwords + 31) / 32) >= 148 * 8 ? 32u : 8u;
+  return (uint64_t)ngroups * ((nwords + 31) / 32) >= 148 * 8 ? 32u : 8u;
 }
 
 void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const FilterRow *rows,
-                   const uint32_t *more, uint32_t nrows, uint32_t threshold, uint32_t *bits, uint32_t *cnt,
-                   uint32_t nwords, cudaStream_t s) {
-  if (nwords == 0 || nrows == 0) return;
-  const uint32_t TS = filter_set_tiles(nrows, nwords);
-  uint32_t R = 1;  // rows per group: the wave's, rounded up to a power of two, at least the tiles side by side
-  while (R < 32 && (R < nrows || 32 / R > TS)) R <<= 1;
-  const uint64_t items = (uint64_t)((nrows + R - 1) / R) * ((nwords + TS - 1) / TS);
+                   const uint32_t *more, const FilterGroup *groups, uint32_t ngroups, uint32_t TS, uint32_t threshold,
+                   uint32_t *bits, uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords,
+                   cudaStream_t s) {
+  if (nwords == 0 || ngroups == 0) return;
+  const uint64_t items = (uint64_t)ngroups * ((nwords + TS - 1) / TS);
   uint64_t blocks = (items + 7) / 8;
   if (blocks > 148ull * 48) blocks = 148ull * 48;
   count_launch();
   if (TS == 32)
-    filter_kernel<32><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, nrows, R, threshold,
-                                                       nwords, bits, cnt);
+    filter_kernel<32><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, groups, ngroups,
+                                                       threshold, nwords, bits, cnt, cols, W);
   else
-    filter_kernel<8><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, nrows, R, threshold,
-                                                      nwords, bits, cnt);
+    filter_kernel<8><<<(uint32_t)blocks, 256, 0, s>>>(g.lab, g.nv, nlc, stride, rows, more, groups, ngroups,
+                                                      threshold, nwords, bits, cnt, cols, W);
 }
 
 // One warp per 32 words of a row: their ranks into the rank words, their
@@ -163,14 +173,14 @@ __global__ void __launch_bounds__(256) rank_rows_kernel(const uint32_t *__restri
   }
 }
 
-void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint64_t *rb,
-                      uint32_t *cand, cudaStream_t s) {
+void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint32_t TS,
+                      uint64_t *rb, uint32_t *cand, cudaStream_t s) {
   const uint64_t items = (uint64_t)nrows * ((nwords + 31) / 32);
   if (items == 0) return;
   uint64_t blocks = (items + 7) / 8;
   if (blocks > 148ull * 64) blocks = 148ull * 64;
   count_launch();
-  rank_rows_kernel<<<(uint32_t)blocks, 256, 0, s>>>(bits, nrows, nwords, ex, filter_set_tiles(nrows, nwords), rb, cand);
+  rank_rows_kernel<<<(uint32_t)blocks, 256, 0, s>>>(bits, nrows, nwords, ex, TS, rb, cand);
 }
 
 // Compaction of bit rows kept in the low halves of rank words

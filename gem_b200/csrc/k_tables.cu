@@ -60,50 +60,38 @@ void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nk
   source_tile_bases_kernel<<<(nsrc + 256) / 256, 256, 0, s>>>(d_src, nsrc, nkeys, tp, out);
 }
 
-// Membership columns: out[v * W + c] holds, in bit b, whether vertex v is in
-// row rows[32c + b] (bits: the wave's membership bit rows, 32 vertices per
-// word).  One block per 32-vertex word j: each warp transposes 32 rows x 32
-// vertices with 32 ballots.  With vtiles, vtiles[v] = ceil(deg(v) / 32) for a
-// vertex in at least one of the rows, else 0.
-__global__ void __launch_bounds__(256) row_columns_kernel(const uint32_t *__restrict__ bits, uint32_t nwords,
-                                                          const uint32_t *__restrict__ rows, uint32_t nrows,
-                                                          uint32_t W, uint32_t nv, uint32_t *__restrict__ out,
-                                                          uint32_t *__restrict__ vtiles,
-                                                          const uint32_t *__restrict__ deg) {
-  __shared__ uint32_t any[32];
-  const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
-  for (uint32_t j = blockIdx.x; j < nwords; j += gridDim.x) {
-    if (threadIdx.x < 32) any[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t v = j * 32u + lane;
-    uint32_t seen = 0;
-    for (uint32_t c = warp; c < W; c += blockDim.x >> 5) {
-      const uint32_t r = c * 32u + lane;
-      const uint32_t word = r < nrows ? __ldg(bits + (uint64_t)__ldg(rows + r) * nwords + j) : 0u;
-      uint32_t col = 0;
-#pragma unroll
-      for (uint32_t b = 0; b < 32; ++b) {
-        const uint32_t m = __ballot_sync(dev::FULL, (word >> b) & 1u);
-        if (lane == b) col = m;
-      }
-      if (v < nv) out[(uint64_t)v * W + c] = col;
-      seen |= col;
-    }
-    if (vtiles) {
-      if (seen) atomicOr(any + lane, 1u);
-      __syncthreads();
-      if (warp == 0 && v < nv) vtiles[v] = any[lane] ? (__ldg(deg + v) + 31u) >> 5 : 0u;
-    }
-    __syncthreads();  // any[] is reset by the next word
+// The wave's label that v has (binary search), or none (words = 0).
+__device__ __forceinline__ RowLabel find_label(const RowLabel *__restrict__ labels, uint32_t n, uint32_t lab) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(&labels[mid].lab) < lab) lo = mid + 1; else hi = mid;
+  }
+  if (lo < n) {
+    const RowLabel r = labels[lo];
+    if (r.lab == lab) return r;
+  }
+  return RowLabel{lab, 0, 0, 0};
+}
+
+__global__ void vertex_tiles_kernel(DevGraph g, const RowLabel *__restrict__ labels, uint32_t nlab,
+                                    const uint32_t *__restrict__ cols, uint32_t W,
+                                    const uint32_t *__restrict__ smask, uint32_t *__restrict__ vtiles) {
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.nv; v += (uint64_t)gridDim.x * blockDim.x) {
+    const RowLabel l = nlab ? find_label(labels, nlab, __ldg(g.lab + v)) : RowLabel{0, 0, 1, 0};
+    uint32_t any = 0;
+    for (uint32_t c = 0; c < l.words && !any; ++c) any = __ldg(cols + v * W + c) & __ldg(smask + l.word0 + c);
+    vtiles[v] = any ? (__ldg(g.deg + v) + 31u) >> 5 : 0u;
   }
 }
 
-void launch_row_columns(const uint32_t *bits, uint32_t nwords, const uint32_t *rows, uint32_t nrows, uint32_t W,
-                        uint32_t nv, uint32_t *out, uint32_t *vtiles, const uint32_t *deg, cudaStream_t s) {
-  if (nwords == 0) return;
-  uint32_t blocks = nwords < 148u * 16 ? nwords : 148u * 16;
+void launch_vertex_tiles(const DevGraph &g, const RowLabel *labels, uint32_t nlab, const uint32_t *cols, uint32_t W,
+                         const uint32_t *smask, uint32_t *vtiles, cudaStream_t s) {
+  if (g.nv == 0) return;
+  uint32_t blocks = (g.nv + 255) / 256;
+  if (blocks > 148u * 32) blocks = 148u * 32;
   count_launch();
-  row_columns_kernel<<<blocks, 256, 0, s>>>(bits, nwords, rows, nrows, W, nv, out, vtiles, deg);
+  vertex_tiles_kernel<<<blocks, 256, 0, s>>>(g, labels, nlab, cols, W, smask, vtiles);
 }
 
 // vt[t] = v for every tile t in [vtp[v], vtp[v + 1]).
@@ -160,9 +148,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // position of v (rank bitmap) and tile index (tp).  The tables of those
 // sources are then flattened into (source, table) pairs, again one per
 // lane, 32 at a time:
-//   count: each lane tests its table's target column bit (tcol) for the 32
-//          arcs of the tile (the warp stages the arcs' target columns in
-//          shared memory, one column per arc) and writes the tile's mask;
+//   count: each lane tests its table's target column bit (tcol) for the
+//          arcs of the tile whose target has the target row's label (a few
+//          of the 32; the warp stages the arcs' columns in shared memory) and
+//          writes the tile's mask;
 //   write: each lane reads its pair's mask and value position into a
 //          per-warp record (records of empty masks dropped); then for each
 //          record the lanes, one per arc, write the arcs whose bit is set
@@ -171,69 +160,91 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // The mask and value positions are those of the source's own tile order
 // (mask[tile_base + lt], lt = the tile's index among the source's tiles), so
 // both passes lay out every table exactly as a pass over the sources would.
-constexpr uint32_t TAB_GRAB = 1;  // units a warp takes from the counter at a time (1: the narrowest window)
-
 struct VRec {
   uint64_t vb;  // first value position of the pair's tile
   uint32_t m;   // the tile's mask
   uint32_t kf;  // key position to record, or 0xFFFFFFFF (no key map)
 };
 
-template <bool WRITE>
+// ONE: waves of at most 32 rows (a plain query): one column word for all of
+// them, zero for other vertices, so an arc-lane holds its target's whole
+// column and a table's mask is one ballot; nothing is staged.
+//
+// A unit is a chain of dependent loads (counter, vertex, offsets, arcs,
+// columns, rank word, tile base), which bounds the passes of few rows; the
+// next unit's counter, vertex and offsets are fetched while this one's are
+// used (the count passes of four plain queries on the scale-22 graph: 2.55 ms
+// staged and without the prefetch, 2.10 ms).
+//
+// Columns hold a vertex's bits for the rows of its own label only: a few
+// words per vertex where one bit per target row of the wave was 80 words (320
+// bytes staged per arc) for 180 mixed-size queries, count pass 4.2 -> 1.0 ms.
+template <bool WRITE, bool ONE>
 __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   constexpr uint32_t G = WRITE ? TAB_WGROUP : 1u;  // tiles of one vertex per unit
-  extern __shared__ uint32_t stage[];  // count: 32 target columns per warp
+  extern __shared__ uint32_t stage[];  // count: 32 columns per warp
   __shared__ VRec rec[WRITE ? 8 : 1][32 * G];  // write: the records of one round
+  __shared__ uint32_t larcs[WRITE || ONE ? 1 : 8][NLC_MAX_LABELS];  // count: the tile's arcs to each label
   const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t *vmap = WRITE ? P.vg : P.vt;
+  const uint64_t *vfirst = WRITE ? P.vgp : P.vtp;
+  // units are taken in order from one counter, so the units in flight
+  // stay a narrow window of consecutive vertices
+  unsigned long long got = 0;
+  if (lane == 0) got = atomicAdd(P.next, 1ull);
+  uint64_t t = P.t0 + __shfl_sync(dev::FULL, got, 0);
+  if (t >= P.t1) return;
+  uint32_t v = __ldg(vmap + t);
+  uint64_t a0 = __ldg(P.off + v), a1 = __ldg(P.off + v + 1);
+  uint64_t c = (t - __ldg(vfirst + v)) * G;  // the unit: tiles c .. c + nt - 1 of vertex v
   for (;;) {
-    // units are taken in order from one counter, so the units in flight
-    // stay a narrow window of consecutive vertices
-    unsigned long long got = 0;
-    if (lane == 0) got = atomicAdd(P.next, (unsigned long long)TAB_GRAB);
-    const uint64_t t0 = P.t0 + __shfl_sync(dev::FULL, got, 0);
-    if (t0 >= P.t1) break;
-    const uint64_t t1 = t0 + TAB_GRAB < P.t1 ? t0 + TAB_GRAB : P.t1;
-    for (uint64_t t = t0; t < t1; ++t) {
-    // the unit: tiles c .. c + nt - 1 of vertex v
-    uint32_t v, nt = 1;
-    uint64_t c;
-    if (WRITE) {
-      v = __ldg(P.vg + t);
-      c = (t - __ldg(P.vgp + v)) * G;
-      const uint64_t tv = __ldg(P.vtp + v + 1) - __ldg(P.vtp + v);
-      nt = tv - c < G ? (uint32_t)(tv - c) : G;
-    } else {
-      v = __ldg(P.vt + t);
-      c = t - __ldg(P.vtp + v);
-    }
-    const uint64_t a0 = __ldg(P.off + v), a1 = __ldg(P.off + v + 1);
+    if (lane == 0) got = atomicAdd(P.next, 1ull);  // the next unit's number, looked at below
+    const uint64_t tiles = (a1 - a0 + 31) >> 5;
+    const uint32_t nt = tiles - c < G ? (uint32_t)(tiles - c) : G;
     uint32_t xs[G];
 #pragma unroll
     for (uint32_t i = 0; i < G; ++i) {
       const uint64_t arc = a0 + (c + i) * 32u + lane;
       xs[i] = i < nt && arc < a1 ? __ldg(P.nbr + (arc - P.arc_shift)) : 0u;
     }
-    const bool valid = a0 + c * 32u + lane < a1;  // lane's arc of the unit's first tile
     const uint32_t nvalid = a1 - a0 - c * 32u < 32u ? (uint32_t)(a1 - a0 - c * 32u) : 32u;  // valid lanes: a prefix
+    const RowLabel vl = ONE ? RowLabel{0, 0, 1, 0} : find_label(P.labels, P.nlab, __ldg(P.lab + v));
+    uint32_t *wst = stage + (uint64_t)warp * 32u * P.W;
+    uint32_t xl = 0xFFFFFFFFu, xc = 0;
     const uint32_t x = xs[0];
-    if (!WRITE) {
-      // stage the target columns of the tile's arcs with asynchronous 16-byte
-      // copies (all in flight at once): lane = (row in group, 16-byte chunk)
+    if (!WRITE && ONE) {
+      if (lane < nvalid) xc = __ldg(P.cols + x);
+    } else if (!WRITE) {
+      // stage the columns of the tile's arcs, with asynchronous 16-byte copies
+      // (all in flight at once) when they are whole 16-byte chunks
+      if (lane < nvalid) xl = __ldg(P.lab + x);
       __syncwarp();  // the previous tile's reads of the stage are done
-      const uint32_t ch = P.WT >> 2, rpi = 32u / ch;  // chunks per column, columns per round
-      const uint32_t r = lane / ch, q = lane - r * ch;
-      uint32_t *wst = stage + (uint64_t)warp * 32u * P.WTp;
-      for (uint32_t g = 0; g < nvalid; g += rpi) {
-        const uint32_t l = g + r;
-        const uint32_t xl = __shfl_sync(dev::FULL, x, l < 32u ? l : 0u);
-        if (r < rpi && l < nvalid) cp_async16(wst + l * P.WTp + q * 4u, P.B + (uint64_t)xl * P.WT + q * 4u);
+      if (P.W >= 4) {
+        const uint32_t ch = P.W >> 2;  // chunks per column
+        for (uint32_t g = lane; g < ((nvalid * ch + 31u) & ~31u); g += 32) {
+          const uint32_t l = g / ch, q = g - l * ch;
+          const uint32_t xa = __shfl_sync(dev::FULL, x, l & 31u);
+          if (l < nvalid) cp_async16(wst + l * P.W + q * 4u, P.cols + (uint64_t)xa * P.W + q * 4u);
+        }
+      } else if (lane < nvalid) {
+        for (uint32_t q = 0; q < P.W; ++q) wst[lane * P.W + q] = __ldg(P.cols + (uint64_t)x * P.W + q);
+      }
+      if (P.nlabels <= NLC_MAX_LABELS) {
+#pragma unroll
+        for (uint32_t l = 0; l < NLC_MAX_LABELS; l += 32) larcs[warp][l + lane] = 0;
+        __syncwarp();
+        const uint32_t peers = __match_any_sync(dev::FULL, xl);
+        if (lane < nvalid && lane == (uint32_t)__ffs(peers) - 1) larcs[warp][xl] = peers;
       }
       cp_async_wait_all();
       __syncwarp();
     }
-    const uint32_t *sv = P.S + (uint64_t)v * P.WS;
-    for (uint32_t wb = 0; wb < P.WS; wb += 32) {
-      const uint32_t word = wb + lane < P.WS ? __ldg(sv + wb + lane) : 0u;
+    const uint64_t tn = P.t0 + __shfl_sync(dev::FULL, got, 0);
+    uint32_t vn = 0;
+    if (tn < P.t1) vn = __ldg(vmap + tn);
+    const uint32_t *sv = P.cols + (uint64_t)v * P.W;
+    for (uint32_t wb = 0; wb < vl.words; wb += 32) {
+      const uint32_t word = wb + lane < vl.words ? __ldg(sv + wb + lane) & __ldg(P.smask + vl.word0 + wb + lane) : 0u;
       const uint32_t cnt = __popc(word);
       uint32_t incl = cnt;
 #pragma unroll
@@ -255,7 +266,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
         uint32_t k = 0, e0 = 0, ne = 0;
         uint64_t lt = 0;
         if (q < total) {
-          const VSrc &src = P.vsrc[(wb + j) * 32u + dev::nth_set_bit(wj, q - exj)];
+          const VSrc &src = P.vsrc[(vl.word0 + wb + j) * 32u + dev::nth_set_bit(wj, q - exj)];
           const uint64_t rw = __ldg(src.rb + (v >> 5));
           k = (uint32_t)(rw >> 32) + __popc((uint32_t)rw & ((1u << (v & 31u)) - 1u));
           lt = __ldg(P.tp + src.key_base + k) - src.stb + c;
@@ -284,14 +295,36 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
           const VEdge E = have ? P.vedge[pe] : VEdge{0, 0, 0};
           const uint64_t maddr = E.tile_base + plt;
           if (!WRITE) {
-            const uint32_t *col = stage + (uint64_t)warp * 32u * P.WTp + (E.tcol >> 5);
-            const uint32_t sh = E.tcol & 31u, st = P.WTp;
-            uint32_t m = 0, l = 0;
-            for (; l + 4 <= nvalid; l += 4) {
-              const uint32_t w0 = col[l * st], w1 = col[(l + 1) * st], w2 = col[(l + 2) * st], w3 = col[(l + 3) * st];
-              m |= (((w0 >> sh) & 1u) | (((w1 >> sh) & 1u) << 1) | (((w2 >> sh) & 1u) << 2) | (((w3 >> sh) & 1u) << 3)) << l;
+            uint32_t m = 0;
+            if (ONE) {  // one ballot per pair
+              const uint32_t np = npairs - pb < 32u ? npairs - pb : 32u;
+              for (uint32_t i = 0; i < np; ++i) {
+                const uint32_t bal = __ballot_sync(dev::FULL, (xc >> (__shfl_sync(dev::FULL, E.tcol, i) & 31u)) & 1u);
+                if (lane == i) m = bal;
+              }
+            } else {
+              // the tile's arcs whose target has the pair's target label
+              uint32_t am = 0;
+              if (P.nlabels <= NLC_MAX_LABELS) {
+                am = larcs[warp][E.tlab & (NLC_MAX_LABELS - 1)];
+              } else {  // one ballot per distinct label among them
+                for (uint32_t left = nvalid == 32u ? dev::FULL : (1u << nvalid) - 1u; left;) {
+                  const uint32_t ll = __shfl_sync(dev::FULL, xl, __ffs(left) - 1);
+                  const uint32_t bal = __ballot_sync(dev::FULL, xl == ll) & left;
+                  if (ll == E.tlab) am = bal;
+                  left &= ~bal;
+                }
+              }
+              const uint32_t *col = wst + ((E.tcol & 0x7FFFFFFFu) >> 5);
+              const uint32_t sh = E.tcol & 31u;
+              while (am) {  // two arcs a step
+                const uint32_t l0 = __ffs(am) - 1;
+                am &= am - 1;
+                const uint32_t l1 = am ? __ffs(am) - 1 : l0;
+                am &= am - 1;
+                m |= ((col[l0 * P.W] >> sh) & 1u) << l0 | ((col[l1 * P.W] >> sh) & 1u) << l1;
+              }
             }
-            for (; l < nvalid; ++l) m |= ((col[l * st] >> sh) & 1u) << l;
             if (have) P.mask[maddr] = m;
           } else {
             // records of the pair's tiles that have values, packed to the
@@ -299,7 +332,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
             // the value position.  A key's tiles are consecutive in its
             // source's tile order, so the unit's masks and positions are
             // consecutive words.
-            const uint32_t kf = have && P.vkey && (E.flags & TAB_KEY_MAP) ? pk : 0xFFFFFFFFu;
+            const uint32_t kf = have && P.vkey && (E.tcol >> 31) ? pk : 0xFFFFFFFFu;
             const uint32_t below = (1u << lane) - 1u;
             uint32_t m[G];
             uint64_t vb[G];
@@ -333,21 +366,23 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
         }
       }
     }
-    }
+    if (tn >= P.t1) return;
+    v = vn;
+    a0 = __ldg(P.off + v);
+    a1 = __ldg(P.off + v + 1);
+    c = (tn - __ldg(vfirst + v)) * G;
   }
 }
 
-// Warps per block of the count pass: each warp stages 32 target columns of
-// WTp words; blocks stay within 96 KB of shared memory so that two fit an SM.
-static uint32_t count_warps(uint32_t WTp) {
-  const uint64_t per_warp = 32ull * WTp * 4;
+// Warps per block of the count pass: each warp stages 32 columns of W words;
+// blocks stay within 96 KB of shared memory so that two fit an SM.
+static uint32_t count_warps(uint32_t W) {
+  const uint64_t per_warp = 32ull * W * 4;
   const uint64_t w = (96ull << 10) / per_warp;
   return w > 8 ? 8u : w < 1 ? 1u : (uint32_t)w;
 }
 
-// Target columns are staged in 16-byte chunks, at most one per lane per
-// column: WT (a multiple of 4) words up to 128.
-bool table_vtx_fits(uint32_t WT) { return WT % 4 == 0 && WT >= 4 && WT <= 128; }
+bool table_vtx_fits(uint32_t W) { return W == 1 || W == 2 || (W % 4 == 0 && W <= 128); }
 
 // Persistent grid: what the SMs hold at once (blocks per SM by occupancy).
 // Its warps take tiles in order from the launch's counter, so the tiles in
@@ -367,20 +402,25 @@ static uint32_t resident_blocks(const void *fn, int threads, size_t smem, uint64
 
 void launch_table_vtx(const VPass &P0, bool write, cudaStream_t s) {
   if (P0.t1 <= P0.t0) return;
-  VPass P = P0;
-  P.WTp = P.WT;  // the lanes of a pair round read one staged column each: no stride padding
-  const uint32_t warps = write ? 8u : count_warps(P.WTp);
+  const VPass &P = P0;
+  const uint32_t warps = write || P.nlab == 0 ? 8u : count_warps(P.W);
   const uint64_t want = (P.t1 - P.t0 + warps - 1) / warps;
   cudaMemsetAsync(P.next, 0, sizeof(unsigned long long), s);
   count_launch();
-  if (write) {
-    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<true>, 256, 0, want);
-    table_vtx_kernel<true><<<blocks, 256, 0, s>>>(P);
+  if (P.nlab == 0) {
+    if (write) {
+      table_vtx_kernel<true, true><<<resident_blocks((const void *)table_vtx_kernel<true, true>, 256, 0, want), 256, 0, s>>>(P);
+    } else {
+      table_vtx_kernel<false, true><<<resident_blocks((const void *)table_vtx_kernel<false, true>, 256, 0, want), 256, 0, s>>>(P);
+    }
+  } else if (write) {
+    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<true, false>, 256, 0, want);
+    table_vtx_kernel<true, false><<<blocks, 256, 0, s>>>(P);
   } else {
-    const size_t smem = (size_t)warps * 32 * P.WTp * 4;
-    cudaFuncSetAttribute(table_vtx_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<false>, (int)warps * 32, smem, want);
-    table_vtx_kernel<false><<<blocks, warps * 32, smem, s>>>(P);
+    const size_t smem = (size_t)warps * 32 * P.W * 4;
+    cudaFuncSetAttribute(table_vtx_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<false, false>, (int)warps * 32, smem, want);
+    table_vtx_kernel<false, false><<<blocks, warps * 32, smem, s>>>(P);
   }
 }
 

@@ -96,30 +96,39 @@ struct FilterDesc {          // one query (gem_filter_static)
   uint8_t nlc[QV][QV];       // nlc[u][k]: neighbours of u with label ql[k]
 };
 
-// A row of a wave's filter: candidates have label `lab` and, over the needs
-// (label-count column << 8 | neighbours wanted, 0 = unused), a deficit of at
-// most the threshold; `need` is the deficit that no vertex can make up
+// A row of a wave's filter: candidates have the row's label and, over the
+// needs (label-count column << 8 | neighbours wanted, 0 = unused), a deficit
+// of at most the threshold; `need` is the deficit that no vertex can make up
 // (neighbour labels that the graph lacks; above the threshold: no candidates).
 constexpr uint32_t FILTER_NEEDS = 4;
 struct FilterRow {
-  uint32_t lab;
   uint32_t row;              // row index of the outputs
   uint32_t need;
   uint32_t more, n_more;     // the needs after the first FILTER_NEEDS, in the wave's list of them
   uint32_t needs[FILTER_NEEDS];
 };
+// Up to 32 rows of one label: n rows from FilterRow row0 on.  A label's
+// rows, in groups, are the bits of its vertices' membership columns: this
+// group's are those of column word `word`.
+struct FilterGroup {
+  uint32_t lab;
+  uint32_t row0, n;
+  uint32_t word, shift;      // the group's column word, and its first bit there
+};
 // Vertex tiles per filter item (the granularity of its counts).
-uint32_t filter_set_tiles(uint32_t nrows, uint32_t nwords);
-// Candidate words of every row, bits[row * nwords + word], and the
-// candidates of every set of filter_set_tiles words, cnt[row * sets + set].
-// rows sorted by label; nlc: label counts of every vertex, stride bytes each.
+uint32_t filter_set_tiles(uint32_t ngroups, uint32_t nwords);
+// Candidate words of every row, bits[row * nwords + word]; the candidates of
+// every set of TS (8 or 32) words, cnt[row * sets + set]; and (optional) the
+// membership columns, cols[v * W + word], of every vertex with a row's label.
+// nlc: label counts of every vertex, stride bytes each.
 void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const FilterRow *rows,
-                   const uint32_t *more, uint32_t nrows, uint32_t threshold, uint32_t *bits, uint32_t *cnt,
-                   uint32_t nwords, cudaStream_t s);
+                   const uint32_t *more, const FilterGroup *groups, uint32_t ngroups, uint32_t TS, uint32_t threshold,
+                   uint32_t *bits, uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords,
+                   cudaStream_t s);
 // Rank words (members before the word << 32 | the word) and the sorted
 // candidate lists back to back, given ex = exclusive scan of cnt.
-void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint64_t *rb,
-                      uint32_t *cand, cudaStream_t s);
+void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint32_t TS,
+                      uint64_t *rb, uint32_t *cand, cudaStream_t s);
 // Given ex = exclusive scan of popcounts over all rows, writes the per-word
 // ranks into the high halves of rb and the sorted candidate lists
 // cand[c_base[row] ...].
@@ -138,8 +147,8 @@ struct TabSource {           // a (query, query vertex) whose candidates are tab
 struct TabEdge {             // a directed table T(u -> w)
   uint32_t src;              // index into TabSource
   uint32_t flags;            // TAB_KEY_MAP: the write pass also records each value's key position
-  uint32_t tcol;             // the target row's bit in the target membership columns
-  uint32_t pad;
+  uint32_t tcol;             // the target row's bit in its label's membership columns
+  uint32_t tlab;             // the target row's label
   uint64_t tile_base;        // first tile of this edge in the flattened edge-tile space
   uint64_t ntiles;
   uint64_t off_base;         // first entry of this edge in the flattened offsets space
@@ -148,11 +157,17 @@ struct TabEdge {             // a directed table T(u -> w)
 // tiles[k] = ceil(deg(key k) / 32) over the flattened key space.
 void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, uint64_t nkeys,
                       uint32_t *tiles, cudaStream_t s);
-// Membership columns of a list of rows: out[v * W + c] bit b = v is in row
-// rows[32c + b] (bits: membership bit rows, nwords u32 words per row).  With
-// vtiles, vtiles[v] = ceil(deg(v) / 32) for a vertex in any of the rows, else 0.
-void launch_row_columns(const uint32_t *bits, uint32_t nwords, const uint32_t *rows, uint32_t nrows, uint32_t W,
-                        uint32_t nv, uint32_t *out, uint32_t *vtiles, const uint32_t *deg, cudaStream_t s);
+// A label of the wave's rows: its rows are the column bits 32 word0 .. of the
+// wave's row positions, `words` column words per vertex of the label.
+struct RowLabel {
+  uint32_t lab, word0, words, pad;
+};
+// vtiles[v] = ceil(deg(v) / 32) for a vertex that some source holds (columns
+// & source masks), else 0.  labels: the wave's labels, sorted, or none (nlab
+// = 0): one column word for all rows, zero for vertices of other labels.
+// smask: bit b of word w = the row at position 32 w + b is a source.
+void launch_vertex_tiles(const DevGraph &g, const RowLabel *labels, uint32_t nlab, const uint32_t *cols, uint32_t W,
+                         const uint32_t *smask, uint32_t *vtiles, cudaStream_t s);
 // vt[t] = v for every vertex tile t in [vtp[v], vtp[v + 1]).
 void launch_vertex_tile_map(const uint64_t *vtp, uint32_t nv, uint32_t *vt, cudaStream_t s);
 // Write-pass units: out[v] = ceil(vtiles[v] / TAB_WGROUP).
@@ -168,14 +183,15 @@ struct VSrc {                // a table source as the vertex-tile passes see it
 };
 struct VEdge {
   uint64_t tile_base;
-  uint32_t tcol;
-  uint32_t flags;
+  uint32_t tlab;             // the target row's label
+  uint32_t tcol;             // its bit in that label's columns | TAB_KEY_MAP << 31
 };
 // One table pass over units [t0, t1): the count pass's units are vertex
 // tiles (vt: tile -> vertex, vtp: first tile of each vertex), the write
-// pass's up to TAB_WGROUP consecutive tiles of one vertex (vg, vgp).  Arcs are read at nbr[arc - arc_shift], with off the
-// device offsets of the data graph.  S: the source membership columns (WS
-// words per vertex), B: the target membership columns (WT words per vertex).
+// pass's up to TAB_WGROUP consecutive tiles of one vertex (vg, vgp).  Arcs
+// are read at nbr[arc - arc_shift], with off the device offsets of the data
+// graph.  cols: the filter's membership columns (W words per vertex), a
+// vertex's sources the bits of its columns & smask, vsrc by row position.
 // count: mask[edge.tile_base + lt] = the 32-bit membership mask of tile lt of
 // the edge's source; write: the values (and key positions) at vp.
 struct VPass {
@@ -187,12 +203,13 @@ struct VPass {
   const uint64_t *vtp;
   const uint32_t *vg;        // write pass: unit -> vertex (units of up to 4 tiles of one vertex)
   const uint64_t *vgp;       // first unit of each vertex
-  const uint32_t *S;
-  uint32_t WS;
-  uint32_t WT;
-  uint32_t WTp;              // set by the launcher
-  uint32_t pad;
-  const uint32_t *B;
+  const uint32_t *lab;
+  const RowLabel *labels;    // the wave's labels, sorted (nlab = 0: one column word for all rows)
+  uint32_t nlabels;          // the graph's
+  uint32_t nlab;
+  uint32_t W;
+  const uint32_t *cols;
+  const uint32_t *smask;
   const VSrc *vsrc;
   const VEdge *vedge;
   const uint64_t *tp;
@@ -203,9 +220,9 @@ struct VPass {
   unsigned long long *next;  // tile counter of the launch (zeroed by the launcher)
 };
 void launch_table_vtx(const VPass &P, bool write, cudaStream_t s);
-// Whether the count pass can stage WT-word target columns (WT a multiple of
-// 4, at most 128: 4,096 target rows).
-bool table_vtx_fits(uint32_t WT);
+// Whether the count pass can stage W-word columns (1, 2 or a multiple of 4
+// words, at most 128: 4,096 rows of one label).
+bool table_vtx_fits(uint32_t W);
 // out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys].
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
                               uint64_t *out, cudaStream_t s);

@@ -1,0 +1,119 @@
+"""Kernels at the sizes where they can go wrong, bit-exact against the CPU
+oracle or a closed form: filter rows on graphs of ragged size and of more
+labels than the resident label counts cover, membership columns of every
+width, hash buckets that overflow, pair items and pair pools of odd lengths,
+scans on both sides of the one-block limit."""
+import math
+
+import numpy as np
+import pytest
+
+import gem_b200 as gem
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def cut(g, n):
+    """The subgraph that the first n vertices induce."""
+    off, nbr, lab = g.arrays()
+    src = np.repeat(np.arange(g.nv), np.diff(off).astype(np.int64))
+    keep = (src < n) & (nbr < n)
+    new = np.zeros(n + 1, np.uint64)
+    np.cumsum(np.bincount(src[keep], minlength=n), out=new[1:])
+    return gem.HostGraph.from_csr(new, nbr[keep], lab[:n])
+
+
+# one row to a full group of them, one tile to several sets, few labels to more than 64 (counted per wave)
+@pytest.mark.parametrize("nv", [9, 31, 33, 257, 1023, 4096 - 7])
+@pytest.mark.parametrize("labels", [1, 3, 23, 64, 65, 150])
+def test_filter_rows(nv, labels):
+    g = cut(gem.HostGraph.rmat(12, 8, seed=91), nv).set_labels(labels, 0.0, seed=7)
+    rng = np.random.default_rng(nv + labels)
+    lab = g.arrays()[2]
+    qs = [gem.Query([lab[0]], []), gem.Query([lab[0], labels + 5], [(0, 1)])]
+    for k in (2, 5, 32):  # random trees: any labels, among them ones that few vertices or none have
+        qs.append(gem.Query(rng.integers(0, labels + 1, k), [(int(rng.integers(0, i)), i) for i in range(1, k)]))
+    # a hub with eleven distinct neighbour labels: more needs than a row holds
+    qs.append(gem.Query([0] + [i % (labels + 1) for i in range(11)], [(0, i) for i in range(1, 12)]))
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        for q in qs:
+            for t in (0, 1, 2):
+                got, exp = c.filter(q, threshold=t), oracle.filter(g, q, threshold=t)
+                for u in range(q.nv):
+                    assert np.array_equal(got[u], exp[u]), (q.nv, t, u)
+
+
+# column widths: 1 word (one for all rows, then per label), 2, and multiples of 4; above 64 labels too
+@pytest.mark.parametrize("labels,n,k", [(3, 2, 4), (90, 40, 6), (40, 60, 6), (16, 120, 6), (5, 120, 6), (2, 60, 5)])
+def test_batch_columns(labels, n, k):
+    g = cut(gem.HostGraph.rmat(10, 6, seed=17), 1001).set_labels(labels, 0.0, seed=5)
+    qs = gem.gen_queries(g, k, gem.SPARSE, n, seed=labels)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        rs = c.batch(qs)[1]
+        rh = c.batch(qs, mode=gem.MODE_HASH)[1] if labels > 10 else None
+        for q, r in list(zip(qs, rs))[:2]:
+            cand = oracle.filter(g, q)
+            for a, b in q.edges.tolist():
+                for u, w in ((a, b), (b, a)):
+                    off, vals = c.edge_table(q, u, w)
+                    eo, ev = oracle.edge_table(g, cand[u], cand[w])
+                    assert np.array_equal(off, eo) and np.array_equal(vals, ev), (u, w)
+    checked = 0
+    for i, q in enumerate(qs):
+        cnt, h, ok = oracle.count(g, q, want_hash=rh is not None, work_cap=20_000_000)
+        if ok:
+            checked += 1
+            assert rs[i]["status"] == "OK" and rs[i]["count"] == cnt, i
+            if rh is not None:
+                assert rh[i]["count"] == cnt and rh[i]["emb_hash"] == h, i
+    assert checked >= n // 3
+
+
+# complete graphs: every neighbourhood hash holds n - 1 keys (one bucket upwards; overflows at every size), every
+# intersection is long, and the counts are falling factorials
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 9, 33, 70])
+def test_complete_graph_paths_and_cycles(n):
+    g = gem.HostGraph.from_edges(n, [(i, j) for i in range(n) for j in range(i + 1, n)], [0] * n)
+    shapes = [[(i, i + 1) for i in range(k - 1)] for k in (2, 3, 4, 5)]
+    shapes += [s + [(0, k - 1)] for s, k in zip(shapes[1:], (3, 4, 5))]
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        for e in shapes:
+            k = max(max(x) for x in e) + 1
+            q, exp = gem.Query([0] * k, e), math.perm(n, k)
+            assert c.run(q)["count"] == exp, (n, e)
+            if exp <= 20_000_000:
+                r = c.run(q, mode=gem.MODE_HASH)
+                assert r["status"] == "OK" and r["count"] == exp, (n, e)
+
+
+# a hub with d leaves, each with its own pendant: pair items and pools of d entries around the sizes of a warp's chunk
+@pytest.mark.parametrize("d", [1, 31, 32, 33, 64, 1000, 5000])
+def test_hub_and_spokes(d):
+    e = [(0, 1 + i) for i in range(d)] + [(1 + i, 1 + d + i) for i in range(d)]
+    g = gem.HostGraph.from_edges(1 + 2 * d, e, [0] + [1] * d + [2] * d)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        path5 = gem.Query([2, 1, 0, 1, 2], [(0, 1), (1, 2), (2, 3), (3, 4)])
+        star = gem.Query([0, 1, 1], [(0, 1), (0, 2)])
+        for q, exp in ((path5, d * (d - 1)), (star, d * (d - 1)), (gem.Query([0, 1, 2], [(0, 1), (1, 2)]), d)):
+            assert c.run(q)["count"] == exp
+            if exp < 3_000_000:
+                r = c.run(q, mode=gem.MODE_ENUMERATE, emb_cap=exp + 1)
+                assert r["count"] == r["n_written"] == exp
+                assert len(np.unique(r["embeddings"], axis=0)) == exp
+
+
+# the one-block scan's limit is 16,384 items: candidate sets, keys, vertex and table tiles on both sides of it
+@pytest.mark.parametrize("nv", [16383, 16384, 16385, 40000])
+def test_scan_limit(nv):
+    # a cycle: every vertex a candidate, one tile and two values per key
+    g = gem.HostGraph.from_edges(nv, [(i, (i + 1) % nv) for i in range(nv)], [0] * nv)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        assert c.run(gem.Query([0, 0, 0], [(0, 1), (1, 2)]))["count"] == 2 * nv
+        off, vals = c.edge_table(gem.Query([0, 0], [(0, 1)]), 0, 1)
+        assert np.array_equal(off, 2 * np.arange(nv + 1, dtype=np.uint64)) and len(vals) == 2 * nv
