@@ -1077,10 +1077,9 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   ST(aalloc(ctx, nkeys ? nkeys : 1, &d_tiles));
   ST(aalloc(ctx, nkeys + 1, &d_tp));
   ST(aalloc(ctx, scan_tmp_words(nkeys), &d_tmp));
-  ST(aalloc(ctx, src.size() + 3, &d_stb));
+  ST(aalloc(ctx, src.size() + 2, &d_stb));
   launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), nkeys, d_tiles, ctx->s);
   launch_scan(d_tiles, SCAN_U32, nkeys, d_tp, d_tmp, ctx->s);
-  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_stb, ctx->s);
   // Vertex tiles: the 32-arc tiles of every vertex that some source holds
   // (its membership column under the sources' bits); the table passes walk
   // those tiles once for all sources.
@@ -1089,29 +1088,23 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   for (uint32_t r : src_row) smask[w.row_pos[r] >> 5] |= 1u << (w.row_pos[r] & 31u);
   RowLabel *d_labels;
   uint32_t *d_smask, *d_vtiles;
-  uint64_t *d_vtp, *d_tmp3;
+  uint64_t *d_vtg, *d_tmp3;
+  unsigned long long *d_next;  // unit counters of the two passes
   ST(aalloc(ctx, w.labels.empty() ? 1 : w.labels.size(), &d_labels));
   CU(h2d(ctx, d_labels, w.labels.data(), w.labels.size() * sizeof(RowLabel)));
   ST(aalloc(ctx, smask.size(), &d_smask));
   CU(h2d(ctx, d_smask, smask.data(), 4 * smask.size()));
   ST(aalloc(ctx, nv ? nv : 1, &d_vtiles));
-  ST(aalloc(ctx, (uint64_t)nv + 1, &d_vtp));
+  ST(aalloc(ctx, (uint64_t)nv + 1, &d_vtg));
   ST(aalloc(ctx, scan_tmp_words(nv), &d_tmp3));
+  ST(aalloc(ctx, 2, &d_next));
   launch_vertex_tiles(ctx->g, d_labels, (uint32_t)w.labels.size(), w.d_cols, w.W, d_smask, d_vtiles, ctx->s);
-  launch_scan(d_vtiles, SCAN_U32, nv, d_vtp, d_tmp3, ctx->s);
-  // the write pass's units: up to TAB_WGROUP consecutive tiles of one vertex
-  uint32_t *d_vunits;
-  uint64_t *d_vgp;
-  ST(aalloc(ctx, nv ? nv : 1, &d_vunits));
-  ST(aalloc(ctx, (uint64_t)nv + 1, &d_vgp));
-  launch_unit_counts(d_vtiles, nv, d_vunits, ctx->s);
-  launch_scan(d_vunits, SCAN_U32, nv, d_vgp, d_tmp3, ctx->s);
-  CU(cudaMemcpyAsync(d_stb + src.size() + 1, d_vtp + nv, 8, cudaMemcpyDeviceToDevice, ctx->s));
-  CU(cudaMemcpyAsync(d_stb + src.size() + 2, d_vgp + nv, 8, cudaMemcpyDeviceToDevice, ctx->s));
-  std::vector<uint64_t> stb(src.size() + 3);
+  launch_scan(d_vtiles, SCAN_TILES, nv, d_vtg, d_tmp3, ctx->s);
+  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_vtg, nv, d_stb, d_next, ctx->s);
+  std::vector<uint64_t> stb(src.size() + 2);
   CU(d2h_sync(ctx, stb.data(), d_stb, 8 * stb.size()));
   CU(cudaGetLastError());
-  const uint64_t vtiles = stb[src.size() + 1], vunits = stb[src.size() + 2];
+  const uint64_t vtiles = (uint32_t)stb[src.size() + 1], vunits = stb[src.size() + 1] >> 32;
   // edges, grouped by source: a source's tables are one range of the edges
   struct EdgeReq {
     uint32_t s, qi, j, k;
@@ -1182,12 +1175,10 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     ctx->err = "too many filter rows of one label in one wave";
     return GEM_ERR_LIMIT;
   }
-  uint32_t *d_vt;
-  uint32_t *d_vg;
+  uint32_t *d_vt, *d_vg;
   ST(aalloc(ctx, vtiles ? vtiles : 1, &d_vt));
-  launch_vertex_tile_map(d_vtp, nv, d_vt, ctx->s);
   ST(aalloc(ctx, vunits ? vunits : 1, &d_vg));
-  launch_vertex_tile_map(d_vgp, nv, d_vg, ctx->s);
+  launch_vertex_maps(d_vtg, nv, d_vt, d_vg, ctx->s);
   std::vector<VSrc> vs(32 * (size_t)w.pos_words);
   for (size_t i = 0; i < src.size(); ++i)
     vs[w.row_pos[src_row[i]]] =
@@ -1210,13 +1201,14 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   bool streamed = false;
   if (ctx->opts.ooc && nparts && ctx->opts.ooc_stream != 2 && vtiles) {
     uint64_t *d_pb;
-    ST(aalloc(ctx, 2ull * (nparts + 1), &d_pb));
-    launch_gather_u64(d_vtp, ctx->d_part_v, nparts + 1, d_pb, ctx->s);
-    launch_gather_u64(d_vgp, ctx->d_part_v, nparts + 1, d_pb + nparts + 1, ctx->s);
-    std::vector<uint64_t> pb(2ull * (nparts + 1));
-    CU(d2h_sync(ctx, pb.data(), d_pb, 16ull * (nparts + 1)));
-    pstart.assign(pb.begin(), pb.begin() + nparts + 1);
-    pstart_w.assign(pb.begin() + nparts + 1, pb.end());
+    ST(aalloc(ctx, nparts + 1ull, &d_pb));
+    launch_gather_u64(d_vtg, ctx->d_part_v, nparts + 1, d_pb, ctx->s);
+    std::vector<uint64_t> pb(nparts + 1ull);
+    CU(d2h_sync(ctx, pb.data(), d_pb, 8ull * (nparts + 1)));
+    for (uint64_t x : pb) {
+      pstart.push_back((uint32_t)x);
+      pstart_w.push_back(x >> 32);
+    }
     uint64_t need = 0;
     for (uint32_t p = 0; p < nparts; ++p)
       if (pstart[p + 1] > pstart[p]) need += 4 * (ctx->part_a[p + 1] - ctx->part_a[p]);
@@ -1226,21 +1218,18 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // One table pass (count or write) over every vertex tile: in place, or
   // partition by partition with the copy of the next partition (side
   // stream, the other staging buffer) overlapping the kernel of the current one.
-  unsigned long long *d_next;
-  ST(aalloc(ctx, 1, &d_next));
   auto table_pass = [&](bool write) -> gem_status {
     VPass P;
     std::memset(&P, 0, sizeof P);
-    P.next = d_next;
+    P.next = d_next + write;
     P.off = ctx->g.off;
     P.nbr = ctx->g.nbr;
     P.arc_shift = 0;
     P.t0 = 0;
     P.t1 = write ? vunits : vtiles;
     P.vt = d_vt;
-    P.vtp = d_vtp;
     P.vg = d_vg;
-    P.vgp = d_vgp;
+    P.vtg = d_vtg;
     P.lab = ctx->g.lab;
     P.labels = d_labels;
     P.nlab = (uint32_t)w.labels.size();
@@ -1276,6 +1265,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
       P.arc_shift = a0;
       P.t0 = write ? pstart_w[p] : pstart[p];
       P.t1 = write ? pstart_w[p + 1] : pstart[p + 1];
+      CU(cudaMemsetAsync(P.next, 0, sizeof *P.next, ctx->s));
       launch_table_vtx(P, write, ctx->s);
       CU(cudaEventRecord(ctx->ev_free[b], ctx->s));
       ctx->ooc.parts_streamed += 1;

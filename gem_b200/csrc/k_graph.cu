@@ -229,6 +229,12 @@ __device__ __forceinline__ void scan_items(const void *in, uint64_t n, uint64_t 
   for (uint32_t j = 0; j < SCAN_I; ++j) v[j] = base + j < n ? scan_item<K>(in, base + j) : 0u;
 }
 
+// What an item adds to the sums.
+template <ScanInput K>
+__device__ __forceinline__ uint64_t scan_term(uint32_t v) {
+  return K == SCAN_TILES ? v | (uint64_t)((v + TAB_WGROUP - 1) / TAB_WGROUP) << 32 : v;
+}
+
 template <ScanInput K>
 __global__ void __launch_bounds__(SCAN_T) scan_partial_kernel(const void *in, uint64_t n, uint64_t *part) {
   const uint64_t base = (uint64_t)blockIdx.x * SCAN_B + (uint64_t)threadIdx.x * SCAN_I;
@@ -236,7 +242,7 @@ __global__ void __launch_bounds__(SCAN_T) scan_partial_kernel(const void *in, ui
   scan_items<K>(in, n, base, v);
   uint64_t s = 0;
 #pragma unroll
-  for (uint32_t j = 0; j < SCAN_I; ++j) s += v[j];
+  for (uint32_t j = 0; j < SCAN_I; ++j) s += scan_term<K>(v[j]);
   __shared__ uint64_t tot;
   (void)block_exclusive_scan(s, &tot);
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
@@ -290,14 +296,14 @@ __global__ void __launch_bounds__(SCAN_T) scan_final_kernel(const void *in, uint
   scan_items<K>(in, n, base, v);
   uint64_t s = 0;
 #pragma unroll
-  for (uint32_t j = 0; j < SCAN_I; ++j) s += v[j];
+  for (uint32_t j = 0; j < SCAN_I; ++j) s += scan_term<K>(v[j]);
   __shared__ uint64_t tot;
   uint64_t ex = block_exclusive_scan(s, &tot) + part[blockIdx.x];
   uint64_t o[SCAN_I];
 #pragma unroll
   for (uint32_t j = 0; j < SCAN_I; ++j) {
     o[j] = ex;
-    ex += v[j];
+    ex += scan_term<K>(v[j]);
   }
   if (base + SCAN_I <= n && ((uintptr_t)(out + base) & 15u) == 0) {
     ulonglong2 *q = (ulonglong2 *)(out + base);  // 16-byte stores
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(1024) scan_small_kernel(const void *in, uint64
     scan_items<K>(in, n, base, v);
     uint64_t x = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < SCAN_I; ++j) x += v[j];
+    for (uint32_t j = 0; j < SCAN_I; ++j) x += scan_term<K>(v[j]);
     uint64_t inc = x;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -348,7 +354,7 @@ __global__ void __launch_bounds__(1024) scan_small_kernel(const void *in, uint64
 #pragma unroll
     for (uint32_t j = 0; j < SCAN_I; ++j) {
       if (base + j < n) out[base + j] = ex;
-      ex += v[j];
+      ex += scan_term<K>(v[j]);
     }
   }
   if (threadIdx.x == 0) out[n] = carry;
@@ -397,6 +403,7 @@ void launch_scan(const void *in, ScanInput kind, uint64_t n, uint64_t *out, uint
   }
   switch (kind) {
     case SCAN_POPC_U64LO: scan_kind<SCAN_POPC_U64LO>(in, n, nb, out, tmp, s); break;
+    case SCAN_TILES: scan_kind<SCAN_TILES>(in, n, nb, out, tmp, s); break;
     case SCAN_POPC_U32: scan_kind<SCAN_POPC_U32>(in, n, nb, out, tmp, s); break;
     default: scan_kind<SCAN_U32>(in, n, nb, out, tmp, s); break;
   }

@@ -49,15 +49,20 @@ void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, 
 }
 
 __global__ void source_tile_bases_kernel(const TabSource *__restrict__ src, uint32_t nsrc, uint64_t nkeys,
-                                         const uint64_t *__restrict__ tp, uint64_t *__restrict__ out) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= nsrc; i += gridDim.x * blockDim.x)
-    out[i] = tp[i < nsrc ? src[i].key_base : nkeys];
+                                         const uint64_t *__restrict__ tp, const uint64_t *__restrict__ vtg,
+                                         uint32_t nv, uint64_t *__restrict__ out,
+                                         unsigned long long *__restrict__ counters) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2) counters[i] = 0;
+  if (i <= nsrc) out[i] = tp[i < nsrc ? src[i].key_base : nkeys];
+  if (i == nsrc + 1) out[i] = vtg[nv];
 }
 
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
-                              uint64_t *out, cudaStream_t s) {
+                              const uint64_t *vtg, uint32_t nv, uint64_t *out, unsigned long long *counters,
+                              cudaStream_t s) {
   count_launch();
-  source_tile_bases_kernel<<<(nsrc + 256) / 256, 256, 0, s>>>(d_src, nsrc, nkeys, tp, out);
+  source_tile_bases_kernel<<<(nsrc + 2 + 255) / 256, 256, 0, s>>>(d_src, nsrc, nkeys, tp, vtg, nv, out, counters);
 }
 
 // The wave's label that v has (binary search), or none (words = 0).
@@ -94,31 +99,41 @@ void launch_vertex_tiles(const DevGraph &g, const RowLabel *labels, uint32_t nla
   vertex_tiles_kernel<<<blocks, 256, 0, s>>>(g, labels, nlab, cols, W, smask, vtiles);
 }
 
-// vt[t] = v for every tile t in [vtp[v], vtp[v + 1]).
-__global__ void vertex_tile_map_kernel(const uint64_t *__restrict__ vtp, uint32_t nv, uint32_t *__restrict__ vt) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-    for (uint64_t t = __ldg(vtp + v), e = __ldg(vtp + v + 1); t < e; ++t) vt[t] = v;
+// map[i] = the vertex of the warp's 32 whose range holds i, for the warp's
+// whole range [b, e) of items; end: the lane's vertex's end.
+__device__ __forceinline__ void fill_map(uint32_t b, uint32_t e, uint32_t end, uint32_t v0, uint32_t *__restrict__ map) {
+  for (uint32_t i0 = b; i0 < e; i0 += 32) {
+    const uint32_t i = i0 + dev::lane_id();
+    uint32_t j = 0;  // the first lane whose end passes i
+#pragma unroll
+    for (uint32_t step = 16; step >= 1; step >>= 1)
+      if (__shfl_sync(dev::FULL, end, j + step - 1) <= i) j += step;
+    if (i < e) map[i] = v0 + j;
+  }
 }
 
-void launch_vertex_tile_map(const uint64_t *vtp, uint32_t nv, uint32_t *vt, cudaStream_t s) {
+// One warp per 32 vertices, whose tiles (and units) are one range: stores are
+// coalesced and a hub's thousands of tiles are 32 to a step (a thread per
+// vertex wrote them one by one, and the two maps apart).
+__global__ void __launch_bounds__(256) vertex_maps_kernel(const uint64_t *__restrict__ vtg, uint32_t nv,
+                                                          uint32_t *__restrict__ vt, uint32_t *__restrict__ vg) {
+  const uint32_t lane = dev::lane_id();
+  const uint64_t nwarps = (uint64_t)gridDim.x * 8;
+  for (uint64_t w = blockIdx.x * 8ull + (threadIdx.x >> 5); w * 32 < nv; w += nwarps) {
+    const uint64_t v = w * 32 + lane;
+    const uint64_t end = __ldg(vtg + (v < nv ? v + 1 : nv)), first = __ldg(vtg + w * 32);
+    const uint64_t last = __shfl_sync(dev::FULL, end, 31);
+    fill_map((uint32_t)first, (uint32_t)last, (uint32_t)end, (uint32_t)(w * 32), vt);
+    fill_map((uint32_t)(first >> 32), (uint32_t)(last >> 32), (uint32_t)(end >> 32), (uint32_t)(w * 32), vg);
+  }
+}
+
+void launch_vertex_maps(const uint64_t *vtg, uint32_t nv, uint32_t *vt, uint32_t *vg, cudaStream_t s) {
   if (nv == 0) return;
   uint32_t blocks = (nv + 255) / 256;
   if (blocks > 148u * 16) blocks = 148u * 16;
   count_launch();
-  vertex_tile_map_kernel<<<blocks, 256, 0, s>>>(vtp, nv, vt);
-}
-
-__global__ void unit_counts_kernel(const uint32_t *__restrict__ vtiles, uint32_t nv, uint32_t *__restrict__ out) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
-    out[v] = (__ldg(vtiles + v) + TAB_WGROUP - 1) / TAB_WGROUP;
-}
-
-void launch_unit_counts(const uint32_t *vtiles, uint32_t nv, uint32_t *out, cudaStream_t s) {
-  if (nv == 0) return;
-  uint32_t blocks = (nv + 255) / 256;
-  if (blocks > 148u * 16) blocks = 148u * 16;
-  count_launch();
-  unit_counts_kernel<<<blocks, 256, 0, s>>>(vtiles, nv, out);
+  vertex_maps_kernel<<<blocks, 256, 0, s>>>(vtg, nv, vt, vg);
 }
 
 __global__ void gather_u64_kernel(const uint64_t *__restrict__ a, const uint32_t *__restrict__ idx, uint32_t n,
@@ -187,7 +202,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   __shared__ uint32_t larcs[WRITE || ONE ? 1 : 8][NLC_MAX_LABELS];  // count: the tile's arcs to each label
   const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
   const uint32_t *vmap = WRITE ? P.vg : P.vt;
-  const uint64_t *vfirst = WRITE ? P.vgp : P.vtp;
+  constexpr uint32_t half = WRITE ? 32 : 0;  // a vertex's first unit in its word of vtg
   // units are taken in order from one counter, so the units in flight
   // stay a narrow window of consecutive vertices
   unsigned long long got = 0;
@@ -196,7 +211,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   if (t >= P.t1) return;
   uint32_t v = __ldg(vmap + t);
   uint64_t a0 = __ldg(P.off + v), a1 = __ldg(P.off + v + 1);
-  uint64_t c = (t - __ldg(vfirst + v)) * G;  // the unit: tiles c .. c + nt - 1 of vertex v
+  uint64_t c = (t - (uint32_t)(__ldg(P.vtg + v) >> half)) * G;  // the unit: tiles c .. c + nt - 1 of vertex v
   for (;;) {
     if (lane == 0) got = atomicAdd(P.next, 1ull);  // the next unit's number, looked at below
     const uint64_t tiles = (a1 - a0 + 31) >> 5;
@@ -370,7 +385,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
     v = vn;
     a0 = __ldg(P.off + v);
     a1 = __ldg(P.off + v + 1);
-    c = (tn - __ldg(vfirst + v)) * G;
+    c = (tn - (uint32_t)(__ldg(P.vtg + v) >> half)) * G;
   }
 }
 
@@ -405,7 +420,6 @@ void launch_table_vtx(const VPass &P0, bool write, cudaStream_t s) {
   const VPass &P = P0;
   const uint32_t warps = write || P.nlab == 0 ? 8u : count_warps(P.W);
   const uint64_t want = (P.t1 - P.t0 + warps - 1) / warps;
-  cudaMemsetAsync(P.next, 0, sizeof(unsigned long long), s);
   count_launch();
   if (P.nlab == 0) {
     if (write) {

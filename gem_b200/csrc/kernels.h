@@ -72,6 +72,7 @@ enum ScanInput : uint32_t {
   SCAN_POPC_U64LO = 0,  // popcount of the low 32 bits of a u64 word
   SCAN_POPC_U32 = 1,    // popcount of a u32 word
   SCAN_U32 = 2,         // plain u32 values
+  SCAN_TILES = 3,       // u32 vertex tiles t: two sums in one word, tiles | write units << 32 (TAB_WGROUP tiles each)
 };
 // out[i] = in[i * stride] for i < n.
 void launch_gather_strided(const uint64_t *in, uint64_t stride, uint32_t n, uint64_t *out, cudaStream_t s);
@@ -168,11 +169,11 @@ struct RowLabel {
 // smask: bit b of word w = the row at position 32 w + b is a source.
 void launch_vertex_tiles(const DevGraph &g, const RowLabel *labels, uint32_t nlab, const uint32_t *cols, uint32_t W,
                          const uint32_t *smask, uint32_t *vtiles, cudaStream_t s);
-// vt[t] = v for every vertex tile t in [vtp[v], vtp[v + 1]).
-void launch_vertex_tile_map(const uint64_t *vtp, uint32_t nv, uint32_t *vt, cudaStream_t s);
-// Write-pass units: out[v] = ceil(vtiles[v] / TAB_WGROUP).
+// The vertex of every vertex tile (vt) and of every write unit (vg): vtg is
+// the scan (SCAN_TILES) of the vertex tiles.  A write unit is up to
+// TAB_WGROUP consecutive tiles of one vertex.
 constexpr uint32_t TAB_WGROUP = 4;
-void launch_unit_counts(const uint32_t *vtiles, uint32_t nv, uint32_t *out, cudaStream_t s);
+void launch_vertex_maps(const uint64_t *vtg, uint32_t nv, uint32_t *vt, uint32_t *vg, cudaStream_t s);
 // out[i] = a[idx[i]].
 void launch_gather_u64(const uint64_t *a, const uint32_t *idx, uint32_t n, uint64_t *out, cudaStream_t s);
 struct VSrc {                // a table source as the vertex-tile passes see it
@@ -187,8 +188,8 @@ struct VEdge {
   uint32_t tcol;             // its bit in that label's columns | TAB_KEY_MAP << 31
 };
 // One table pass over units [t0, t1): the count pass's units are vertex
-// tiles (vt: tile -> vertex, vtp: first tile of each vertex), the write
-// pass's up to TAB_WGROUP consecutive tiles of one vertex (vg, vgp).  Arcs
+// tiles (vt: tile -> vertex), the write pass's up to TAB_WGROUP consecutive
+// tiles of one vertex (vg); vtg: the first tile and unit of each vertex.  Arcs
 // are read at nbr[arc - arc_shift], with off the device offsets of the data
 // graph.  cols: the filter's membership columns (W words per vertex), a
 // vertex's sources the bits of its columns & smask, vsrc by row position.
@@ -200,9 +201,8 @@ struct VPass {
   uint64_t arc_shift;
   uint64_t t0, t1;
   const uint32_t *vt;
-  const uint64_t *vtp;
-  const uint32_t *vg;        // write pass: unit -> vertex (units of up to 4 tiles of one vertex)
-  const uint64_t *vgp;       // first unit of each vertex
+  const uint32_t *vg;
+  const uint64_t *vtg;
   const uint32_t *lab;
   const RowLabel *labels;    // the wave's labels, sorted (nlab = 0: one column word for all rows)
   uint32_t nlabels;          // the graph's
@@ -217,15 +217,17 @@ struct VPass {
   const uint64_t *vp;
   uint32_t *values;
   uint32_t *vkey;
-  unsigned long long *next;  // tile counter of the launch (zeroed by the launcher)
+  unsigned long long *next;  // unit counter of the launch (zero at its start)
 };
 void launch_table_vtx(const VPass &P, bool write, cudaStream_t s);
 // Whether the count pass can stage W-word columns (1, 2 or a multiple of 4
 // words, at most 128: 4,096 rows of one label).
 bool table_vtx_fits(uint32_t W);
-// out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys].
+// out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys],
+// out[nsrc + 1] = vtg[nv]; zeroes the two counters.
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
-                              uint64_t *out, cudaStream_t s);
+                              const uint64_t *vtg, uint32_t nv, uint64_t *out, unsigned long long *counters,
+                              cudaStream_t s);
 // out[e] = vp[edges[e].tile_base] for e < nedge and out[nedge] = vp[tiles]:
 // the first value position of every table (and the total), so that table e
 // holds out[e + 1] - out[e] values.
