@@ -165,12 +165,11 @@ static gem_status aalloc(gem_ctx *ctx, uint64_t n, T **out) {
 static gem_status exec_init(gem_ctx *ctx) {
   CU(cudaStreamCreateWithFlags(&ctx->s, cudaStreamNonBlocking));
   for (auto &ev : ctx->ev) CU(cudaEventCreate(&ev));
-  CU(cudaMalloc(&ctx->d_ctl, sizeof(JControl)));
   CU(cudaMalloc(&ctx->d_queue, sizeof(JTask) * TASK_CAP));
   CU(cudaMalloc(&ctx->d_qends, sizeof(JQueueEnds) * QUEUE_SUBQ));
   CU(cudaMalloc(&ctx->d_err, sizeof(uint32_t) * 4));
   CU(cudaHostAlloc(&ctx->h_small, H_SMALL_BYTES, cudaHostAllocDefault));
-  ctx->device_bytes += sizeof(JControl) + sizeof(JTask) * TASK_CAP + sizeof(JQueueEnds) * QUEUE_SUBQ + 16;
+  ctx->device_bytes += sizeof(JTask) * TASK_CAP + sizeof(JQueueEnds) * QUEUE_SUBQ + 16;
   return GEM_OK;
 }
 
@@ -341,7 +340,6 @@ extern "C" void gem_ctx_destroy(gem_ctx *ctx) {
   else if (ctx->part_mem) cudaFree(ctx->part_mem);  // a lane's own staging buffers
   if (ctx->ev_ref && !ctx->borrowed_graph) cudaEventDestroy(ctx->ev_ref);
   destroy_join_graph(ctx->jgraph);
-  if (ctx->d_ctl) cudaFree(ctx->d_ctl);
   if (ctx->d_queue) cudaFree(ctx->d_queue);
   if (ctx->d_qends) cudaFree(ctx->d_qends);
   if (ctx->d_err) cudaFree(ctx->d_err);
@@ -844,6 +842,31 @@ static cudaError_t h2d(gem_ctx *ctx, void *dst, const void *src, size_t bytes) {
   return cudaMemcpyAsync(dst, st, bytes, cudaMemcpyHostToDevice, ctx->s);
 }
 
+// Arrays that go to the device in one allocation and one copy: a wave sends
+// a dozen arrays of a few hundred bytes, and a copy of its own costs each
+// about 2 us of the stream.  add() returns the array's offset; send() fills
+// `base` (device), at which the offsets are valid.
+struct Upload {
+  std::vector<char> host;
+  char *base = nullptr;
+  template <class T>
+  size_t add(const std::vector<T> &v) {
+    const size_t at = (host.size() + 63) & ~(size_t)63;
+    host.resize(at + v.size() * sizeof(T));
+    if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
+    return at;
+  }
+  template <class T>
+  T *at(size_t off) const {
+    return reinterpret_cast<T *>(base + off);
+  }
+  gem_status send(gem_ctx *ctx) {
+    ST(aalloc(ctx, host.empty() ? 1 : host.size(), &base));
+    CU(h2d(ctx, base, host.data(), host.size()));
+    return GEM_OK;
+  }
+};
+
 // Device-to-host copy that completes with a stream synchronisation.
 static cudaError_t d2h_sync(gem_ctx *ctx, void *dst, const void *src, size_t bytes) {
   if (!bytes) return cudaSuccess;
@@ -952,26 +975,17 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
     w.pos_words += words;
   }
   w.W = widest <= 2 ? widest : (widest + 3) / 4 * 4;
+  Upload up;
+  const size_t o_fr = up.add(fr), o_more = up.add(more), o_groups = up.add(groups), o_wl = up.add(wl);
+  ST(up.send(ctx));
   if (!stride && !wl.empty()) {
     stride = (uint32_t)((wl.size() + 15) / 16) * 16;
-    uint32_t *d_wl;
     uint8_t *d_nlc;
-    ST(aalloc(ctx, wl.size(), &d_wl));
-    CU(h2d(ctx, d_wl, wl.data(), 4 * wl.size()));
     ST(aalloc(ctx, (uint64_t)ctx->g.nv * stride, &d_nlc));
-    launch_nlc_labels(ctx->g, d_wl, (uint32_t)wl.size(), d_nlc, stride, ctx->s);
+    launch_nlc_labels(ctx->g, up.at<uint32_t>(o_wl), (uint32_t)wl.size(), d_nlc, stride, ctx->s);
     nlc = d_nlc;
   }
-  FilterRow *d_fr;
-  uint32_t *d_more;
-  ST(aalloc(ctx, rows ? rows : 1, &d_fr));
-  CU(h2d(ctx, d_fr, fr.data(), rows * sizeof(FilterRow)));
-  ST(aalloc(ctx, more.empty() ? 1 : more.size(), &d_more));
-  CU(h2d(ctx, d_more, more.data(), 4 * more.size()));
   const uint64_t nbits = (uint64_t)rows * nwords;
-  FilterGroup *d_groups;
-  ST(aalloc(ctx, groups.empty() ? 1 : groups.size(), &d_groups));
-  CU(h2d(ctx, d_groups, groups.data(), groups.size() * sizeof(FilterGroup)));
   w.d_cols = nullptr;
   if (columns) {
     ST(aalloc(ctx, (uint64_t)ctx->g.nv * w.W, &w.d_cols));
@@ -988,8 +1002,8 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   ST(aalloc(ctx, nsc + 1, &d_ex));
   ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
-  launch_filter(ctx->g, nlc, stride, d_fr, d_more, d_groups, (uint32_t)groups.size(), ts, threshold, d_bits, d_cnt,
-                w.d_cols, w.W, nwords, ctx->s);
+  launch_filter(ctx->g, nlc, stride, up.at<FilterRow>(o_fr), up.at<uint32_t>(o_more), up.at<FilterGroup>(o_groups),
+                (uint32_t)groups.size(), ts, threshold, d_bits, d_cnt, w.d_cols, w.W, nwords, ctx->s);
   launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
   launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
   std::vector<uint64_t> rs(rows + 1);
@@ -1041,6 +1055,24 @@ static gem_status spill_buffer(gem_ctx *ctx, uint64_t bytes) {
   return GEM_OK;
 }
 
+// The tables' value total, and the algorithmic bytes of the two passes: per
+// vertex tile (each pass) its offsets, 32 neighbour ids and column, and
+// (count) the 32 neighbours' columns and labels; per tile of a source (each
+// pass) the rank word and tile base; per table tile the mask written and read
+// and the value position; per value its id (and key position); the offsets;
+// per key its tile count and scan.
+static void wave_table_sizes(Wave &w, uint64_t src_tiles, uint64_t vtiles, uint64_t nvals) {
+  w.table_values = nvals;
+  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * w.W) + vtiles * 32ull * 4 * (w.W + 1) + 2 * src_tiles * 16 +
+                   w.table_tiles * (4 + 4 + 8) + nvals * (w.d_vkey ? 8 : 4) + w.n_offs * 8 + w.nkeys * (4 + 8 + 4);
+}
+
+// Waves of up to this many queries may size their tables by bounds, when the
+// bounds take no more than this (a mask's word and position per tile, two
+// words per value).
+constexpr size_t BOUNDED_QUERIES = 8;
+constexpr uint64_t BOUNDED_BYTES = 512ull << 20;
+
 static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // sources and edges of every active query
   std::vector<TabSource> src;
@@ -1069,42 +1101,6 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   }
   w.nsrc = (uint32_t)src.size();
   if (src.empty()) return GEM_OK;
-  TabSource *d_src;
-  ST(aalloc(ctx, src.size(), &d_src));
-  CU(h2d(ctx, d_src, src.data(), src.size() * sizeof(TabSource)));
-  uint32_t *d_tiles;
-  uint64_t *d_tp, *d_tmp, *d_stb;
-  ST(aalloc(ctx, nkeys ? nkeys : 1, &d_tiles));
-  ST(aalloc(ctx, nkeys + 1, &d_tp));
-  ST(aalloc(ctx, scan_tmp_words(nkeys), &d_tmp));
-  ST(aalloc(ctx, src.size() + 2, &d_stb));
-  launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), nkeys, d_tiles, ctx->s);
-  launch_scan(d_tiles, SCAN_U32, nkeys, d_tp, d_tmp, ctx->s);
-  // Vertex tiles: the 32-arc tiles of every vertex that some source holds
-  // (its membership column under the sources' bits); the table passes walk
-  // those tiles once for all sources.
-  const uint32_t nv = ctx->g.nv;
-  std::vector<uint32_t> smask(w.pos_words, 0);
-  for (uint32_t r : src_row) smask[w.row_pos[r] >> 5] |= 1u << (w.row_pos[r] & 31u);
-  RowLabel *d_labels;
-  uint32_t *d_smask, *d_vtiles;
-  uint64_t *d_vtg, *d_tmp3;
-  unsigned long long *d_next;  // unit counters of the two passes
-  ST(aalloc(ctx, w.labels.empty() ? 1 : w.labels.size(), &d_labels));
-  CU(h2d(ctx, d_labels, w.labels.data(), w.labels.size() * sizeof(RowLabel)));
-  ST(aalloc(ctx, smask.size(), &d_smask));
-  CU(h2d(ctx, d_smask, smask.data(), 4 * smask.size()));
-  ST(aalloc(ctx, nv ? nv : 1, &d_vtiles));
-  ST(aalloc(ctx, (uint64_t)nv + 1, &d_vtg));
-  ST(aalloc(ctx, scan_tmp_words(nv), &d_tmp3));
-  ST(aalloc(ctx, 2, &d_next));
-  launch_vertex_tiles(ctx->g, d_labels, (uint32_t)w.labels.size(), w.d_cols, w.W, d_smask, d_vtiles, ctx->s);
-  launch_scan(d_vtiles, SCAN_TILES, nv, d_vtg, d_tmp3, ctx->s);
-  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_vtg, nv, d_stb, d_next, ctx->s);
-  std::vector<uint64_t> stb(src.size() + 2);
-  CU(d2h_sync(ctx, stb.data(), d_stb, 8 * stb.size()));
-  CU(cudaGetLastError());
-  const uint64_t vtiles = (uint32_t)stb[src.size() + 1], vunits = stb[src.size() + 1] >> 32;
   // edges, grouped by source: a source's tables are one range of the edges
   struct EdgeReq {
     uint32_t s, qi, j, k;
@@ -1121,7 +1117,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   }
   std::stable_sort(reqs.begin(), reqs.end(), [](const EdgeReq &x, const EdgeReq &y) { return x.s < y.s; });
   std::vector<uint32_t> sedge(2 * src.size(), 0);
-  uint64_t tiles = 0, offs = 0;
+  uint64_t offs = 0;
   bool key_map = false;
   // a table is keyed by its source row and filtered by its target row: queries
   // (or twin query vertices) that need the same pair share one table
@@ -1146,52 +1142,129 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     if (!w.labels.empty())
       e.tcol -= 32 * std::lower_bound(w.labels.begin(), w.labels.end(), e.tlab,
                                       [](const RowLabel &x, uint32_t l) { return x.lab < l; })->word0;
-    e.tile_base = tiles;
-    e.ntiles = stb[rq.s + 1] - stb[rq.s];
+    e.tile_base = e.ntiles = 0;  // below
     e.off_base = offs;
     e.offsets = nullptr;
-    tiles += e.ntiles;
     offs += (uint64_t)src[rq.s].nkeys + 1;
     if (sedge[2 * rq.s + 1] == 0) sedge[2 * rq.s] = (uint32_t)edge.size();
     sedge[2 * rq.s + 1]++;
     w.edge_of[rq.qi][rq.j * QV + rq.k] = (uint32_t)edge.size();
     edge.push_back(e);
   }
-  const uint64_t src_tiles = stb[src.size()];
+  // Small waves skip the two read-backs that size the tables (the sources'
+  // tiles, the tables' values): each costs the stream's drain and a host
+  // round trip, about as much as a plain query's table kernels.  They take
+  // the label statistics' bounds instead: a table's tiles are at most its
+  // keys plus a 32nd of its label's arcs, its values at most the arcs between
+  // the two labels.  Gaps that the bounds leave hold zero masks.
+  const uint32_t nv = ctx->g.nv;
+  const size_t NL = ctx->label_freq.size();
+  auto tile_bound = [&](const TabEdge &e) -> uint64_t {
+    const uint32_t l = w.row_lab[src_row[e.src]];
+    return l < NL ? src[e.src].nkeys + ctx->label_arcs[l] / 32 : 0;
+  };
+  auto value_bound = [&](const TabEdge &e) -> uint64_t {
+    const uint32_t l = w.row_lab[src_row[e.src]];
+    return l < NL && e.tlab < NL ? ctx->label_pair_arcs[l * NL + e.tlab] : 0;
+  };
+  const uint64_t all_tiles = nv + ctx->g.narcs / 32;
+  uint64_t tiles = 0, value_cap = 0;
+  bool bounded = !ctx->opts.ooc && !ctx->label_pair_arcs.empty() && w.q.size() <= BOUNDED_QUERIES;
+  if (bounded) {
+    for (const TabEdge &e : edge) {
+      tiles += tile_bound(e);
+      value_cap += value_bound(e);
+    }
+    const uint64_t need = 12 * tiles + 8 * value_cap + 8 * all_tiles;
+    uint64_t free_bytes = ctx->budget > ctx->device_bytes ? ctx->budget - ctx->device_bytes : 0;
+    for (const auto &ch : ctx->arena.chunks) free_bytes += ch.size - ch.used;
+    bounded = need <= BOUNDED_BYTES && need <= free_bytes / 4;
+  }
+  std::vector<uint32_t> smask(w.pos_words, 0);
+  for (uint32_t r : src_row) smask[w.row_pos[r] >> 5] |= 1u << (w.row_pos[r] & 31u);
   uint64_t *d_offs;
   ST(aalloc(ctx, offs, &d_offs));
   for (auto &e : edge) e.offsets = d_offs + e.off_base;
-  TabEdge *d_edge;
-  ST(aalloc(ctx, edge.size(), &d_edge));
-  CU(h2d(ctx, d_edge, edge.data(), edge.size() * sizeof(TabEdge)));
+  // the sources (by row position) and tables as the passes read them
+  std::vector<VSrc> vs(32 * (size_t)w.pos_words);
+  for (size_t i = 0; i < src.size(); ++i)
+    vs[w.row_pos[src_row[i]]] =
+        VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, sedge[2 * i], sedge[2 * i + 1]};
+  std::vector<VEdge> ve(edge.size());
+  // stb: the sources' first tiles (exact sizes only)
+  std::vector<uint64_t> stb(src.size() + 2, 0);
+  auto place_edges = [&] {
+    tiles = 0;
+    for (size_t i = 0; i < edge.size(); ++i) {
+      TabEdge &e = edge[i];
+      e.tile_base = tiles;
+      e.ntiles = bounded ? tile_bound(e) : stb[e.src + 1] - stb[e.src];
+      tiles += e.ntiles;
+      ve[i] = VEdge{e.tile_base, e.tlab, e.tcol | (e.flags & TAB_KEY_MAP) << 31};
+    }
+  };
+  if (bounded) place_edges();
+  Upload up, up2;
+  const size_t o_src = up.add(src), o_labels = up.add(w.labels), o_smask = up.add(smask), o_vs = up.add(vs);
+  size_t o_edge = 0, o_ve = 0;
+  if (bounded) {
+    o_edge = up.add(edge);
+    o_ve = up.add(ve);
+  }
+  ST(up.send(ctx));
+  const TabSource *d_src = up.at<TabSource>(o_src);
+  const RowLabel *d_labels = up.at<RowLabel>(o_labels);
+  const uint32_t *d_smask = up.at<uint32_t>(o_smask);
+  uint32_t *d_tiles;
+  uint64_t *d_tp, *d_tmp, *d_sizes;  // d_sizes: stb, then the tables' first values
+  ST(aalloc(ctx, nkeys ? nkeys : 1, &d_tiles));
+  ST(aalloc(ctx, nkeys + 1, &d_tp));
+  ST(aalloc(ctx, scan_tmp_words(nkeys), &d_tmp));
+  ST(aalloc(ctx, stb.size() + edge.size() + 1, &d_sizes));
+  uint64_t *d_stb = d_sizes, *d_ebase = d_sizes + stb.size();
+  launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), nkeys, d_tiles, ctx->s);
+  launch_scan(d_tiles, SCAN_U32, nkeys, d_tp, d_tmp, ctx->s);
+  // Vertex tiles: the 32-arc tiles of every vertex that some source holds
+  // (its membership column under the sources' bits); the table passes walk
+  // those tiles once for all sources.
+  uint32_t *d_vtiles;
+  uint64_t *d_vtg, *d_tmp3;
+  unsigned long long *d_next;  // unit counters of the two passes
+  ST(aalloc(ctx, nv ? nv : 1, &d_vtiles));
+  ST(aalloc(ctx, (uint64_t)nv + 1, &d_vtg));
+  ST(aalloc(ctx, scan_tmp_words(nv), &d_tmp3));
+  ST(aalloc(ctx, 2, &d_next));
+  launch_vertex_tiles(ctx->g, d_labels, (uint32_t)w.labels.size(), w.d_cols, w.W, d_smask, d_vtiles, ctx->s);
+  launch_scan(d_vtiles, SCAN_TILES, nv, d_vtg, d_tmp3, ctx->s);
+  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_vtg, nv, d_stb, d_next, ctx->s);
+  uint64_t vtiles = all_tiles, vunits = all_tiles;
+  if (!bounded) {
+    CU(d2h_sync(ctx, stb.data(), d_stb, 8 * stb.size()));
+    CU(cudaGetLastError());
+    vtiles = (uint32_t)stb[src.size() + 1];
+    vunits = stb[src.size() + 1] >> 32;
+    place_edges();
+    o_edge = up2.add(edge);
+    o_ve = up2.add(ve);
+    ST(up2.send(ctx));
+  }
+  const Upload &ue = bounded ? up : up2;
+  const TabEdge *d_edge = ue.at<TabEdge>(o_edge);
   uint32_t *d_mask;
   uint64_t *d_vp, *d_tmp2;
   ST(aalloc(ctx, tiles ? tiles : 1, &d_mask));
   ST(aalloc(ctx, tiles + 1, &d_vp));
   ST(aalloc(ctx, scan_tmp_words(tiles), &d_tmp2));
-  // the tile -> vertex map, and the sources (by row position) and tables as
-  // the passes read them
+  if (bounded) CU(cudaMemsetAsync(d_mask, 0, 4 * tiles, ctx->s));
   if (!table_vtx_fits(w.W)) {
     ctx->err = "too many filter rows of one label in one wave";
     return GEM_ERR_LIMIT;
   }
+  // the vertex of every tile and unit
   uint32_t *d_vt, *d_vg;
   ST(aalloc(ctx, vtiles ? vtiles : 1, &d_vt));
   ST(aalloc(ctx, vunits ? vunits : 1, &d_vg));
   launch_vertex_maps(d_vtg, nv, d_vt, d_vg, ctx->s);
-  std::vector<VSrc> vs(32 * (size_t)w.pos_words);
-  for (size_t i = 0; i < src.size(); ++i)
-    vs[w.row_pos[src_row[i]]] =
-        VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, stb[i], sedge[2 * i], sedge[2 * i + 1]};
-  std::vector<VEdge> ve(edge.size());
-  for (size_t i = 0; i < edge.size(); ++i)
-    ve[i] = VEdge{edge[i].tile_base, edge[i].tlab, edge[i].tcol | (edge[i].flags & TAB_KEY_MAP) << 31};
-  VSrc *d_vs;
-  VEdge *d_ve;
-  ST(aalloc(ctx, vs.size(), &d_vs));
-  CU(h2d(ctx, d_vs, vs.data(), vs.size() * sizeof(VSrc)));
-  ST(aalloc(ctx, ve.size(), &d_ve));
-  CU(h2d(ctx, d_ve, ve.data(), ve.size() * sizeof(VEdge)));
   // Out-of-core: the vertex tiles of a partition (a vertex range) are one
   // range of the tile order.  Stream the partitions that hold tiles when
   // they are filled enough (their bytes at most twice what the tiles would
@@ -1227,6 +1300,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.arc_shift = 0;
     P.t0 = 0;
     P.t1 = write ? vunits : vtiles;
+    P.end = bounded ? d_vtg + nv : nullptr;
     P.vt = d_vt;
     P.vg = d_vg;
     P.vtg = d_vtg;
@@ -1237,8 +1311,8 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.W = w.W;
     P.cols = w.d_cols;
     P.smask = d_smask;
-    P.vsrc = d_vs;
-    P.vedge = d_ve;
+    P.vsrc = up.at<VSrc>(o_vs);
+    P.vedge = ue.at<VEdge>(o_ve);
     P.tp = d_tp;
     P.mask = d_mask;
     P.vp = d_vp;
@@ -1279,15 +1353,27 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   launch_scan(d_mask, SCAN_POPC_U32, tiles, d_vp, d_tmp2, ctx->s);
   // every table's first value position and the total (table sizes order the
   // wave's queries by estimated join work)
-  uint64_t *d_ebase;
-  ST(aalloc(ctx, edge.size() + 1, &d_ebase));
   launch_edge_value_bases(d_edge, (uint32_t)edge.size(), d_vp, tiles, d_ebase, ctx->s);
-  std::vector<uint64_t> ebase(edge.size() + 1);
-  CU(d2h_sync(ctx, ebase.data(), d_ebase, 8 * ebase.size()));
-  CU(cudaGetLastError());
-  const uint64_t nvals = ebase[edge.size()];
   w.edge_vals.resize(edge.size());
-  for (size_t e = 0; e < edge.size(); ++e) w.edge_vals[e] = ebase[e + 1] - ebase[e];
+  w.s_sizes = nullptr;
+  uint64_t nvals = value_cap;
+  if (bounded) {  // the sizes arrive with the join's results
+    w.n_sizes = stb.size() + edge.size() + 1;
+    uint64_t *to = static_cast<uint64_t *>(stage(ctx, 8 * w.n_sizes));
+    if (!to) {  // staging used up: pageable
+      w.sizes.resize(w.n_sizes);
+      to = w.sizes.data();
+    }
+    CU(cudaMemcpyAsync(to, d_sizes, 8 * w.n_sizes, cudaMemcpyDeviceToHost, ctx->s));
+    w.s_sizes = to;
+    for (size_t e = 0; e < edge.size(); ++e) w.edge_vals[e] = value_bound(edge[e]);
+  } else {
+    std::vector<uint64_t> ebase(edge.size() + 1);
+    CU(d2h_sync(ctx, ebase.data(), d_ebase, 8 * ebase.size()));
+    CU(cudaGetLastError());
+    nvals = ebase[edge.size()];
+    for (size_t e = 0; e < edge.size(); ++e) w.edge_vals[e] = ebase[e + 1] - ebase[e];
+  }
   // The values (and key positions) of the wave's tables.  Out of core, a
   // single query whose tables do not fit the device budget keeps them in
   // mapped pinned host memory, which the write pass and the join reach over
@@ -1324,16 +1410,11 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   w.table_passes = true;
   CU(cudaGetLastError());
   w.edges = edge;
-  w.table_values = nvals;
+  w.value_cap = nvals;
+  w.nkeys = nkeys;
+  w.n_offs = offs;
   w.table_tiles = tiles;
-  // algorithmic bytes of the two passes: per vertex tile (each pass) its
-  // offsets, 32 neighbour ids and column, and (count) the 32 neighbours'
-  // columns and labels; per tile of a source (each pass) the rank word and tile base;
-  // per table tile the mask written and read and the value position; per
-  // value its id (and key position); the offsets; per key its tile count
-  // and scan.
-  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * w.W) + vtiles * 32ull * 4 * (w.W + 1) + 2 * src_tiles * 16 +
-                   tiles * (4 + 4 + 8) + nvals * (w.d_vkey ? 8 : 4) + offs * 8 + nkeys * (4 + 8 + 4);
+  if (!bounded) wave_table_sizes(w, stb[src.size()], vtiles, nvals);
   return GEM_OK;
 }
 
@@ -1426,12 +1507,11 @@ static double join_cost(const Wave &w, size_t qi) {
 static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, uint64_t emb_cap) {
   std::vector<JQuery> jq;
   std::vector<JBack> jb;
-  std::vector<uint64_t> rp, terms, lpp;
+  std::vector<uint64_t> terms, lpp;
   std::vector<uint32_t> lpq, lp2q;
   uint64_t lp_roots = 0;
-  bool pair_items = false;
+  bool pair_items = false, ordinary = false;
   w.jq_index.assign(w.q.size(), UINT32_MAX);
-  uint64_t roots = 0;
   // Queries take the grid's warps in order of estimated work, cheapest
   // first: under a time cap the queries that can finish do so before the
   // expensive ones take the warps, and a wave's result for a query does not
@@ -1463,7 +1543,6 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
     const uint32_t r0 = w.row_of[qi][p.order[0]];
     J.root_cand = w.d_cand + w.c_base[r0];
     J.n_root = w.cnt[r0];
-    J.root_base = roots;
     for (uint32_t k = 0; k < p.n; ++k) {
       JLevel &L = J.lv[k];
       L.u = p.order[k];
@@ -1492,76 +1571,55 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
       lpq.push_back((uint32_t)jq.size());
       lpp.push_back(lp_roots);
       lp_roots += J.n_root;
-      J.root_base = roots;
-      rp.push_back(roots);
     } else if (w.pair[qi] == PAIR_POOL && w.d_vkey) {
       // (root, first level) pair pool; an empty range in the ordinary pool
       lp2q.push_back((uint32_t)jq.size());
-      J.root_base = roots;
-      rp.push_back(roots);
     } else {
       // items of the ordinary pool: the entries of the root table (every
       // root with each of its first-level vertices), so that a hub's many
       // subtrees start on as many warps; else the roots
       J.pairs = w.pair[qi] == PAIR_ITEMS && w.d_vkey;
       pair_items |= J.pairs != 0;
-      rp.push_back(roots);
-      roots += J.pairs ? w.edge_vals[w.edge_of[qi][1]] : J.n_root;
+      J.pool = 1;
+      ordinary = true;
     }
     jq.push_back(J);
   }
-  rp.push_back(roots);
   lpp.push_back(lp_roots);
   w.out.assign(w.q.size(), JOut());
-  uint32_t *d_lp2q = nullptr;
-  uint64_t *d_lp2p = nullptr;
   if (jq.empty()) return GEM_OK;
-  JQuery *d_jq;
-  JBack *d_jb;
-  uint64_t *d_rp, *d_terms;
-  JOut *d_out;
-  ST(aalloc(ctx, terms.size() ? terms.size() : 1, &d_terms));
-  uint32_t *d_lpq;
-  uint64_t *d_lpp;
-  ST(aalloc(ctx, lpq.size() ? lpq.size() : 1, &d_lpq));
-  ST(aalloc(ctx, lpp.size(), &d_lpp));
-  if (!lpq.empty()) CU(h2d(ctx, d_lpq, lpq.data(), lpq.size() * 4));
-  if (!lp2q.empty()) {
-    ST(aalloc(ctx, lp2q.size(), &d_lp2q));
-    ST(aalloc(ctx, lp2q.size() + 1, &d_lp2p));  // filled by the prepare kernel
-    CU(h2d(ctx, d_lp2q, lp2q.data(), lp2q.size() * 4));
-  }
-  CU(h2d(ctx, d_lpp, lpp.data(), lpp.size() * 8));
-  if (!terms.empty())
-    CU(h2d(ctx, d_terms, terms.data(), terms.size() * 8));
-  ST(aalloc(ctx, jq.size(), &d_jq));
-  ST(aalloc(ctx, jb.size() ? jb.size() : 1, &d_jb));
-  ST(aalloc(ctx, rp.size(), &d_rp));
-  ST(aalloc(ctx, jq.size(), &d_out));
-  CU(h2d(ctx, d_jq, jq.data(), jq.size() * sizeof(JQuery)));
-  if (!jb.empty()) CU(h2d(ctx, d_jb, jb.data(), jb.size() * sizeof(JBack)));
-  CU(h2d(ctx, d_rp, rp.data(), rp.size() * 8));
+  Upload up;
+  const size_t o_terms = up.add(terms), o_lpq = up.add(lpq), o_lpp = up.add(lpp), o_lp2q = up.add(lp2q),
+               o_jq = up.add(jq), o_jb = up.add(jb);
+  ST(up.send(ctx));
+  // filled by the prepare kernel: the pools' item prefixes, the control block
+  // and (behind it, so that one copy brings both back) the queries' outputs
+  uint64_t *d_rp;
+  ST(aalloc(ctx, jq.size() + lp2q.size() + 2, &d_rp));
+  char *d_res;
+  const size_t res_bytes = sizeof(JControl) + jq.size() * sizeof(JOut);
+  ST(aalloc(ctx, res_bytes, &d_res));
   const uint64_t cap_ms = ctx->opts.time_cap_ms ? ctx->opts.time_cap_ms : 600000u;
   JoinArgs a;
   std::memset(&a, 0, sizeof a);
-  a.queries = d_jq;
+  a.queries = up.at<JQuery>(o_jq);
   a.nquery = (uint32_t)jq.size();
   a.mode = (uint32_t)mode;
-  a.backs = d_jb;
+  a.backs = up.at<JBack>(o_jb);
   a.values = w.d_values;
   a.root_prefix = d_rp;
-  a.terms = d_terms;
-  a.n_roots = roots;
-  a.lp_query = d_lpq;
-  a.lp_prefix = d_lpp;
+  a.terms = up.at<uint64_t>(o_terms);
+  a.ordinary = ordinary;
+  a.lp_query = up.at<uint32_t>(o_lpq);
+  a.lp_prefix = up.at<uint64_t>(o_lpp);
   a.lp_nq = (uint32_t)lpq.size();
   a.lp_roots = lp_roots;
-  a.lp2_query = d_lp2q;
+  a.lp2_query = up.at<uint32_t>(o_lp2q);
   a.lp2_nq = (uint32_t)lp2q.size();
-  a.lp2_prefix = d_lp2p;
+  a.lp2_prefix = d_rp + jq.size() + 1;
   a.vkey = w.d_vkey;
-  a.out = d_out;
-  a.ctl = ctx->d_ctl;
+  a.out = reinterpret_cast<JOut *>(d_res + sizeof(JControl));
+  a.ctl = reinterpret_cast<JControl *>(d_res);
   a.queue = ctx->d_queue;
   a.qends = ctx->d_qends;
   a.emb = emb_dev;
@@ -1581,7 +1639,7 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   a.nv = ctx->g.nv;
   a.vnh_off = ctx->g.off;
   a.vnh_buckets = ctx->vnh_buckets;
-  a.n_values = w.table_values;
+  a.n_values = w.value_cap;
   a.n_backs = (uint32_t)jb.size();
   a.n_terms = (uint32_t)terms.size();
   int bps = ctx->join_bps[mode];
@@ -1596,13 +1654,17 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   CU(cudaGetLastError());
   std::vector<JOut> out(jq.size());
   JControl hc;
-  JOut *s_out = static_cast<JOut *>(stage(ctx, out.size() * sizeof(JOut)));
-  JControl *s_ctl = static_cast<JControl *>(stage(ctx, sizeof(JControl)));
-  CU(cudaMemcpyAsync(s_out ? s_out : out.data(), d_out, out.size() * sizeof(JOut), cudaMemcpyDeviceToHost, ctx->s));
-  CU(cudaMemcpyAsync(s_ctl ? s_ctl : &hc, ctx->d_ctl, sizeof hc, cudaMemcpyDeviceToHost, ctx->s));
+  char *s_res = static_cast<char *>(stage(ctx, res_bytes));
+  std::vector<char> pageable(s_res ? 0 : res_bytes);
+  if (!s_res) s_res = pageable.data();
+  CU(cudaMemcpyAsync(s_res, d_res, res_bytes, cudaMemcpyDeviceToHost, ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
-  if (s_out) std::memcpy(out.data(), s_out, out.size() * sizeof(JOut));
-  if (s_ctl) std::memcpy(&hc, s_ctl, sizeof hc);
+  std::memcpy(&hc, s_res, sizeof hc);
+  std::memcpy(out.data(), s_res + sizeof hc, out.size() * sizeof(JOut));
+  if (w.s_sizes) {
+    const uint64_t *z = w.s_sizes, n = w.nsrc;
+    wave_table_sizes(w, z[n], (uint32_t)z[n + 1], z[w.n_sizes - 1]);
+  }
   w.join_ms = ev_ms(ctx->ev[6], ctx->ev[7]);
   // Donated tasks still queued when the grid stopped (deadline) were never
   // run: their queries are incomplete.
@@ -2004,6 +2066,7 @@ extern "C" gem_status gem_filter(gem_ctx *ctx, const gem_query *q, uint32_t thre
   w.q.resize(1);
   ST(make_host_query(q, w.q[0], ctx->err));
   ctx->arena.reset();
+  ctx->h_used = 0;  // the previous call ended with a synchronisation
   w.share_rows = false;  // rows in query-vertex order, one each
   ST(wave_filter(ctx, w, threshold, false));
   CU(cudaStreamSynchronize(ctx->s));
@@ -2025,6 +2088,7 @@ extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t 
   const HostQuery &hq = w.q[0];
   if (u >= hq.nv || wv >= hq.nv || !(hq.adj[u] & (1u << wv))) return GEM_ERR_ARG;
   ctx->arena.reset();
+  ctx->h_used = 0;  // the previous call ended with a synchronisation
   w.share_rows = false;  // rows in query-vertex order, one each
   w.active.assign(1, 1);
   ST(wave_filter(ctx, w, 0, true));
@@ -2061,6 +2125,7 @@ extern "C" gem_status gem_index_probe(gem_ctx *ctx, const gem_query *q, uint32_t
   ST(make_host_query(q, w.q[0], ctx->err));
   if (u >= w.q[0].nv) return GEM_ERR_ARG;
   ctx->arena.reset();
+  ctx->h_used = 0;  // the previous call ended with a synchronisation
   w.share_rows = false;  // rows in query-vertex order, one each
   w.active.assign(1, 1);
   w.idx_kind.assign(1, std::vector<uint32_t>(QV, 0));

@@ -99,6 +99,11 @@ struct Wave {
   std::vector<uint64_t> edge_vals;  // values per table (edges[e])
   uint32_t *d_values = nullptr;
   uint64_t table_values = 0, table_tiles = 0;
+  uint64_t value_cap = 0;           // entries of d_values: table_values, or the bound it was sized by
+  uint64_t nkeys = 0, n_offs = 0;   // keys of the sources, offsets of the tables
+  const uint64_t *s_sizes = nullptr;  // pinned: sizes that arrive with the join's results (n_sizes words)
+  size_t n_sizes = 0;
+  std::vector<uint64_t> sizes;      // their place when the pinned staging is used up
   const gem::CuckooTable *ck_tabs = nullptr;
   uint32_t cuckoo_round = 0;
   std::vector<uint32_t> jq_index;
@@ -172,7 +177,6 @@ struct gem_ctx {
   Server *server = nullptr;          // serving thread (gem_submit / gem_poll)
   // scratch
   Arena arena;
-  gem::JControl *d_ctl = nullptr;
   gem::JTask *d_queue = nullptr;
   gem::JQueueEnds *d_qends = nullptr;
   uint32_t *d_err = nullptr;

@@ -1352,8 +1352,9 @@ __device__ __forceinline__ uint32_t find_query(const uint64_t *__restrict__ rp, 
 // grid drains quickly; the queries owning withdrawn roots are marked too.
 __device__ void abandon(const JoinArgs &a, uint32_t q) {
   if (q < a.nquery) atomicOr(&a.out[q].pad[0], 1ull);
-  const unsigned long long r0 = atomicExch(&a.ctl->root_next, (unsigned long long)a.n_roots);
-  if (r0 < a.n_roots)
+  const unsigned long long items = __ldg(a.root_prefix + a.nquery);
+  const unsigned long long r0 = atomicExch(&a.ctl->root_next, items);
+  if (r0 < items)
     for (uint32_t k = find_query(a.root_prefix, a.nquery, r0); k < a.nquery; ++k) atomicOr(&a.out[k].pad[0], 1ull);
 }
 
@@ -1365,7 +1366,7 @@ __device__ __forceinline__ void root_item(const JoinArgs &a, uint64_t r, uint32_
                                           uint32_t &f1, uint32_t &k1) {
   q = find_query(a.root_prefix, a.nquery, r);
   const JQuery *Q = a.queries + q;
-  const uint64_t rl = r - Q->root_base;
+  const uint64_t rl = r - __ldg(a.root_prefix + q);
   f0 = f1 = k1 = 0;
   k0 = 0xFFFFFFFFu;
   if (!Q->pairs) {
@@ -1660,6 +1661,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
     }
   }
 
+  const uint64_t n_items = PART & PART_DFS ? __ldg(a.root_prefix + a.nquery) : ~0ull;  // of the ordinary pool
   // Lane i's item of the batch held (rb_first + i): its query, and the matched
   // vertices and positions of its prefix (a root, or a root and a first level).
   uint64_t rb_first = 0;
@@ -1675,17 +1677,17 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
         unsigned long long rr = 0, cnt = 1;
         if (lane == 0) {
           const unsigned long long seen = ld_vol(&ctl->root_next);
-          const unsigned long long left = seen < a.n_roots ? a.n_roots - seen : 0;
+          const unsigned long long left = seen < n_items ? n_items - seen : 0;
           cnt = left / (4ull * total_warps);
           cnt = cnt < 1 ? 1 : (cnt > a.root_batch_max ? a.root_batch_max : cnt);
           atomicAdd(&ctl->busy, 1u);
           __threadfence();
           rr = atomicAdd(&ctl->root_next, cnt);
-          if (rr >= a.n_roots) atomicSub(&ctl->busy, 1u);
+          if (rr >= n_items) atomicSub(&ctl->busy, 1u);
         }
         rb_cur = __shfl_sync(FULL, rr, 0);
         cnt = __shfl_sync(FULL, cnt, 0);
-        rb_end = rb_cur < a.n_roots ? (rb_cur + cnt < a.n_roots ? rb_cur + cnt : a.n_roots) : rb_cur;
+        rb_end = rb_cur < n_items ? (rb_cur + cnt < n_items ? rb_cur + cnt : n_items) : rb_cur;
         rb_first = rb_cur;
         if (rb_cur < rb_end && err_set(a)) {
           // past the deadline: the batch is not processed
@@ -2062,46 +2064,54 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
   }
 }
 
-// Zeroes the control block and the per-query outputs, resets the task queue
-// and sets the deadline; runs right before the join in the same graph.
+// prefix[i] = sum of size(0..i-1) for i <= n, by one block.
+template <class F>
+__device__ void block_prefix(uint32_t n, uint64_t *prefix, F size) {
+  __shared__ uint64_t wsum[32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint64_t carry = 0;
+  for (uint32_t b0 = 0; b0 < n; b0 += blockDim.x) {
+    const uint32_t i = b0 + threadIdx.x;
+    const uint64_t x = i < n ? size(i) : 0;
+    uint64_t incl = x;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t o = __shfl_up_sync(FULL, incl, d);
+      if (lane >= (uint32_t)d) incl += o;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint64_t before = carry, all = 0;
+    for (uint32_t w = 0; w < nw; ++w) {
+      if (w < warp) before += wsum[w];
+      all += wsum[w];
+    }
+    if (i < n) prefix[i] = before + incl - x;
+    carry += all;
+    __syncthreads();  // wsum is rewritten by the next step
+  }
+  if (threadIdx.x == 0) prefix[n] = carry;
+}
+
+// Zeroes the control block and the per-query outputs, resets the task queue,
+// sets the deadline and lays out the pools; runs right before the join in
+// the same graph.
 __global__ void join_prepare_kernel(JControl *ctl, JOut *out, uint32_t nquery, JTask *cells, JQueueEnds *qends,
-                                    uint64_t cap_ns, const JQuery *queries, const JBack *backs,
+                                    uint64_t cap_ns, const JQuery *queries, const JBack *backs, uint64_t *root_prefix,
                                     const uint32_t *lp2q, uint32_t lp2_nq, uint64_t *lp2_prefix) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  // pair pool: each query's (root, first level) pairs are the entries of its
-  // root table, padded to whole chunks of 32 so no chunk spans two queries;
-  // block 0 scans the padded sizes, one query per thread
-  if (blockIdx.x == 0 && lp2_nq) {
-    __shared__ uint64_t wsum[32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint64_t carry = 0;
-    for (uint32_t b0 = 0; b0 < lp2_nq; b0 += blockDim.x) {
-      const uint32_t i = b0 + threadIdx.x;
-      uint64_t n = 0;
-      if (i < lp2_nq) {
-        const JQuery *Q = queries + lp2q[i];
-        const JBack *b = backs + Q->lv[1].back_base;
-        n = ((b->off[b->nkeys] - b->off[0]) + 31) & ~31ull;
-      }
-      uint64_t incl = n;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint64_t o = __shfl_up_sync(FULL, incl, d);
-        if (lane >= (uint32_t)d) incl += o;
-      }
-      if (lane == 31) wsum[warp] = incl;
-      __syncthreads();
-      uint64_t before = carry, tile = 0;
-      for (uint32_t w = 0; w < nw; ++w) {
-        if (w < warp) before += wsum[w];
-        tile += wsum[w];
-      }
-      if (i < lp2_nq) lp2_prefix[i] = before + incl - n;
-      carry += tile;
-      __syncthreads();  // wsum is rewritten by the next step
-    }
-    if (threadIdx.x == 0) lp2_prefix[lp2_nq] = carry;
-  }
+  // the entries of a query's root table (its (root, first level) pairs)
+  auto pairs = [&](const JQuery *Q) {
+    const JBack *b = backs + Q->lv[1].back_base;
+    return b->off[b->nkeys] - b->off[0];
+  };
+  // pair pool: padded to whole chunks of 32 so that no chunk spans two queries
+  if (blockIdx.x == 0) block_prefix(lp2_nq, lp2_prefix, [&](uint32_t i) { return (pairs(queries + lp2q[i]) + 31) & ~31ull; });
+  if (blockIdx.x == 1)
+    block_prefix(nquery, root_prefix, [&](uint32_t i) -> uint64_t {
+      const JQuery *Q = queries + i;
+      return !Q->pool ? 0 : Q->pairs ? pairs(Q) : Q->n_root;
+    });
   for (uint32_t i = t; i < TASK_CAP; i += nt) cells[i].seq = i & (QUEUE_SUBQ_CAP - 1);
   for (uint32_t i = t; i < QUEUE_SUBQ; i += nt) {
     qends[i].head = 0;
@@ -2173,14 +2183,15 @@ cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns,
   uint64_t cap = cap_ns;
   const JQuery *queries = a.queries;
   const JBack *backs = a.backs;
+  uint64_t *root_prefix = const_cast<uint64_t *>(a.root_prefix);
   const uint32_t *lp2q = a.lp2_query;
   uint32_t lp2_nq = a.lp2_nq;
   uint64_t *lp2_prefix = const_cast<uint64_t *>(a.lp2_prefix);
-  void *prep_params[] = {&ctl, &out, &nq, &cells, &qends, &cap, &queries, &backs, &lp2q, &lp2_nq, &lp2_prefix};
+  void *prep_params[] = {&ctl, &out, &nq, &cells, &qends, &cap, &queries, &backs, &root_prefix, &lp2q, &lp2_nq, &lp2_prefix};
   void *join_params[] = {&args};
   // the kernels this wave needs, in order
   const bool split = a.mode == MODE_COUNT;
-  const bool pools = split && (a.lp_roots || a.lp2_nq), dfs = !split || a.n_roots;
+  const bool pools = split && (a.lp_roots || a.lp2_nq), dfs = !split || a.ordinary;
   cudaKernelNodeParams kp[3] = {};
   uint32_t nk = 0;
   auto node = [&](void *fn, uint32_t blocks, uint32_t smem, void **params) {

@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   unsigned long long got = 0;
   if (lane == 0) got = atomicAdd(P.next, 1ull);
   uint64_t t = P.t0 + __shfl_sync(dev::FULL, got, 0);
-  if (t >= P.t1) return;
+  const uint64_t t1 = P.end ? (uint64_t)(uint32_t)(__ldg(P.end) >> half) : P.t1;
+  if (t >= t1) return;
   uint32_t v = __ldg(vmap + t);
   uint64_t a0 = __ldg(P.off + v), a1 = __ldg(P.off + v + 1);
   uint64_t c = (t - (uint32_t)(__ldg(P.vtg + v) >> half)) * G;  // the unit: tiles c .. c + nt - 1 of vertex v
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
     }
     const uint64_t tn = P.t0 + __shfl_sync(dev::FULL, got, 0);
     uint32_t vn = 0;
-    if (tn < P.t1) vn = __ldg(vmap + tn);
+    if (tn < t1) vn = __ldg(vmap + tn);
     const uint32_t *sv = P.cols + (uint64_t)v * P.W;
     for (uint32_t wb = 0; wb < vl.words; wb += 32) {
       const uint32_t word = wb + lane < vl.words ? __ldg(sv + wb + lane) & __ldg(P.smask + vl.word0 + wb + lane) : 0u;
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
           const VSrc &src = P.vsrc[(vl.word0 + wb + j) * 32u + dev::nth_set_bit(wj, q - exj)];
           const uint64_t rw = __ldg(src.rb + (v >> 5));
           k = (uint32_t)(rw >> 32) + __popc((uint32_t)rw & ((1u << (v & 31u)) - 1u));
-          lt = __ldg(P.tp + src.key_base + k) - src.stb + c;
+          lt = __ldg(P.tp + src.key_base + k) - __ldg(P.tp + src.key_base) + c;
           e0 = src.e0;
           ne = src.ne;
         }
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
         }
       }
     }
-    if (tn >= P.t1) return;
+    if (tn >= t1) return;
     v = vn;
     a0 = __ldg(P.off + v);
     a1 = __ldg(P.off + v + 1);

@@ -179,7 +179,6 @@ void launch_gather_u64(const uint64_t *a, const uint32_t *idx, uint32_t n, uint6
 struct VSrc {                // a table source as the vertex-tile passes see it
   const uint64_t *rb;        // rank bitmap row of its candidates
   uint64_t key_base;         // first key in the flattened key space
-  uint64_t stb;              // tp[key_base]: its first tile
   uint32_t e0, ne;           // its tables: edges [e0, e0 + ne)
 };
 struct VEdge {
@@ -199,7 +198,8 @@ struct VPass {
   const uint64_t *off;
   const uint32_t *nbr;
   uint64_t arc_shift;
-  uint64_t t0, t1;
+  uint64_t t0, t1;           // t1: a bound of the units when `end` (the last word of vtg) has their number
+  const uint64_t *end;
   const uint32_t *vt;
   const uint32_t *vg;
   const uint64_t *vtg;
@@ -322,12 +322,11 @@ struct JQuery {
   const uint32_t *root_cand; // C(root)
   uint32_t n_root;
   uint32_t n_enum;           // levels enumerated; levels n_enum..n-1 are counted in closed form
-  uint64_t root_base;        // first global root index of this query
   uint32_t n_groups;         // label groups of the suffix
   uint32_t flat;             // balanced lane-level counting: subset values per prefix match
                              // (bits 0-7; 0 = not eligible) and those needing a scan (bits 8-15)
+  uint32_t pool;             // its items are in the ordinary pool
   uint32_t pairs;            // items of the ordinary pool: (root, first level) pairs instead of roots
-  uint32_t pad;
   uint32_t grp_first[MAX_GROUPS];
   uint32_t grp_size[MAX_GROUPS];
   uint32_t term_base[MAX_GROUPS];
@@ -391,7 +390,7 @@ struct JoinArgs {
   const JBack *backs;
   JQueueEnds *qends;          // QUEUE_SUBQ sub-queue ends (cells in `queue`)
   const uint32_t *values;     // edge-table values of the whole wave
-  const uint64_t *root_prefix; // nquery + 1 global root offsets
+  const uint64_t *root_prefix; // nquery + 1 item offsets of the ordinary pool (written by the prepare kernel)
   // Lane-parallel root pool: queries whose only enumerated level is the root
   // (count mode with n_enum == 1, or single-vertex queries); 32 roots per warp.
   const uint32_t *lp_query;    // query index of each pool segment
@@ -400,7 +399,8 @@ struct JoinArgs {
   uint32_t pad_lp;
   uint64_t lp_roots;
   const uint64_t *terms;      // inclusion-exclusion terms of every query's suffix groups
-  uint64_t n_roots;
+  uint32_t ordinary;          // some query has items in the ordinary pool
+  uint32_t pad_items;
   JOut *out;
   JControl *ctl;
   JTask *queue;
