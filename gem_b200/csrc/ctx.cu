@@ -194,6 +194,7 @@ extern "C" gem_status gem_ctx_create(const gem_opts *opts, gem_ctx **out) {
   CU(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->opts.device));
   for (uint32_t m = 0; m < 3; ++m) ctx->join_bps[m] = join_blocks_per_sm(m);
   ctx->pool_bps = join_pool_blocks_per_sm();
+  ctx->hashed_bps = join_hashed_blocks_per_sm();
   CU(cudaEventCreate(&ctx->ev_ref));
   ST(exec_init(ctx));
   *out = c.release();
@@ -239,6 +240,7 @@ gem_status lane_create(gem_ctx *root, uint64_t budget, gem_ctx **out) {
   ctx->sms = root->sms;
   for (uint32_t m = 0; m < 3; ++m) ctx->join_bps[m] = root->join_bps[m];
   ctx->pool_bps = root->pool_bps;
+  ctx->hashed_bps = root->hashed_bps;
   ctx->budget = budget;
   ctx->loaded = true;
   ctx->borrowed_graph = true;
@@ -1646,9 +1648,13 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   if (tu.blocks_per_sm && (int)tu.blocks_per_sm < bps) bps = (int)tu.blocks_per_sm;
   bps = std::max(1, bps / (int)std::max(1u, ctx->join_grid_div));
   CU(cudaEventRecord(ctx->ev[6], ctx->s));
-  // the pools' kernel takes the same share of its blocks per SM
+  // the pools' and the hashed depth-first kernels take the same share of
+  // their blocks per SM
+  const int dfs_bps = mode == GEM_MODE_COUNT && ctx->vnh_buckets
+                          ? std::max(1, ctx->hashed_bps * bps / std::max(1, ctx->join_bps[mode]))
+                          : bps;
   const int pool_bps = std::max(1, ctx->pool_bps * bps / std::max(1, ctx->join_bps[mode]));
-  CU(launch_join_graph(ctx->jgraph, a, cap_ms * 1000000ull, (uint32_t)(ctx->sms * bps),
+  CU(launch_join_graph(ctx->jgraph, a, cap_ms * 1000000ull, (uint32_t)(ctx->sms * dfs_bps),
                        (uint32_t)(ctx->sms * pool_bps), ctx->s));
   CU(cudaEventRecord(ctx->ev[7], ctx->s));
   CU(cudaGetLastError());

@@ -144,7 +144,7 @@ struct gem_ctx {
   cudaEvent_t ev[12] = {};
   int sms = 148;
   int join_bps[3] = {1, 1, 1};
-  int pool_bps = 1;                  // blocks per SM of the counting pools
+  int pool_bps = 1, hashed_bps = 1;  // blocks per SM of the counting pools and of the hashed depth-first part
   uint64_t budget = 0, device_bytes = 0;
   std::string err;
   // graph

@@ -278,20 +278,23 @@ __device__ __forceinline__ uint32_t index_of(const JoinArgs &a, const JLevel *__
 // of chains of dependent L2 loads.  A slot is tagged by the list's absolute
 // range in the values array, which identifies the list for the whole launch.
 // ---------------------------------------------------------------------------
-template <bool CACHED>
+// What a counter finds in the warp's shared memory: nothing (the
+// lane-parallel pools, whose prefixes are the lanes' own), the ranges of the
+// lists keyed by the shared prefix, or those and copies of the two longest
+// lists.  Copies serve contexts without a neighbourhood hash only: against
+// the hash, the nine steps of a shared-memory search lose (path [5,1,2,1,5]
+// at scale 22: 491 ms searching copies, 351 ms probing the hash).
+enum : int { LC_NONE = 0, LC_RANGES = 1, LC_COPIES = 2 };
+template <int C>
 struct ListCacheT {
   uint32_t *buf;            // LIST_CACHE_SLOTS * LIST_CACHE_CAP entries
   unsigned long long *tag;  // {lo, hi} per slot
   unsigned long long *rng;  // {lo, hi} of suffix back entries b0 + i (lo ~0: not keyed by the prefix); rng[64] = b0
 };
 
-// CACHED = false: the counters of the lane-parallel pools, whose prefixes are
-// the lanes' own, so that nothing is shared and nothing is cached.
-using ListCache = ListCacheT<true>;
-
-template <bool C>
+template <int C>
 __device__ __forceinline__ int cache_slot(const ListCacheT<C> &lc, uint64_t lo, uint64_t hi) {
-  if (C && hi > lo)
+  if (C == LC_COPIES && hi > lo)
 #pragma unroll
     for (int k = 0; k < (int)LIST_CACHE_SLOTS; ++k)
       if (lc.tag[2 * k] == lo && lc.tag[2 * k + 1] == hi) return k;
@@ -336,7 +339,7 @@ __device__ __forceinline__ uint32_t smem_member8(const uint32_t *b, uint32_t n, 
 // x in list [lo, hi): from the cache slot when there is one, else by binary
 // search of the values array from *cur (lists are probed in ascending x, so
 // the search start only moves forward).
-template <bool C>
+template <int C>
 __device__ __forceinline__ bool list_member(const JoinArgs &a, const ListCacheT<C> &lc, int slot, uint64_t lo,
                                             uint64_t hi, uint64_t &cur, uint32_t x) {
   if (slot >= 0) return smem_contains(lc.buf + slot * LIST_CACHE_CAP, (uint32_t)(hi - lo), x);
@@ -379,8 +382,9 @@ __device__ __forceinline__ uint32_t list_member8(const JoinArgs &a, uint64_t &cu
 
 // Warp-collective: caches the longest suffix lists keyed by levels below L
 // (the prefix is sf/sidx).  Lists already cached stay in their slots.
+template <int C>
 __device__ void cache_suffix_lists(const JoinArgs &a, const JQuery *__restrict__ Q, uint32_t L,
-                                   const uint32_t *sidx, const ListCache &lc, bool copy = true) {
+                                   const uint32_t *sidx, const ListCacheT<C> &lc, bool copy) {
   const uint32_t lane = lane_id();
   const uint32_t n = Q->n, ne = Q->n_enum;
   if (ne >= n || n > QV) {
@@ -407,7 +411,7 @@ __device__ void cache_suffix_lists(const JoinArgs &a, const JQuery *__restrict__
   }
   if (lane == 0) lc.rng[64] = b0;
   __syncwarp();  // every lane reads the range table
-  if (!copy) return;
+  if (C != LC_COPIES || !copy) return;
   uint64_t pick_lo[LIST_CACHE_SLOTS], pick_hi[LIST_CACHE_SLOTS];
 #pragma unroll
   for (int k = 0; k < (int)LIST_CACHE_SLOTS; ++k) {
@@ -469,7 +473,7 @@ __device__ void cache_suffix_lists(const JoinArgs &a, const JQuery *__restrict__
 // warp's shared copy (sf, sidx).  Lists are addressed by index through the
 // members' backward entries, so no per-lane arrays are needed.
 // ---------------------------------------------------------------------------
-template <bool C>
+template <int C>
 struct LaneCtx {
   const JQuery *Q;
   uint32_t L, w, widx;
@@ -481,18 +485,18 @@ struct LaneCtx {
 };
 
 // Vertex and candidate position of prefix level j for this lane.
-template <bool C>
+template <int C>
 __device__ __forceinline__ uint32_t lvl_vertex(const LaneCtx<C> &x, uint32_t j) {
   return j == x.L ? x.w : j == x.ownp ? x.wp : x.sf[j];
 }
-template <bool C>
+template <int C>
 __device__ __forceinline__ uint32_t lvl_index(const LaneCtx<C> &x, uint32_t j) {
   return j == x.L ? x.widx : j == x.ownp ? x.widxp : x.sidx[j];
 }
 
 // List li of the subset `members` of a suffix group: its range, its key
 // vertex (f of the key level) and the level of the member it belongs to.
-template <bool C>
+template <int C>
 __device__ __forceinline__ void lane_list(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                           uint32_t li, uint64_t &lo, uint64_t &hi, uint32_t &kv, uint32_t &mlvl) {
   lo = hi = 0;
@@ -537,7 +541,7 @@ __device__ __forceinline__ bool vnh_list_has(const JoinArgs &a, const JQuery *Q,
 // Lists of one subset, at most three: ranges computed once, cached lists read
 // from shared memory, the others probed through the neighbourhood hash (or
 // searched from a moving start without it).
-template <bool C>
+template <int C>
 __device__ uint64_t lane_subset_count3(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                        uint32_t nl, uint32_t dup_mask, Stats &st, bool &heavy) {
   uint64_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0, lo2 = 0, hi2 = 0;
@@ -642,7 +646,7 @@ __device__ uint64_t lane_subset_count3(const JoinArgs &a, const LaneCtx<C> &x, u
   return c;
 }
 
-template <bool C>
+template <int C>
 __device__ uint64_t lane_subset_count(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                       uint32_t dup_mask, Stats &st, bool &heavy) {
   uint32_t nl = 0;
@@ -703,23 +707,20 @@ __device__ uint64_t lane_subset_count(const JoinArgs &a, const LaneCtx<C> &x, ui
 // FLAT_MAX_VALUES subset values of at most three lists each.
 // ---------------------------------------------------------------------------
 struct FJob {
-  uint64_t s;     // scanned list: start in the values array, or offset in its cache slot
-  uint64_t ra;    // probe a: cached list length, or the first bucket of the key vertex's hash table
+  uint64_t s;     // scanned list: start in the values array
+  uint64_t ra;    // probe a: first bucket of the key vertex's hash table
   uint64_t rb;    // probe b (three-list subsets)
   uint32_t na;    // probe a: buckets of that table
   uint32_t nb;    // probe b
   uint32_t len;   // scanned entries
   uint32_t w;     // the prefix match's vertex at level L (a duplicate candidate)
   uint32_t dup;   // earlier same-label levels
-  uint32_t meta;  // bit 0: three lists; bits 1-2 / 3-4 / 5-6: cache slot + 1 (0: none) of the
-                  // scanned list and of probes a, b; bits 7-11 / 12-16 / 17-21: their member levels
+  uint32_t meta;  // bit 0: three lists; bits 1-5 / 6-10 / 11-15: member levels of the scanned
+                  // list and of probes a, b
 };
 static_assert(sizeof(FJob) == FLAT_JOB_BYTES, "job record size");
 
-__device__ __forceinline__ uint64_t flat_probe_word(const JoinArgs &a, int slot, uint64_t lo, uint64_t hi,
-                                                    uint32_t kv, uint32_t &nb) {
-  nb = 0;
-  if (slot >= 0) return hi - lo;
+__device__ __forceinline__ uint64_t flat_probe_word(const JoinArgs &a, uint32_t kv, uint32_t &nb) {
   const uint64_t b0 = vnh_base(__ldg(a.vnh_off + kv));
   nb = (uint32_t)(vnh_base(__ldg(a.vnh_off + kv + 1)) - b0);
   return b0;
@@ -732,14 +733,10 @@ __device__ __forceinline__ uint32_t flat_blocks(uint64_t s, uint32_t len) {
 }
 
 // Keys among `want` that are in the probed list (word and nb from
-// flat_probe_word, slot1 = cache slot + 1 or 0); keys come from a list of
-// member level sml.
-template <bool C>
-__device__ __forceinline__ uint32_t flat_probe8(const JoinArgs &a, const JQuery *Q, const ListCacheT<C> &lc,
-                                                uint32_t slot1, uint64_t word, uint32_t nb, uint32_t ml,
-                                                uint32_t sml, const uint32_t (&vv)[8], uint32_t want) {
+// flat_probe_word); keys come from a list of member level sml.
+__device__ __forceinline__ uint32_t flat_probe8(const JoinArgs &a, const JQuery *Q, uint64_t word, uint32_t nb,
+                                                uint32_t ml, uint32_t sml, const uint32_t (&vv)[8], uint32_t want) {
   if (!want) return 0;
-  if (C && slot1) return smem_member8(lc.buf + (slot1 - 1) * LIST_CACHE_CAP, (uint32_t)word, vv, want);
   const VnhRow r{a.vnh_buckets + word, nb};
   uint32_t f = vnh_has8(r, vv, want);
   if (ml != sml) {
@@ -760,24 +757,13 @@ struct FlatOrigin {
   uint64_t pos, end;  // the chunk's positions [pos, end) in the source list
 };
 
-// v (any vertex) in a list: its cache slot, the neighbourhood hash with a
-// candidate test, or a binary search.
-template <bool C>
-__device__ __forceinline__ bool list_has_vertex(const JoinArgs &a, const LaneCtx<C> &x, int slot, uint64_t lo,
-                                                uint64_t hi, uint32_t kv, uint32_t ml, uint32_t v) {
-  if (slot >= 0) return smem_contains(x.lc.buf + slot * LIST_CACHE_CAP, (uint32_t)(hi - lo), v);
-  if (a.vnh_buckets) return vnh_list_has(a, x.Q, kv, ml, ~0u, v);
-  uint64_t cur = lo;
-  return list_member(a, x.lc, -1, lo, hi, cur, v);
-}
-
 // Counts the suffix completions of the chunk's prefix matches (lanes in m);
 // *my_cnt receives this lane's.  While the chunk holds more than
 // a.flat_donate_blocks blocks and other warps are idle, the positions of the
 // upper half of its work go to the queue (the recipient evaluates them
 // again) and their lanes count nothing here.  Returns false, having done
 // nothing, when the chunk's jobs do not fit the job table.
-template <bool C>
+template <int C>
 __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx<C> &x, uint32_t m, char *fbase,
                                                 const FlatOrigin &org, const LaneState &c, bool &pushed,
                                                 Stats &st, uint64_t &my_cnt) {
@@ -819,27 +805,17 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
         const uint64_t shi = s == 0 ? hi[0] : s == 1 ? hi[1] : hi[2];
         const uint32_t skv = s == 0 ? kv[0] : s == 1 ? kv[1] : kv[2];
         const uint32_t sml = s == 0 ? ml[0] : s == 1 ? ml[1] : ml[2];
-        const int ss = cache_slot(x.lc, slo, shi);
         if (nl == 1) {
-          uint64_t cnt = shi - slo, cur = slo;
-          for (uint32_t dm = dup; dm; dm &= dm - 1) {
-            const uint32_t j = __ffs(dm) - 1;
-            const uint32_t v = lvl_vertex(x, j);
-            cur = slo;
-            const bool in = ss >= 0 ? list_member(a, x.lc, ss, slo, shi, cur, v)
-                                    : vnh_list_has(a, Q, skv, sml, ~0u, v);
-            if (in) --cnt;
-          }
+          uint64_t cnt = shi - slo;
+          for (uint32_t dm = dup; dm; dm &= dm - 1)
+            if (vnh_list_has(a, Q, skv, sml, ~0u, lvl_vertex(x, __ffs(dm) - 1))) --cnt;
           val[k] = cnt;
           continue;
         }
         // the probed lists: the two (or one) other than s
         const uint32_t ia = s == 0 ? 1 : 0, ib = s == 2 ? 1 : 2;
-        const uint64_t alo = ia == 0 ? lo[0] : lo[1], ahi = ia == 0 ? hi[0] : hi[1];
-        const uint64_t blo = ib == 1 ? lo[1] : lo[2], bhi = ib == 1 ? hi[1] : hi[2];
         const uint32_t akv = ia == 0 ? kv[0] : kv[1], bkv = ib == 1 ? kv[1] : kv[2];
         const uint32_t aml = ia == 0 ? ml[0] : ml[1], bml = ib == 1 ? ml[1] : ml[2];
-        const int sa = cache_slot(x.lc, alo, ahi), sb = nl > 2 ? cache_slot(x.lc, blo, bhi) : -1;
         // With a shared prefix the blocks skip the earlier same-label
         // vertices themselves; with a per-lane level the job counts the whole
         // intersection and those vertices (distinct) found in it are
@@ -847,22 +823,21 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
         uint64_t corr = 0;
         for (uint32_t dm = x.ownp < QV ? dup : 0u; dm; dm &= dm - 1) {
           const uint32_t d = lvl_vertex(x, __ffs(dm) - 1);
-          if (list_has_vertex(a, x, ss, slo, shi, skv, sml, d) && list_has_vertex(a, x, sa, alo, ahi, akv, aml, d) &&
-              (nl < 3 || list_has_vertex(a, x, sb, blo, bhi, bkv, bml, d)))
+          if (vnh_list_has(a, Q, skv, sml, ~0u, d) && vnh_list_has(a, Q, akv, aml, ~0u, d) &&
+              (nl < 3 || vnh_list_has(a, Q, bkv, bml, ~0u, d)))
             ++corr;
         }
         val[k] = corr;
         FJob jb;
-        jb.s = ss >= 0 ? 0 : slo;
+        jb.s = slo;
         jb.len = (uint32_t)(shi - slo);
-        jb.ra = flat_probe_word(a, sa, alo, ahi, akv, jb.na);
+        jb.ra = flat_probe_word(a, akv, jb.na);
         jb.rb = 0;
         jb.nb = 0;
-        if (nl > 2) jb.rb = flat_probe_word(a, sb, blo, bhi, bkv, jb.nb);
+        if (nl > 2) jb.rb = flat_probe_word(a, bkv, jb.nb);
         jb.w = x.w;
         jb.dup = x.ownp < QV ? 0u : dup;
-        jb.meta = (nl > 2 ? 1u : 0u) | ((uint32_t)(ss + 1) << 1) | ((uint32_t)(sa + 1) << 3) |
-                  ((uint32_t)(sb + 1) << 5) | ((sml & 31u) << 7) | ((aml & 31u) << 12) | ((bml & 31u) << 17);
+        jb.meta = (nl > 2 ? 1u : 0u) | ((sml & 31u) << 1) | ((aml & 31u) << 6) | ((bml & 31u) << 11);
         jobs[jbase + jn] = jb;
         res[jbase + jn] = 0;
         my_blocks += flat_blocks(jb.s, jb.len);
@@ -925,14 +900,12 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
       }
       cur_j = lo;
       const FJob jb = jobs[lo];
-      const uint32_t ss1 = C ? (jb.meta >> 1) & 3u : 0u, sa1 = (jb.meta >> 3) & 3u, sb1 = (jb.meta >> 5) & 3u;
-      const uint32_t sml = (jb.meta >> 7) & 31u, aml = (jb.meta >> 12) & 31u, bml = (jb.meta >> 17) & 31u;
+      const uint32_t sml = (jb.meta >> 1) & 31u, aml = (jb.meta >> 6) & 31u, bml = (jb.meta >> 11) & 31u;
       // the block's sector: two 16-byte loads (the values array is a whole
       // number of sectors), the entries outside the list masked
       const uint64_t p0 = ((jb.s >> 3) + (bid - start[lo])) << 3;
-      const uint4 *sec = reinterpret_cast<const uint4 *>(ss1 ? x.lc.buf + (ss1 - 1) * LIST_CACHE_CAP + p0
-                                                             : a.values + p0);
-      const uint4 v0 = ss1 ? sec[0] : __ldg(sec), v1 = ss1 ? sec[1] : __ldg(sec + 1);
+      const uint4 *sec = reinterpret_cast<const uint4 *>(a.values + p0);
+      const uint4 v0 = __ldg(sec), v1 = __ldg(sec + 1);
       const uint32_t vv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
       const uint32_t skip = p0 < jb.s ? (uint32_t)(jb.s - p0) : 0u;
       const uint64_t left = jb.s + jb.len - p0;
@@ -946,7 +919,7 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
       }
 #pragma unroll 1
       for (uint32_t pr = 0; pr <= (jb.meta & 1u); ++pr)
-        okm = flat_probe8(a, Q, x.lc, pr ? sb1 : sa1, pr ? jb.rb : jb.ra, pr ? jb.nb : jb.na, pr ? bml : aml, sml, vv, okm);
+        okm = flat_probe8(a, Q, pr ? jb.rb : jb.ra, pr ? jb.nb : jb.na, pr ? bml : aml, sml, vv, okm);
       cur_c += __popc(okm);
     }
   }
@@ -993,7 +966,7 @@ __device__ __forceinline__ bool flat_lane_chunk(const JoinArgs &a, const LaneCtx
 
 // Suffix completions of one lane's prefix match; sets `heavy` (and returns
 // 0) when an intersection is too long for one lane.
-template <bool C>
+template <int C>
 __device__ uint64_t lane_suffix_count(const JoinArgs &a, const LaneCtx<C> &x, Stats &st, bool &heavy) {
   const JQuery *Q = x.Q;
   uint64_t total = 1;
@@ -1036,7 +1009,7 @@ __device__ uint64_t lane_suffix_count(const JoinArgs &a, const LaneCtx<C> &x, St
 // Warp-cooperative form for one deferred (heavy) prefix match: every lane
 // receives the same context; lists are spread one per lane and the shortest
 // is scanned 32 entries at a time.
-template <bool C>
+template <int C>
 __device__ uint64_t warp_subset_count(const JoinArgs &a, const LaneCtx<C> &x, uint32_t first, uint32_t members,
                                       uint32_t dup_mask, Stats &st) {
   const uint32_t lane = lane_id();
@@ -1150,7 +1123,7 @@ __device__ uint64_t warp_subset_count(const JoinArgs &a, const LaneCtx<C> &x, ui
   return cnt;
 }
 
-template <bool C>
+template <int C>
 __device__ uint64_t warp_suffix_count(const JoinArgs &a, const LaneCtx<C> &x, Stats &st) {
   const JQuery *Q = x.Q;
   uint64_t total = 1;
@@ -1417,16 +1390,23 @@ __device__ __forceinline__ void emit_last(const JoinArgs &a, const JQuery *__res
 // stack nor cached lists.  PART_DFS: the ordinary pool and the task queue.
 // The enumerating modes run both in one kernel (their pool holds the
 // single-vertex queries only).
-enum : uint32_t { PART_POOLS = 1, PART_DFS = 2 };
+// PART_HASHED: the depth-first part with a neighbourhood hash, which keeps no
+// list copies.
+enum : uint32_t { PART_POOLS = 1, PART_DFS = 2, PART_HASHED = 4 };
 
 // Dynamic shared memory of a join block: the list caches and job tables that
 // only counting uses, the job tables alone in the pools.
 static uint32_t join_smem(uint32_t mode, uint32_t part) {
-  return mode != MODE_COUNT ? 0u : part == PART_POOLS ? JOIN_WARPS_PER_BLOCK * FLAT_WARP_BYTES : JOIN_DYN_SMEM;
+  return mode != MODE_COUNT     ? 0u
+         : part == PART_POOLS   ? JOIN_WARPS_PER_BLOCK * FLAT_WARP_BYTES
+         : part & PART_HASHED   ? JOIN_WARPS_PER_BLOCK * (FLAT_WARP_BYTES + SUFFIX_RANGE_BYTES)
+                                : JOIN_DYN_SMEM;
 }
 
 template <uint32_t MODE, uint32_t PART>
-__global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) join_kernel(JoinArgs a) {
+__global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART & PART_HASHED ? HASHED_BLOCKS : 2)
+    join_kernel(JoinArgs a) {
+  constexpr int LC = PART & PART_HASHED ? LC_RANGES : LC_COPIES;
   const uint32_t lane = lane_id();
   JControl *ctl = a.ctl;
   const uint64_t deadline = ctl->deadline_ns;
@@ -1434,14 +1414,17 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
   __shared__ unsigned long long s_ctag[JOIN_WARPS_PER_BLOCK][2 * LIST_CACHE_SLOTS];
   extern __shared__ __align__(16) uint32_t s_lcache[];  // JOIN_DYN_SMEM bytes: per warp LIST_CACHE_SLOTS lists
   uint32_t *sf = s_pref[threadIdx.x >> 5][0], *sidx = s_pref[threadIdx.x >> 5][1];
-  ListCache lc;
-  // per warp: the list cache, then the balanced-counting job table
-  lc.buf = s_lcache + (threadIdx.x >> 5) * (JOIN_WARP_SMEM / 4);
-  char *fbuf = PART == PART_POOLS ? reinterpret_cast<char *>(s_lcache) + (threadIdx.x >> 5) * FLAT_WARP_BYTES
-                                  : reinterpret_cast<char *>(lc.buf + LIST_CACHE_SLOTS * LIST_CACHE_CAP);
+  ListCacheT<LC> lc;
+  // per warp: the list copies (LC_COPIES), the balanced-counting job table,
+  // the suffix ranges
+  constexpr uint32_t copies = LC == LC_COPIES && PART != PART_POOLS ? LIST_CACHE_SLOTS * LIST_CACHE_CAP * 4 : 0;
+  char *wbuf = reinterpret_cast<char *>(s_lcache) +
+               (threadIdx.x >> 5) * (copies + FLAT_WARP_BYTES + (PART == PART_POOLS ? 0 : SUFFIX_RANGE_BYTES));
+  lc.buf = reinterpret_cast<uint32_t *>(wbuf);
+  char *fbuf = wbuf + copies;
   lc.rng = reinterpret_cast<unsigned long long *>(fbuf + FLAT_WARP_BYTES);
   lc.tag = s_ctag[threadIdx.x >> 5];
-  const ListCacheT<false> nolc{};
+  const ListCacheT<LC_NONE> nolc{};
   if (MODE == MODE_COUNT && (PART & PART_DFS)) {
     lc.rng[2 * lane] = ~0ull;
     if (lane == 0) lc.rng[64] = 0;
@@ -1508,7 +1491,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
                 if (s < a.emb_cap) a.emb[s] = w0;
               }
             } else if (MODE == MODE_COUNT) {  // a suffix: count mode's plans only
-              LaneCtx<false> x;
+              LaneCtx<LC_NONE> x;
               x.Q = Q;
               x.L = 0;
               x.w = w0;
@@ -1531,7 +1514,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
       for (uint32_t hm = MODE == MODE_COUNT ? __ballot_sync(FULL, heavy) : 0u; hm; hm &= hm - 1) {
         const uint32_t hl = __ffs(hm) - 1;
         const uint32_t qh = __shfl_sync(FULL, hq, hl);
-        LaneCtx<false> x;
+        LaneCtx<LC_NONE> x;
         x.Q = a.queries + qh;
         x.L = 0;
         x.w = __shfl_sync(FULL, hw, hl);
@@ -1610,7 +1593,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
         }
       }
       const uint32_t m = __ballot_sync(FULL, valid);
-      LaneCtx<false> x;
+      LaneCtx<LC_NONE> x;
       x.Q = Q;
       x.L = 1;
       x.w = f1;
@@ -1632,7 +1615,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
         cnt = valid ? lane_suffix_count(a, x, st, heavy) : 0;
         for (uint32_t hm = __ballot_sync(FULL, heavy); hm; hm &= hm - 1) {
           const uint32_t hl = __ffs(hm) - 1;
-          LaneCtx<false> y = x;
+          LaneCtx<LC_NONE> y = x;
           y.w = __shfl_sync(FULL, f1, hl);
           y.widx = __shfl_sync(FULL, i1, hl);
           y.wp = __shfl_sync(FULL, f0, hl);
@@ -1886,8 +1869,8 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
             filled_epoch = epoch;
           }
           bool flat_done = false;
-          if (Q->flat && a.vnh_buckets) {
-            LaneCtx<true> x;
+          if ((PART & PART_HASHED) && Q->flat) {
+            LaneCtx<LC> x;
             x.Q = Q;
             x.L = lvl;
             x.w = w;
@@ -1909,7 +1892,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
           uint32_t widx = 0;
           uint64_t my_cnt = 0;
           if (!flat_done && ((m >> lane) & 1u)) {
-            LaneCtx<true> x;
+            LaneCtx<LC> x;
             x.Q = Q;
             x.L = lvl;
             x.w = w;
@@ -1942,7 +1925,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : 2) joi
           lane_cnt += my_cnt;
           for (; hm; hm &= hm - 1) {
             const uint32_t hl = __ffs(hm) - 1;
-            LaneCtx<true> x;
+            LaneCtx<LC> x;
             x.Q = Q;
             x.L = lvl;
             x.w = __shfl_sync(FULL, w, hl);
@@ -2130,7 +2113,9 @@ __global__ void join_prepare_kernel(JControl *ctl, JOut *out, uint32_t nquery, J
 
 static void *join_fn(uint32_t mode, uint32_t part) {
   if (mode == MODE_COUNT)
-    return part == PART_POOLS ? (void *)join_kernel<MODE_COUNT, PART_POOLS> : (void *)join_kernel<MODE_COUNT, PART_DFS>;
+    return part == PART_POOLS               ? (void *)join_kernel<MODE_COUNT, PART_POOLS>
+           : part == (PART_DFS | PART_HASHED) ? (void *)join_kernel<MODE_COUNT, PART_DFS | PART_HASHED>
+                                              : (void *)join_kernel<MODE_COUNT, PART_DFS>;
   return mode == MODE_HASH ? (void *)join_kernel<MODE_HASH, PART_POOLS | PART_DFS>
                            : (void *)join_kernel<MODE_ENUM, PART_POOLS | PART_DFS>;
 }
@@ -2139,7 +2124,7 @@ static void *join_fn(uint32_t mode, uint32_t part) {
 // above the default 48 KiB limit: the counting instances opt in once.
 static cudaError_t join_smem_optin() {
   static cudaError_t done = [] {
-    for (uint32_t part : {PART_POOLS, PART_DFS}) {
+    for (uint32_t part : {(uint32_t)PART_POOLS, (uint32_t)PART_DFS, (uint32_t)PART_DFS | PART_HASHED}) {
       const cudaError_t e = cudaFuncSetAttribute(join_fn(MODE_COUNT, part), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)join_smem(MODE_COUNT, part));
       if (e != cudaSuccess) return e;
@@ -2162,6 +2147,7 @@ static int blocks_per_sm(uint32_t mode, uint32_t part) {
 }
 
 int join_blocks_per_sm(uint32_t mode) { return blocks_per_sm(mode, PART_DFS); }
+int join_hashed_blocks_per_sm() { return blocks_per_sm(MODE_COUNT, PART_DFS | PART_HASHED); }
 int join_pool_blocks_per_sm() { return blocks_per_sm(MODE_COUNT, PART_POOLS); }
 
 void destroy_join_graph(JoinGraph &jg) {
@@ -2202,12 +2188,13 @@ cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns,
     kp[nk].kernelParams = params;
     ++nk;
   };
+  const uint32_t part = split && a.vnh_buckets ? (uint32_t)PART_DFS | PART_HASHED : (uint32_t)PART_DFS;
   node((void *)join_prepare_kernel, 32, 0, prep_params);
   if (pools) node(join_fn(a.mode, PART_POOLS), pool_grid, join_smem(a.mode, PART_POOLS), join_params);
-  if (dfs) node(join_fn(a.mode, PART_DFS), grid, join_smem(a.mode, PART_DFS), join_params);
+  if (dfs) node(join_fn(a.mode, part), grid, join_smem(a.mode, part), join_params);
   cudaError_t e;
   if ((e = join_smem_optin()) != cudaSuccess) return e;
-  JoinGraph::Shape &g = jg.shape[a.mode == MODE_COUNT ? (pools ? 1 : 0) + (dfs ? 2 : 0) : 3 + a.mode];
+  JoinGraph::Shape &g = jg.shape[split ? (pools ? 1 : 0) + (dfs ? 2 : 0) + (a.vnh_buckets ? 4 : 0) : 7 + a.mode];
   if (!g.exec) {
     if ((e = cudaGraphCreate(&g.graph, 0)) != cudaSuccess) return e;
     for (uint32_t i = 0; i < nk; ++i)

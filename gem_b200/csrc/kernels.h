@@ -435,13 +435,15 @@ struct JoinGraph {
     cudaGraphExec_t exec = nullptr;
     cudaGraphNode_t node[3] = {nullptr, nullptr, nullptr};
   };
-  Shape shape[6];  // counting: pools | depth-first part << 1; then the hash and enumerate modes
+  Shape shape[10];  // counting: pools | depth-first part << 1 | with hash << 2; then the hash and enumerate modes
 };
-constexpr int POOL_BLOCKS = 3;  // blocks per SM of the pools' kernel
+constexpr int POOL_BLOCKS = 3;    // blocks per SM of the pools' kernel
+constexpr int HASHED_BLOCKS = 2;  // and of the depth-first part with the hash
 cudaError_t launch_join_graph(JoinGraph &jg, const JoinArgs &a, uint64_t cap_ns, uint32_t grid, uint32_t pool_grid,
                               cudaStream_t s);
 void destroy_join_graph(JoinGraph &jg);
 int join_blocks_per_sm(uint32_t mode);
 int join_pool_blocks_per_sm();
+int join_hashed_blocks_per_sm();
 
 }  // namespace gem
