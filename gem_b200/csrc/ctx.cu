@@ -818,6 +818,55 @@ static uint32_t flat_code(const Plan &p, int mode) {
   return nval <= FLAT_MAX_VALUES ? nval | (nscan << 8) : 0;
 }
 
+// Whether some automorphism of q (labels kept) exchanges u and w, by a
+// backtracking search; `steps` counts down the assignments tried.
+constexpr uint32_t SWAP_STEPS = 2000;
+static bool swaps(const HostQuery &q, uint32_t u, uint32_t w, uint32_t &steps) {
+  // vertices in an order that keeps each (after the first two) next to an earlier one
+  uint32_t order[GEM_MAX_QV] = {u, w}, n = 2, seen = 1u << u | 1u << w;
+  for (uint32_t i = 0; i < n; ++i)
+    for (uint32_t x = q.adj[order[i]] & ~seen; x; x &= x - 1) {
+      order[n++] = (uint32_t)__builtin_ctz(x);
+      seen |= 1u << order[n - 1];
+    }
+  uint32_t image[GEM_MAX_QV], used = 1u << u | 1u << w;
+  image[u] = w;
+  image[w] = u;
+  std::function<bool(uint32_t)> rec = [&](uint32_t k) {
+    if (k == n) return true;
+    const uint32_t x = order[k];
+    for (uint32_t y = 0; y < q.nv; ++y) {
+      if ((used >> y & 1u) || q.lab[y] != q.lab[x] || q.deg(y) != q.deg(x)) continue;
+      if (steps == 0) return false;
+      --steps;
+      bool ok = true;
+      for (uint32_t i = 0; i < k && ok; ++i)
+        ok = (q.adj[x] >> order[i] & 1u) == (q.adj[y] >> image[order[i]] & 1u);
+      if (!ok) continue;
+      image[x] = y;
+      used |= 1u << y;
+      if (rec(k + 1)) return true;
+      used &= ~(1u << y);
+    }
+    return false;
+  };
+  return n == q.nv && rec(2);
+}
+
+// Two enumerated levels i < j of a plan (the smallest j) that an automorphism
+// exchanges, or false.  Embeddings with f(i) < f(j) and with f(i) > f(j) are
+// then equally many: the automorphism turns each into the other.
+static bool mirror_levels(const HostQuery &q, const Plan &p, const std::vector<uint32_t> &row_of, uint32_t &i,
+                          uint32_t &j) {
+  uint32_t steps = SWAP_STEPS;
+  for (j = 1; j < p.n_enum; ++j)
+    for (i = 0; i < j; ++i) {
+      const uint32_t u = p.order[i], w = p.order[j];
+      if (q.lab[u] == q.lab[w] && q.deg(u) == q.deg(w) && row_of[u] == row_of[w] && swaps(q, u, w, steps)) return true;
+    }
+  return false;
+}
+
 // Queries counted through the (root, first level) pair pool: count mode, an
 // enumerated prefix of a root and one neighbour level, a closed-form suffix
 // eligible for balanced counting, and the neighbourhood hash.
@@ -1566,6 +1615,11 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
         b.off = w.edges[ei].offsets;
         jb.push_back(b);
       }
+    }
+    uint32_t mi, mj;
+    if (mode == GEM_MODE_COUNT && mirror_levels(w.q[qi], p, w.row_of[qi], mi, mj)) {
+      J.mirror = 1;
+      J.lv[mj].above = mi + 1;
     }
     w.jq_index[qi] = (uint32_t)jq.size();
     if (J.n == 1 || (mode == GEM_MODE_COUNT && J.n_enum == 1)) {

@@ -236,7 +236,8 @@ __device__ __noinline__ uint32_t vnh_has8_call(VnhRow r, uint4 lo, uint4 hi, uin
 // (f_j, w); without it, a binary search of the list.
 __device__ __forceinline__ uint32_t eval_chunk(const JoinArgs &a, uint64_t cpos, uint64_t end, uint32_t nback,
                                                uint32_t src, uint64_t my_lo, uint64_t my_hi, uint32_t my_kv,
-                                               uint32_t dup_mask, const LaneState &c, uint32_t *w_out, Stats &st) {
+                                               uint32_t dup_mask, uint32_t above, const LaneState &c, uint32_t *w_out,
+                                               Stats &st) {
   const uint32_t lane = lane_id();
   const uint64_t e = cpos + lane;
   bool ok = e < end;
@@ -251,6 +252,10 @@ __device__ __forceinline__ uint32_t eval_chunk(const JoinArgs &a, uint64_t cpos,
     const uint32_t j = __ffs(dm) - 1;
     const uint32_t fj = __shfl_sync(FULL, c.f, j);
     if (w == fj) ok = false;
+  }
+  if (above) {
+    const uint32_t fa = __shfl_sync(FULL, c.f, above - 1);
+    if (w < fa) ok = false;
   }
   if (lane == 0) {
     const uint64_t k = (end - cpos) < 32 ? (end - cpos) : 32;
@@ -1333,7 +1338,7 @@ __device__ void abandon(const JoinArgs &a, uint32_t q) {
 
 // Item r of the ordinary pool: a root of its query, or (JQuery::pairs) an
 // entry of the query's root table, which is a root and a first-level vertex.
-// k0 = 0xFFFFFFFF: a bounds check failed.
+// k0 = 0xFFFFFFFF: nothing to count here (or a bounds check failed).
 template <uint32_t MODE>
 __device__ __forceinline__ void root_item(const JoinArgs &a, uint64_t r, uint32_t &q, uint32_t &f0, uint32_t &k0,
                                           uint32_t &f1, uint32_t &k1) {
@@ -1356,6 +1361,7 @@ __device__ __forceinline__ void root_item(const JoinArgs &a, uint64_t r, uint32_
   if (!inb(a, SITE_ROOT, kr, Q->n_root)) return;
   f1 = __ldg(a.values + p);
   f0 = __ldg(Q->root_cand + kr);
+  if (L1->above && f0 > f1) return;  // counted with (f1, f0)
   k1 = index_of(a, L1, f1);
   k0 = kr;
 }
@@ -1590,6 +1596,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
           f0 = __ldg(Q->root_cand + k0);
           f1 = __ldg(a.values + p);
           i1 = index_of(a, L1, f1);
+          if (L1->above && f0 > f1) valid = false;
         }
       }
       const uint32_t m = __ballot_sync(FULL, valid);
@@ -1627,7 +1634,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
 #pragma unroll
       for (int d = 16; d; d >>= 1) cnt += __shfl_xor_sync(FULL, cnt, d);
       if (lane == 0) {
-        if (cnt) atomicAdd(&a.out[q].count, (unsigned long long)cnt);
+        if (cnt) atomicAdd(&a.out[q].count, (unsigned long long)cnt << Q->mirror);
         st.nodes += __popc(m);
       }
       if (err_set(a)) {
@@ -1768,7 +1775,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
       lvl = 0;
       base_lvl = 1;
       ++epoch;
-      if (k0 != 0xFFFFFFFFu) {  // not a failed bounds check
+      if (k0 != 0xFFFFFFFFu) {
         const uint64_t h0 = MODE == MODE_COUNT ? 0ull : emb_term(Q->root_u, f0);
         if (lane == 0) {
           c.f = f0;
@@ -1826,7 +1833,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
         level_ranges(a, L, c, nb, lo, hi, &kv);
         const uint32_t src = __shfl_sync(FULL, c.src, lvl);
         uint32_t w;
-        const uint32_t m = eval_chunk(a, pos, end, nb, src, lo, hi, kv, L->dup_mask, c, &w, st);
+        const uint32_t m = eval_chunk(a, pos, end, nb, src, lo, hi, kv, L->dup_mask, L->above, c, &w, st);
         if (MODE != MODE_COUNT && lvl == n - 1) {
           emit_last<MODE>(a, Q, lvl, m, w, c, lane_cnt, lane_hash);
           if (lane == lvl) c.pos = pos + 32;
@@ -2026,7 +2033,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
           for (uint32_t k = q; k <= q1; ++k) atomicOr(&a.out[k].pad[0], 1ull);
         }
       }
-      if (tc) atomicAdd(&a.out[q].count, (unsigned long long)tc);
+      if (tc) atomicAdd(&a.out[q].count, (unsigned long long)tc << Q->mirror);
       if (MODE != MODE_COUNT && th) atomicAdd(&a.out[q].hash, (unsigned long long)th);
       if (release) {
         if (pushed) __threadfence();  // donated tasks are visible before quiescence can be observed

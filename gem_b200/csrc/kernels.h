@@ -280,7 +280,7 @@ struct JLevel {
   uint32_t back_base;  // first entry in the JBack array
   uint32_t dup_mask;   // earlier levels with the same label (injectivity)
   uint32_t idx_kind;   // how this level's vertex finds its position in C(u)
-  uint32_t pad;
+  uint32_t above;      // 0, or 1 + the level whose vertex this level's must be above (JQuery::mirror)
   const uint64_t *rb;          // IDX_RANK
   const CuckooTable *ck;       // IDX_CUCKOO
 };
@@ -327,6 +327,11 @@ struct JQuery {
                              // (bits 0-7; 0 = not eligible) and those needing a scan (bits 8-15)
   uint32_t pool;             // its items are in the ordinary pool
   uint32_t pairs;            // items of the ordinary pool: (root, first level) pairs instead of roots
+  // Counting a query with an automorphism that exchanges two enumerated
+  // levels: only embeddings whose later level's vertex is above the earlier's
+  // (JLevel::above) are counted, twice.
+  uint32_t mirror;
+  uint32_t pad;
   uint32_t grp_first[MAX_GROUPS];
   uint32_t grp_size[MAX_GROUPS];
   uint32_t term_base[MAX_GROUPS];

@@ -117,3 +117,23 @@ def test_scan_limit(nv):
         assert c.run(gem.Query([0, 0, 0], [(0, 1), (1, 2)]))["count"] == 2 * nv
         off, vals = c.edge_table(gem.Query([0, 0], [(0, 1)]), 0, 1)
         assert np.array_equal(off, 2 * np.arange(nv + 1, dtype=np.uint64)) and len(vals) == 2 * nv
+
+
+# queries with an automorphism that exchanges two enumerated levels (counted by one of the two orders, twice), next to
+# ones that only look like it
+@pytest.mark.parametrize("labels,edges", [
+    ([0, 1, 1, 0], "01 12 23"), ([0, 1, 1, 2], "01 12 23"), ([0, 0, 0, 0], "01 12 23"), ([0, 1, 0, 1], "01 12 23 03"),
+    ([0, 1, 0, 2], "01 12 23 03"), ([0, 0, 0], "01 12 02"), ([1, 0, 0, 2], "01 02 12 13 23"),
+    ([0, 0, 0, 0], "01 02 03 12 13 23"), ([2, 1, 0, 1, 2], "01 12 23 34"), ([2, 1, 0, 1, 0], "01 12 23 34"),
+    ([0, 1, 0, 1, 2], "01 12 23 03 24"), ([0, 1, 1, 0, 2, 2], "01 12 23 14 25"), ([0, 1, 1, 0, 2], "01 12 23 14")])
+def test_symmetric_queries(labels, edges):
+    g = cut(gem.HostGraph.rmat(10, 6, seed=23), 777).set_labels(3, 0.0, seed=11)
+    q = gem.Query(labels, [(int(e[0]), int(e[1])) for e in edges.split()])
+    exp, h, ok = oracle.count(g, q, want_hash=True, work_cap=2_000_000_000)
+    assert ok and exp > 0
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        assert c.run(q)["count"] == exp
+        r = c.run(q, mode=gem.MODE_HASH)
+        assert (r["count"], r["emb_hash"]) == (exp, h)
+        assert [r["count"] for r in c.batch([q] * 40)[1]] == [exp] * 40
