@@ -1343,6 +1343,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // partition by partition with the copy of the next partition (side
   // stream, the other staging buffer) overlapping the kernel of the current one.
   auto table_pass = [&](bool write) -> gem_status {
+    const bool units = write || table_count_tiles(w.W, (uint32_t)w.labels.size(), vtiles, vunits) > 1;
     VPass P;
     std::memset(&P, 0, sizeof P);
     P.next = d_next + write;
@@ -1350,7 +1351,8 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.nbr = ctx->g.nbr;
     P.arc_shift = 0;
     P.t0 = 0;
-    P.t1 = write ? vunits : vtiles;
+    P.t1 = units ? vunits : vtiles;
+    P.units = units;
     P.end = bounded ? d_vtg + nv : nullptr;
     P.vt = d_vt;
     P.vg = d_vg;
@@ -1388,8 +1390,8 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
       CU(cudaStreamWaitEvent(ctx->s, ctx->ev_ready[b], 0));
       P.nbr = ctx->d_stage[b];
       P.arc_shift = a0;
-      P.t0 = write ? pstart_w[p] : pstart[p];
-      P.t1 = write ? pstart_w[p + 1] : pstart[p + 1];
+      P.t0 = units ? pstart_w[p] : pstart[p];
+      P.t1 = units ? pstart_w[p + 1] : pstart[p + 1];
       CU(cudaMemsetAsync(P.next, 0, sizeof *P.next, ctx->s));
       launch_table_vtx(P, write, ctx->s);
       CU(cudaEventRecord(ctx->ev_free[b], ctx->s));

@@ -156,7 +156,7 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// The table passes over vertex tiles.  One warp per tile (32 arcs of one
+// The table passes over vertex tiles.  One warp per unit (G tiles of 32 arcs of one
 // vertex v): the arcs are read once for every source whose candidates hold
 // v.  Those sources are the set bits of v's source column; the warp takes
 // them 32 at a time, one per lane, and each lane computes its source's key
@@ -194,15 +194,14 @@ struct VRec {
 // Columns hold a vertex's bits for the rows of its own label only: a few
 // words per vertex where one bit per target row of the wave was 80 words (320
 // bytes staged per arc) for 180 mixed-size queries, count pass 4.2 -> 1.0 ms.
-template <bool WRITE, bool ONE>
+template <bool WRITE, bool ONE, uint32_t G>
 __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
-  constexpr uint32_t G = WRITE ? TAB_WGROUP : 1u;  // tiles of one vertex per unit
-  extern __shared__ uint32_t stage[];  // count: 32 columns per warp
+  extern __shared__ uint32_t stage[];  // count: 32 columns per tile and warp
   __shared__ VRec rec[WRITE ? 8 : 1][32 * G];  // write: the records of one round
-  __shared__ uint32_t larcs[WRITE || ONE ? 1 : 8][NLC_MAX_LABELS];  // count: the tile's arcs to each label
+  __shared__ uint32_t larcs[WRITE || ONE ? 1 : 8][G][NLC_MAX_LABELS];  // count: a tile's arcs to each label
   const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t *vmap = WRITE ? P.vg : P.vt;
-  constexpr uint32_t half = WRITE ? 32 : 0;  // a vertex's first unit in its word of vtg
+  const uint32_t *vmap = G > 1 ? P.vg : P.vt;
+  constexpr uint32_t half = G > 1 ? 32 : 0;  // a vertex's first unit in its word of vtg
   // units are taken in order from one counter, so the units in flight
   // stay a narrow window of consecutive vertices
   unsigned long long got = 0;
@@ -223,34 +222,45 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
       const uint64_t arc = a0 + (c + i) * 32u + lane;
       xs[i] = i < nt && arc < a1 ? __ldg(P.nbr + (arc - P.arc_shift)) : 0u;
     }
-    const uint32_t nvalid = a1 - a0 - c * 32u < 32u ? (uint32_t)(a1 - a0 - c * 32u) : 32u;  // valid lanes: a prefix
+    // the valid lanes of tile i are a prefix of nvalid(i)
+    const uint64_t left = a1 - a0 - c * 32u;
+    auto nvalid = [&](uint32_t i) -> uint32_t {
+      return left <= i * 32u ? 0u : left - i * 32u < 32u ? (uint32_t)(left - i * 32u) : 32u;
+    };
     const RowLabel vl = ONE ? RowLabel{0, 0, 1, 0} : find_label(P.labels, P.nlab, __ldg(P.lab + v));
-    uint32_t *wst = stage + (uint64_t)warp * 32u * P.W;
-    uint32_t xl = 0xFFFFFFFFu, xc = 0;
-    const uint32_t x = xs[0];
+    uint32_t *wst = stage + (uint64_t)warp * G * 32u * P.W;
+    uint32_t xl[G], xc[G];
     if (!WRITE && ONE) {
-      if (lane < nvalid) xc = __ldg(P.cols + x);
-    } else if (!WRITE) {
-      // stage the columns of the tile's arcs, with asynchronous 16-byte copies
-      // (all in flight at once) when they are whole 16-byte chunks
-      if (lane < nvalid) xl = __ldg(P.lab + x);
-      __syncwarp();  // the previous tile's reads of the stage are done
-      if (P.W >= 4) {
-        const uint32_t ch = P.W >> 2;  // chunks per column
-        for (uint32_t g = lane; g < ((nvalid * ch + 31u) & ~31u); g += 32) {
-          const uint32_t l = g / ch, q = g - l * ch;
-          const uint32_t xa = __shfl_sync(dev::FULL, x, l & 31u);
-          if (l < nvalid) cp_async16(wst + l * P.W + q * 4u, P.cols + (uint64_t)xa * P.W + q * 4u);
-        }
-      } else if (lane < nvalid) {
-        for (uint32_t q = 0; q < P.W; ++q) wst[lane * P.W + q] = __ldg(P.cols + (uint64_t)x * P.W + q);
-      }
-      if (P.nlabels <= NLC_MAX_LABELS) {
 #pragma unroll
-        for (uint32_t l = 0; l < NLC_MAX_LABELS; l += 32) larcs[warp][l + lane] = 0;
-        __syncwarp();
-        const uint32_t peers = __match_any_sync(dev::FULL, xl);
-        if (lane < nvalid && lane == (uint32_t)__ffs(peers) - 1) larcs[warp][xl] = peers;
+      for (uint32_t i = 0; i < G; ++i) xc[i] = lane < nvalid(i) ? __ldg(P.cols + xs[i]) : 0u;
+    } else if (!WRITE) {
+      // stage the columns of the tiles' arcs, with asynchronous 16-byte copies
+      // (all in flight at once) when they are whole 16-byte chunks
+#pragma unroll
+      for (uint32_t i = 0; i < G; ++i) xl[i] = lane < nvalid(i) ? __ldg(P.lab + xs[i]) : 0xFFFFFFFFu;
+      __syncwarp();  // the previous unit's reads of the stage are done
+#pragma unroll
+      for (uint32_t i = 0; i < G; ++i) {
+        const uint32_t nv = nvalid(i), x = xs[i];
+        if (nv == 0) break;
+        uint32_t *st = wst + i * 32u * P.W;
+        if (P.W >= 4) {
+          const uint32_t ch = P.W >> 2;  // chunks per column
+          for (uint32_t g = lane; g < ((nv * ch + 31u) & ~31u); g += 32) {
+            const uint32_t l = g / ch, q = g - l * ch;
+            const uint32_t xa = __shfl_sync(dev::FULL, x, l & 31u);
+            if (l < nv) cp_async16(st + l * P.W + q * 4u, P.cols + (uint64_t)xa * P.W + q * 4u);
+          }
+        } else if (lane < nv) {
+          for (uint32_t q = 0; q < P.W; ++q) st[lane * P.W + q] = __ldg(P.cols + (uint64_t)x * P.W + q);
+        }
+        if (P.nlabels <= NLC_MAX_LABELS) {
+#pragma unroll
+          for (uint32_t l = 0; l < NLC_MAX_LABELS; l += 32) larcs[warp][i][l + lane] = 0;
+          __syncwarp();
+          const uint32_t peers = __match_any_sync(dev::FULL, xl[i]);
+          if (lane < nv && lane == (uint32_t)__ffs(peers) - 1) larcs[warp][i][xl[i]] = peers;
+        }
       }
       cp_async_wait_all();
       __syncwarp();
@@ -311,37 +321,50 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
           const VEdge E = have ? P.vedge[pe] : VEdge{0, 0, 0};
           const uint64_t maddr = E.tile_base + plt;
           if (!WRITE) {
-            uint32_t m = 0;
-            if (ONE) {  // one ballot per pair
+            uint32_t m[G];
+#pragma unroll
+            for (uint32_t g = 0; g < G; ++g) m[g] = 0;
+            if (ONE) {  // one ballot per pair and tile
               const uint32_t np = npairs - pb < 32u ? npairs - pb : 32u;
               for (uint32_t i = 0; i < np; ++i) {
-                const uint32_t bal = __ballot_sync(dev::FULL, (xc >> (__shfl_sync(dev::FULL, E.tcol, i) & 31u)) & 1u);
-                if (lane == i) m = bal;
-              }
-            } else {
-              // the tile's arcs whose target has the pair's target label
-              uint32_t am = 0;
-              if (P.nlabels <= NLC_MAX_LABELS) {
-                am = larcs[warp][E.tlab & (NLC_MAX_LABELS - 1)];
-              } else {  // one ballot per distinct label among them
-                for (uint32_t left = nvalid == 32u ? dev::FULL : (1u << nvalid) - 1u; left;) {
-                  const uint32_t ll = __shfl_sync(dev::FULL, xl, __ffs(left) - 1);
-                  const uint32_t bal = __ballot_sync(dev::FULL, xl == ll) & left;
-                  if (ll == E.tlab) am = bal;
-                  left &= ~bal;
+                const uint32_t tc = __shfl_sync(dev::FULL, E.tcol, i) & 31u;
+#pragma unroll
+                for (uint32_t g = 0; g < G; ++g) {
+                  const uint32_t bal = __ballot_sync(dev::FULL, (xc[g] >> tc) & 1u);
+                  if (lane == i) m[g] = bal;
                 }
               }
-              const uint32_t *col = wst + ((E.tcol & 0x7FFFFFFFu) >> 5);
+            } else {
               const uint32_t sh = E.tcol & 31u;
-              while (am) {  // two arcs a step
-                const uint32_t l0 = __ffs(am) - 1;
-                am &= am - 1;
-                const uint32_t l1 = am ? __ffs(am) - 1 : l0;
-                am &= am - 1;
-                m |= ((col[l0 * P.W] >> sh) & 1u) << l0 | ((col[l1 * P.W] >> sh) & 1u) << l1;
+#pragma unroll
+              for (uint32_t g = 0; g < G; ++g) {
+                const uint32_t nv = nvalid(g);
+                if (nv == 0) break;
+                // the tile's arcs whose target has the pair's target label
+                uint32_t am = 0;
+                if (P.nlabels <= NLC_MAX_LABELS) {
+                  am = larcs[warp][g][E.tlab & (NLC_MAX_LABELS - 1)];
+                } else {  // one ballot per distinct label among them
+                  for (uint32_t rest = nv == 32u ? dev::FULL : (1u << nv) - 1u; rest;) {
+                    const uint32_t ll = __shfl_sync(dev::FULL, xl[g], __ffs(rest) - 1);
+                    const uint32_t bal = __ballot_sync(dev::FULL, xl[g] == ll) & rest;
+                    if (ll == E.tlab) am = bal;
+                    rest &= ~bal;
+                  }
+                }
+                const uint32_t *col = wst + g * 32u * P.W + ((E.tcol & 0x7FFFFFFFu) >> 5);
+                while (am) {  // two arcs a step
+                  const uint32_t l0 = __ffs(am) - 1;
+                  am &= am - 1;
+                  const uint32_t l1 = am ? __ffs(am) - 1 : l0;
+                  am &= am - 1;
+                  m[g] |= ((col[l0 * P.W] >> sh) & 1u) << l0 | ((col[l1 * P.W] >> sh) & 1u) << l1;
+                }
               }
             }
-            if (have) P.mask[maddr] = m;
+#pragma unroll
+            for (uint32_t g = 0; g < G; ++g)
+              if (have && g < nt) P.mask[maddr + g] = m[g];
           } else {
             // records of the pair's tiles that have values, packed to the
             // front; the tile's index in the unit rides in the top byte of
@@ -390,10 +413,19 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   }
 }
 
-// Warps per block of the count pass: each warp stages 32 columns of W words;
-// blocks stay within 96 KB of shared memory so that two fit an SM.
-static uint32_t count_warps(uint32_t W) {
-  const uint64_t per_warp = 32ull * W * 4;
+// Tiles per unit of the count pass.  Four, as in the write pass, let a hub's
+// chain of loads serve four tiles: four plain queries on the scale-22 graph
+// 2.09 -> 0.81 ms, 100 at once 5.4 -> 3.7 ms.  With few hubs the units hold
+// one tile and only the larger kernel shows (mixed sizes on equal degrees 1.01
+// -> 1.12 ms), so there, and for wide columns (the stage grows with both), one.
+uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits) {
+  return nlab == 0 || (W <= 8 && vtiles >= vunits + vunits / 4) ? TAB_WGROUP : 1u;
+}
+
+// Warps per block of the count pass: each warp stages 32 columns of W words
+// per tile; blocks stay within 96 KB of shared memory so that two fit an SM.
+static uint32_t count_warps(uint32_t W, uint32_t G) {
+  const uint64_t per_warp = 32ull * G * W * 4;
   const uint64_t w = (96ull << 10) / per_warp;
   return w > 8 ? 8u : w < 1 ? 1u : (uint32_t)w;
 }
@@ -416,27 +448,24 @@ static uint32_t resident_blocks(const void *fn, int threads, size_t smem, uint64
   return (uint32_t)(b ? b : 1);
 }
 
-void launch_table_vtx(const VPass &P0, bool write, cudaStream_t s) {
-  if (P0.t1 <= P0.t0) return;
-  const VPass &P = P0;
-  const uint32_t warps = write || P.nlab == 0 ? 8u : count_warps(P.W);
-  const uint64_t want = (P.t1 - P.t0 + warps - 1) / warps;
+template <bool WRITE, bool ONE, uint32_t G>
+static void launch_vtx(const VPass &P, uint32_t warps, size_t smem, cudaStream_t s) {
+  const void *fn = (const void *)table_vtx_kernel<WRITE, ONE, G>;
+  if (smem) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const uint32_t blocks = resident_blocks(fn, (int)warps * 32, smem, (P.t1 - P.t0 + warps - 1) / warps);
+  table_vtx_kernel<WRITE, ONE, G><<<blocks, warps * 32, smem, s>>>(P);
+}
+
+void launch_table_vtx(const VPass &P, bool write, cudaStream_t s) {
+  if (P.t1 <= P.t0) return;
   count_launch();
-  if (P.nlab == 0) {
-    if (write) {
-      table_vtx_kernel<true, true><<<resident_blocks((const void *)table_vtx_kernel<true, true>, 256, 0, want), 256, 0, s>>>(P);
-    } else {
-      table_vtx_kernel<false, true><<<resident_blocks((const void *)table_vtx_kernel<false, true>, 256, 0, want), 256, 0, s>>>(P);
-    }
-  } else if (write) {
-    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<true, false>, 256, 0, want);
-    table_vtx_kernel<true, false><<<blocks, 256, 0, s>>>(P);
-  } else {
-    const size_t smem = (size_t)warps * 32 * P.W * 4;
-    cudaFuncSetAttribute(table_vtx_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const uint32_t blocks = resident_blocks((const void *)table_vtx_kernel<false, false>, (int)warps * 32, smem, want);
-    table_vtx_kernel<false, false><<<blocks, warps * 32, smem, s>>>(P);
-  }
+  if (write && P.nlab == 0) return launch_vtx<true, true, TAB_WGROUP>(P, 8, 0, s);
+  if (write) return launch_vtx<true, false, TAB_WGROUP>(P, 8, 0, s);
+  if (P.nlab == 0) return launch_vtx<false, true, TAB_WGROUP>(P, 8, 0, s);
+  const uint32_t G = P.units ? TAB_WGROUP : 1u, warps = count_warps(P.W, G);
+  const size_t smem = (size_t)warps * 32 * G * P.W * 4;
+  if (G > 1) launch_vtx<false, false, TAB_WGROUP>(P, warps, smem, s);
+  else launch_vtx<false, false, 1>(P, warps, smem, s);
 }
 
 __global__ void edge_value_bases_kernel(const TabEdge *__restrict__ edges, uint32_t nedge,

@@ -186,9 +186,9 @@ struct VEdge {
   uint32_t tlab;             // the target row's label
   uint32_t tcol;             // its bit in that label's columns | TAB_KEY_MAP << 31
 };
-// One table pass over units [t0, t1): the count pass's units are vertex
-// tiles (vt: tile -> vertex), the write pass's up to TAB_WGROUP consecutive
-// tiles of one vertex (vg); vtg: the first tile and unit of each vertex.  Arcs
+// One table pass over units [t0, t1): up to TAB_WGROUP consecutive tiles of
+// one vertex (vg: unit -> vertex), or, for a count pass of wide columns
+// (table_count_tiles), single tiles (vt); vtg: the first tile and unit of each vertex.  Arcs
 // are read at nbr[arc - arc_shift], with off the device offsets of the data
 // graph.  cols: the filter's membership columns (W words per vertex), a
 // vertex's sources the bits of its columns & smask, vsrc by row position.
@@ -200,6 +200,7 @@ struct VPass {
   uint64_t arc_shift;
   uint64_t t0, t1;           // t1: a bound of the units when `end` (the last word of vtg) has their number
   const uint64_t *end;
+  uint32_t units;            // [t0, t1) are units of TAB_WGROUP tiles, else tiles
   const uint32_t *vt;
   const uint32_t *vg;
   const uint64_t *vtg;
@@ -223,6 +224,7 @@ void launch_table_vtx(const VPass &P, bool write, cudaStream_t s);
 // Whether the count pass can stage W-word columns (1, 2 or a multiple of 4
 // words, at most 128: 4,096 rows of one label).
 bool table_vtx_fits(uint32_t W);
+uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits);
 // out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys],
 // out[nsrc + 1] = vtg[nv]; zeroes the two counters.
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
