@@ -1273,7 +1273,9 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   ST(aalloc(ctx, scan_tmp_words(nkeys), &d_tmp));
   ST(aalloc(ctx, stb.size() + edge.size() + 1, &d_sizes));
   uint64_t *d_stb = d_sizes, *d_ebase = d_sizes + stb.size();
-  launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), nkeys, d_tiles, ctx->s);
+  uint64_t most_keys = 0;
+  for (const TabSource &x : src) most_keys = std::max<uint64_t>(most_keys, x.nkeys);
+  launch_key_tiles(ctx->g, d_src, (uint32_t)src.size(), most_keys, d_tiles, ctx->s);
   launch_scan(d_tiles, SCAN_U32, nkeys, d_tp, d_tmp, ctx->s);
   // Vertex tiles: the 32-arc tiles of every vertex that some source holds
   // (its membership column under the sources' bits); the table passes walk
@@ -1456,7 +1458,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   } else if (vst != GEM_OK) {
     return vst;
   }
-  launch_table_offsets(d_src, d_edge, (uint32_t)edge.size(), d_tp, d_vp, offs, ctx->s);
+  launch_table_offsets(d_src, d_edge, (uint32_t)edge.size(), d_tp, d_vp, most_keys, ctx->s);
   CU(cudaEventRecord(ctx->ev[10], ctx->s));
   ST(table_pass(true));
   CU(cudaEventRecord(ctx->ev[11], ctx->s));

@@ -137,7 +137,8 @@ void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const
                                                       threshold, nwords, bits, cnt, cols, W);
 }
 
-// One warp per 32 words of a row: their ranks into the rank words, their
+// One warp per 32 words of a row (a row per grid line: a 64-bit division per
+// 32 words to find them cost as much as the rest): their ranks into the rank words, their
 // candidates to the row's list.  ex: exclusive scan of the filter's counts
 // (all rows' sets of TS words in order), which is where a set's candidates
 // start in the lists laid back to back.
@@ -146,11 +147,11 @@ __global__ void __launch_bounds__(256) rank_rows_kernel(const uint32_t *__restri
                                                         uint32_t TS, uint64_t *__restrict__ rb,
                                                         uint32_t *__restrict__ cand) {
   const uint32_t lane = dev::lane_id();
-  const uint32_t G = (nwords + 31) / 32, nsets = (nwords + TS - 1) / TS;
-  const uint64_t items = (uint64_t)nrows * G;
-  for (uint64_t it = blockIdx.x * 8ull + (threadIdx.x >> 5); it < items; it += gridDim.x * 8ull) {
-    const uint32_t r = (uint32_t)(it / G), w0 = (uint32_t)(it % G) * 32, w = w0 + lane;
-    const uint64_t at = __ldg(ex + (uint64_t)r * nsets + w0 / TS), row0 = __ldg(ex + (uint64_t)r * nsets);
+  const uint32_t G = (nwords + 31) / 32, nsets = (nwords + TS - 1) / TS, per = 32 / TS;  // TS: 8 or 32
+  for (uint32_t r = blockIdx.y; r < nrows; r += gridDim.y)
+  for (uint32_t g = blockIdx.x * 8 + (threadIdx.x >> 5); g < G; g += gridDim.x * 8) {
+    const uint32_t w0 = g * 32, w = w0 + lane;
+    const uint64_t at = __ldg(ex + (uint64_t)r * nsets + g * per), row0 = __ldg(ex + (uint64_t)r * nsets);
     const uint64_t i = (uint64_t)r * nwords + w;
     const uint32_t word = w < nwords ? __ldg(bits + i) : 0u, c = __popc(word);
     uint32_t incl = c;
@@ -161,6 +162,11 @@ __global__ void __launch_bounds__(256) rank_rows_kernel(const uint32_t *__restri
     }
     if (w < nwords) rb[i] = ((at - row0 + incl - c) << 32) | word;
     const uint32_t total = __shfl_sync(dev::FULL, incl, 31);
+    if (__reduce_max_sync(dev::FULL, c) <= 4) {  // sparse words: every lane its own
+      uint32_t *to = cand + at + incl - c;
+      for (uint32_t m = word; m; m &= m - 1) *to++ = w * 32u + __ffs(m) - 1;
+      continue;
+    }
     for (uint32_t b = 0; b < total; b += 32) {  // a candidate per lane: the first word whose count passes it
       const uint32_t q = b + lane;
       uint32_t j = 0;
@@ -175,12 +181,14 @@ __global__ void __launch_bounds__(256) rank_rows_kernel(const uint32_t *__restri
 
 void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint32_t TS,
                       uint64_t *rb, uint32_t *cand, cudaStream_t s) {
-  const uint64_t items = (uint64_t)nrows * ((nwords + 31) / 32);
-  if (items == 0) return;
-  uint64_t blocks = (items + 7) / 8;
-  if (blocks > 148ull * 64) blocks = 148ull * 64;
+  const uint32_t G = (nwords + 31) / 32;
+  if (nrows == 0 || G == 0) return;
+  // all of the row's words in flight for a few rows, a few blocks each for many
+  uint32_t bx = (G + 7) / 8, share = 148 * 48 / nrows;
+  if (share < 8) share = 8;
+  if (bx > share) bx = share;
   count_launch();
-  rank_rows_kernel<<<(uint32_t)blocks, 256, 0, s>>>(bits, nrows, nwords, ex, TS, rb, cand);
+  rank_rows_kernel<<<dim3(bx, nrows < 65535 ? nrows : 65535), 256, 0, s>>>(bits, nrows, nwords, ex, TS, rb, cand);
 }
 
 // Compaction of bit rows kept in the low halves of rank words

@@ -156,7 +156,8 @@ struct TabEdge {             // a directed table T(u -> w)
   uint64_t *offsets;         // nkeys + 1 absolute positions into the values array
 };
 // tiles[k] = ceil(deg(key k) / 32) over the flattened key space.
-void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, uint64_t nkeys,
+// (most_keys: the largest source's).
+void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, uint64_t most_keys,
                       uint32_t *tiles, cudaStream_t s);
 // A label of the wave's rows: its rows are the column bits 32 word0 .. of the
 // wave's row positions, `words` column words per vertex of the label.
@@ -236,7 +237,7 @@ void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nk
 void launch_edge_value_bases(const TabEdge *d_edge, uint32_t nedge, const uint64_t *vp, uint64_t tiles,
                              uint64_t *out, cudaStream_t s);
 void launch_table_offsets(const TabSource *d_src, const TabEdge *d_edge, uint32_t nedge,
-                          const uint64_t *tp, const uint64_t *vp, uint64_t total_offsets,
+                          const uint64_t *tp, const uint64_t *vp, uint64_t most_keys,
                           cudaStream_t s);
 constexpr uint32_t TAB_KEY_MAP = 1;
 
