@@ -78,6 +78,7 @@ gem_status Arena::alloc(gem_ctx *ctx, uint64_t bytes, void **out) {
     }
   }
   uint64_t sz = std::max<uint64_t>(bytes, 512ull << 20);
+  if (ctx->device_bytes + sz > ctx->budget && !ctx->keep_live) release_keep(ctx);
   if (ctx->device_bytes + sz > ctx->budget) {
     // chunks this wave has not used (too small for what it asked) go back
     // to the budget before the new one is taken
@@ -155,6 +156,16 @@ static gem_status aalloc(gem_ctx *ctx, uint64_t n, T **out) {
   gem_status s = ctx->arena.alloc(ctx, n * sizeof(T), &p);
   *out = (T *)p;
   return s;
+}
+
+void release_keep(gem_ctx *ctx) {
+  if (ctx->keep_mem) {
+    cudaFree(ctx->keep_mem);
+    ctx->device_bytes -= ctx->keep_bytes;
+  }
+  ctx->keep_mem = nullptr;
+  ctx->keep_bytes = 0;
+  ctx->keep_live = false;
 }
 
 // ---------------------------------------------------------------------------
@@ -280,6 +291,7 @@ static void free_graph(gem_ctx *ctx) {
     ctx->pinned_nbr = nullptr;
   }
   ctx->host_nbr = nullptr;
+  release_keep(ctx);
   if (ctx->part_mem) {
     cudaFree(ctx->part_mem);
     ctx->device_bytes -= ctx->part_bytes;
@@ -338,6 +350,7 @@ extern "C" void gem_ctx_destroy(gem_ctx *ctx) {
   cudaSetDevice(ctx->opts.device);
   cudaStreamSynchronize(ctx->s);
   ctx->arena.release(ctx);
+  release_keep(ctx);
   if (!ctx->borrowed_graph) free_graph(ctx);
   else if (ctx->part_mem) cudaFree(ctx->part_mem);  // a lane's own staging buffers
   if (ctx->ev_ref && !ctx->borrowed_graph) cudaEventDestroy(ctx->ev_ref);
@@ -1324,7 +1337,9 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // read from the mapped adjacency), else read in place.
   const uint32_t nparts = ctx->part_v.empty() ? 0u : (uint32_t)ctx->part_v.size() - 1;
   std::vector<uint64_t> pstart, pstart_w;  // each partition's first tile and first write unit
+  std::vector<uint64_t> keep_at;           // each partition's first word in keep_mem
   bool streamed = false;
+  ctx->keep_live = false;
   if (ctx->opts.ooc && nparts && ctx->opts.ooc_stream != 2 && vtiles) {
     uint64_t *d_pb;
     ST(aalloc(ctx, nparts + 1ull, &d_pb));
@@ -1339,6 +1354,29 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     for (uint32_t p = 0; p < nparts; ++p)
       if (pstart[p + 1] > pstart[p]) need += 4 * (ctx->part_a[p + 1] - ctx->part_a[p]);
     streamed = ctx->opts.ooc_stream == 1 || need <= 2 * 128 * vtiles;
+    // both passes read these partitions: with an ample budget they cross the
+    // host link once (50 four-vertex queries at scale 20: write pass 2.4 -> 1.0
+    // ms, the 125 MB at 55 GB/s of the count pass stay)
+    if (streamed) {
+      const uint64_t room = ctx->budget > ctx->device_bytes ? ctx->budget - ctx->device_bytes : 0;
+      if (ctx->keep_bytes < need && need <= (room + ctx->keep_bytes) / 16) {
+        release_keep(ctx);
+        if (cudaMalloc(&ctx->keep_mem, need) == cudaSuccess) {
+          ctx->keep_bytes = need;
+          ctx->device_bytes += need;
+        } else {
+          cudaGetLastError();
+          ctx->keep_mem = nullptr;
+        }
+      }
+      ctx->keep_live = ctx->keep_bytes >= need;
+      keep_at.assign(nparts, 0);
+      uint64_t at = 0;
+      for (uint32_t p = 0; p < nparts; ++p) {
+        keep_at[p] = at;
+        if (pstart[p + 1] > pstart[p]) at += ctx->part_a[p + 1] - ctx->part_a[p];
+      }
+    }
   }
   if (ctx->opts.ooc) ++(streamed ? ctx->ooc.waves_streamed : ctx->ooc.waves_in_place);
   // One table pass (count or write) over every vertex tile: in place, or
@@ -1385,20 +1423,24 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
       if (pstart[p + 1] == pstart[p]) continue;
       const int b = (int)(k++ & 1u);
       const uint64_t a0 = ctx->part_a[p], bytes = 4 * (ctx->part_a[p + 1] - a0);
-      CU(cudaStreamWaitEvent(ctx->s_copy, ctx->ev_free[b], 0));
-      CU(cudaMemcpyAsync(ctx->d_stage[b], static_cast<const uint32_t *>(ctx->host_nbr) + a0, bytes,
-                         cudaMemcpyHostToDevice, ctx->s_copy));
-      CU(cudaEventRecord(ctx->ev_ready[b], ctx->s_copy));
-      CU(cudaStreamWaitEvent(ctx->s, ctx->ev_ready[b], 0));
-      P.nbr = ctx->d_stage[b];
+      const bool kept = ctx->keep_live;
+      uint32_t *to = kept ? reinterpret_cast<uint32_t *>(ctx->keep_mem) + keep_at[p] : ctx->d_stage[b];
+      if (!kept || !write) {
+        if (!kept) CU(cudaStreamWaitEvent(ctx->s_copy, ctx->ev_free[b], 0));
+        CU(cudaMemcpyAsync(to, static_cast<const uint32_t *>(ctx->host_nbr) + a0, bytes, cudaMemcpyHostToDevice,
+                           ctx->s_copy));
+        CU(cudaEventRecord(ctx->ev_ready[b], ctx->s_copy));
+        CU(cudaStreamWaitEvent(ctx->s, ctx->ev_ready[b], 0));
+        ctx->ooc.parts_streamed += 1;
+        ctx->ooc.bytes_streamed += bytes;
+      }
+      P.nbr = to;
       P.arc_shift = a0;
       P.t0 = units ? pstart_w[p] : pstart[p];
       P.t1 = units ? pstart_w[p + 1] : pstart[p + 1];
       CU(cudaMemsetAsync(P.next, 0, sizeof *P.next, ctx->s));
       launch_table_vtx(P, write, ctx->s);
-      CU(cudaEventRecord(ctx->ev_free[b], ctx->s));
-      ctx->ooc.parts_streamed += 1;
-      ctx->ooc.bytes_streamed += bytes;
+      if (!kept) CU(cudaEventRecord(ctx->ev_free[b], ctx->s));
     }
     return GEM_OK;
   };
@@ -1439,8 +1481,18 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   const uint64_t nv_alloc = nvals ? nvals : 1;
   const bool map_needed = key_map && std::find(w.pair.begin(), w.pair.end(), PAIR_POOL) != w.pair.end();
   gem_status vst = aalloc(ctx, nv_alloc, &w.d_values);
+  if (vst == GEM_ERR_OOM && ctx->keep_live) {  // the values before the partitions: the write pass streams again
+    release_keep(ctx);  // the count pass has completed (its sizes were read back)
+    ctx->err.clear();
+    vst = aalloc(ctx, nv_alloc, &w.d_values);
+  }
   if (vst == GEM_OK && key_map) {
     vst = aalloc(ctx, nv_alloc, &w.d_vkey);
+    if (vst == GEM_ERR_OOM && ctx->keep_live) {
+      release_keep(ctx);
+      ctx->err.clear();
+      vst = aalloc(ctx, nv_alloc, &w.d_vkey);
+    }
     if (vst == GEM_ERR_OOM && !map_needed) {
       ctx->err.clear();
       w.d_vkey = nullptr;
@@ -1461,6 +1513,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   launch_table_offsets(d_src, d_edge, (uint32_t)edge.size(), d_tp, d_vp, most_keys, ctx->s);
   CU(cudaEventRecord(ctx->ev[10], ctx->s));
   ST(table_pass(true));
+  ctx->keep_live = false;  // may be given back from here on (cudaFree waits for the pass)
   CU(cudaEventRecord(ctx->ev[11], ctx->s));
   w.table_passes = true;
   CU(cudaGetLastError());
@@ -1769,6 +1822,7 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
 
 gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_t *emb_dev, uint64_t emb_cap) {
   ctx->h_used = 0;  // the previous wave's copies have completed (it ended with a synchronising readback)
+  ctx->keep_live = false;
   if (!ctx->loaded) {
     ctx->err = "no data graph loaded";
     return GEM_ERR_STATE;

@@ -166,6 +166,12 @@ struct gem_ctx {
   uint32_t *d_stage[2] = {nullptr, nullptr};
   cudaStream_t s_copy = nullptr;
   cudaEvent_t ev_ready[2] = {nullptr, nullptr}, ev_free[2] = {nullptr, nullptr};
+  // out of core: the partitions that a table build's count pass streamed, kept
+  // for its write pass when the budget is ample (kept between waves, given
+  // back when the arena needs the room; live: this wave's write pass reads it)
+  char *keep_mem = nullptr;
+  uint64_t keep_bytes = 0;
+  bool keep_live = false;
   gem_ooc_stats ooc{};
   void *spill_host = nullptr;        // out-of-core: mapped pinned values of tables that exceed the budget
   void *spill_dev = nullptr;
@@ -210,6 +216,8 @@ gem_status lane_create(gem_ctx *root, uint64_t budget, gem_ctx **out);
 void drop_batch_lane(gem_ctx *ctx);
 // Adds a lane's out-of-core counters to its root's and clears them.
 void merge_ooc_stats(gem_ctx *root, gem_ctx *lane);
+
+void release_keep(gem_ctx *ctx);
 
 gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_t *emb_dev, uint64_t emb_cap);
 void wave_result(const gem_ctx *ctx, const Wave &w, size_t qi, gem_result *r);

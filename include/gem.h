@@ -161,15 +161,16 @@ const char *gem_last_error(const gem_ctx *ctx);
  * ooc_part_kib KiB (a vertex whose list is longer gets a partition of its
  * own); a table build either streams the partitions its sources touch into
  * two device staging buffers on a side stream, each copy overlapping the
- * table kernels of the previous partition, or reads the mapped adjacency in
- * place. */
+ * table kernels of the previous partition, or, when the budget is ample, into
+ * a buffer that keeps them for the build's second pass; or reads the mapped
+ * adjacency in place. */
 typedef struct gem_ooc_stats {
   uint32_t partitions;          /* partitions of the loaded graph */
   uint32_t reserved0;
   uint64_t max_part_bytes;      /* largest partition (each staging buffer's size) */
   uint64_t waves_streamed;      /* table builds that streamed partitions */
   uint64_t waves_in_place;      /* table builds that read the mapped adjacency */
-  uint64_t parts_streamed;      /* partition copies issued (two table passes per build) */
+  uint64_t parts_streamed;      /* partition copies issued (one per build, or one per table pass) */
   uint64_t bytes_streamed;      /* bytes those copies moved */
   uint64_t waves_spilled;       /* single-query waves whose edge-table values exceeded the device
                                    budget and were kept in mapped pinned host memory */
