@@ -134,6 +134,17 @@ void Arena::reserve(gem_ctx *ctx, uint64_t bytes) {
   chunks.push_back({p, bytes, 0});
   reserved = true;
 }
+Arena::Mark Arena::mark() const {
+  return cur < chunks.size() ? Mark{chunks[cur].base, chunks[cur].used, in_use} : Mark{nullptr, 0, in_use};
+}
+void Arena::rewind(const Mark &m) {
+  size_t i = 0;
+  while (m.base && i < chunks.size() && chunks[i].base != m.base) ++i;
+  if (i >= chunks.size()) return;  // the marked chunk is gone: keep what was allocated since
+  for (size_t k = i; k < chunks.size(); ++k) chunks[k].used = k == i && m.base ? m.used : 0;
+  cur = i;
+  in_use = m.in_use;
+}
 void Arena::reset() {
   for (auto &c : chunks) c.used = 0;
   cur = 0;
@@ -1042,13 +1053,6 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   Upload up;
   const size_t o_fr = up.add(fr), o_more = up.add(more), o_groups = up.add(groups), o_wl = up.add(wl);
   ST(up.send(ctx));
-  if (!stride && !wl.empty()) {
-    stride = (uint32_t)((wl.size() + 15) / 16) * 16;
-    uint8_t *d_nlc;
-    ST(aalloc(ctx, (uint64_t)ctx->g.nv * stride, &d_nlc));
-    launch_nlc_labels(ctx->g, up.at<uint32_t>(o_wl), (uint32_t)wl.size(), d_nlc, stride, ctx->s);
-    nlc = d_nlc;
-  }
   const uint64_t nbits = (uint64_t)rows * nwords;
   w.d_cols = nullptr;
   if (columns) {
@@ -1066,8 +1070,19 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   ST(aalloc(ctx, nsc + 1, &d_ex));
   ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
+  // the wave's own label counts: read by the filter alone, so what is allocated
+  // next may lie over them (the stream orders both)
+  const Arena::Mark before_counts = ctx->arena.mark();
+  if (!stride && !wl.empty()) {
+    stride = (uint32_t)((wl.size() + 15) / 16) * 16;
+    uint8_t *d_nlc;
+    ST(aalloc(ctx, (uint64_t)ctx->g.nv * stride, &d_nlc));
+    launch_nlc_labels(ctx->g, up.at<uint32_t>(o_wl), (uint32_t)wl.size(), d_nlc, stride, ctx->s);
+    nlc = d_nlc;
+  }
   launch_filter(ctx->g, nlc, stride, up.at<FilterRow>(o_fr), up.at<uint32_t>(o_more), up.at<FilterGroup>(o_groups),
                 (uint32_t)groups.size(), ts, threshold, d_bits, d_cnt, w.d_cols, w.W, nwords, ctx->s);
+  ctx->arena.rewind(before_counts);
   launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
   launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
   std::vector<uint64_t> rs(rows + 1);
@@ -1744,9 +1759,9 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   a.donate_max_level = tu.donate_max_level ? tu.donate_max_level : ctx->donate_max_level;
   a.donate_min_lane = tu.donate_min_lane ? tu.donate_min_lane : 32;
   a.donate_min_desc = tu.donate_min_desc ? tu.donate_min_desc : 1;
-  // pairs are ten to a hundred times as many as roots: a warp may take 32, one
+// pairs are ten to a hundred times as many as roots: a warp may take 32, one
   // per lane to look up (fewer once a quarter of an even share is less)
-  a.root_batch_max = std::min(32u, tu.root_batch_max ? tu.root_batch_max : pair_items ? 32u : 1u);
+  a.root_batch_max = pair_items ? 32u : std::min(32u, tu.root_batch_max ? tu.root_batch_max : 1u);
   a.lane_scan_max = tu.lane_scan_max ? tu.lane_scan_max : 48;
   a.flat_donate_blocks = tu.split_blocks ? tu.split_blocks : 32;
   a.nv = ctx->g.nv;

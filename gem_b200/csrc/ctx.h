@@ -34,6 +34,13 @@ struct Arena {
   // of any size then never call cudaMalloc or cudaFree, whose frees wait for
   // the whole device.  Falls back to growing chunks when it cannot allocate.
   void reserve(gem_ctx *ctx, uint64_t bytes);
+  // rewind(mark()) gives back what was allocated in between.
+  struct Mark {
+    char *base;
+    uint64_t used, in_use;
+  };
+  Mark mark() const;
+  void rewind(const Mark &m);
   void reset();
   void release(gem_ctx *ctx);
 };

@@ -59,10 +59,20 @@ __global__ void __launch_bounds__(256) filter_kernel(const uint32_t *__restrict_
     uint32_t n = 0;
     for (uint32_t t0 = 0; t0 < TS; t0 += nsub) {
       uint32_t m = 0;
-      for (uint32_t j = 0; j < nsub; ++j) {
-        const uint64_t v = ((uint64_t)set * TS + t0 + j) * 32 + lane;
-        const uint32_t b = __ballot_sync(dev::FULL, v < nv && __ldg(lab + v) == g.lab);
+      const uint64_t v0 = ((uint64_t)set * TS + t0) * 32 + lane;
+      for (uint32_t j = 0; nsub < 8 && j < nsub; ++j) {
+        const uint32_t b = __ballot_sync(dev::FULL, v0 + j * 32 < nv && __ldg(lab + v0 + j * 32) == g.lab);
         if (sub == j) m = b;
+      }
+      for (uint32_t j0 = 0; nsub >= 8 && j0 < nsub; j0 += 8) {  // eight tiles' labels in flight (nsub: a power of two)
+        uint32_t l[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) l[j] = v0 + (j0 + j) * 32 < nv ? __ldg(lab + v0 + (j0 + j) * 32) : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+          const uint32_t b = __ballot_sync(dev::FULL, v0 + (j0 + j) * 32 < nv && l[j] == g.lab);
+          if (sub == j0 + j) m = b;
+        }
       }
       const uint64_t vb = ((uint64_t)set * TS + t0 + sub) * 32;
       uint32_t word = 0;

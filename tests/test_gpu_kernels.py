@@ -137,3 +137,23 @@ def test_symmetric_queries(labels, edges):
         r = c.run(q, mode=gem.MODE_HASH)
         assert (r["count"], r["emb_hash"]) == (exp, h)
         assert [r["count"] for r in c.batch([q] * 40)[1]] == [exp] * 40
+
+
+def test_out_of_core_partitions_kept_or_streamed_twice():
+    """With an ample budget the write pass reads the partitions that the count
+    pass streamed; with a tight one both passes stream them.  Same counts."""
+    g = gem.HostGraph.rmat(16, 8, seed=0x47454D10).set_labels(8, 0.0, seed=3)
+    qs = gem.gen_queries(g, 4, gem.ANY, 5, seed=8)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        exp = [c.run(q)["count"] for q in qs]
+    streamed = []
+    for budget in (0, 72 << 20):  # the adjacency is 3.8 MB: more than a sixteenth of what 72 MiB leaves
+        with gem.Context(time_cap_ms=20000, ooc=True, ooc_stream=1, ooc_part_kib=256, budget_bytes=budget) as c:
+            c.load_graph(g)
+            assert [c.run(q)["count"] for q in qs] == exp
+            assert [r["count"] for r in c.batch(qs[:2])[1]] == exp[:2]
+            s = c.ooc_stats()
+            assert s["waves_in_place"] == 0
+            streamed.append(s["bytes_streamed"])
+    assert streamed[1] == 2 * streamed[0]
