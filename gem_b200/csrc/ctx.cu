@@ -2202,12 +2202,12 @@ extern "C" gem_status gem_filter(gem_ctx *ctx, const gem_query *q, uint32_t thre
   ctx->h_used = 0;  // the previous call ended with a synchronisation
   w.share_rows = false;  // rows in query-vertex order, one each
   ST(wave_filter(ctx, w, threshold, false));
-  CU(cudaStreamSynchronize(ctx->s));
   for (uint32_t u = 0; u < q->nv; ++u) counts[u] = w.cnt[u];
-  if (w.cand_total > cand_cap) return GEM_ERR_OVERFLOW;
-  if (w.cand_total && cand_out)
-    CU(cudaMemcpy(cand_out, w.d_cand, w.cand_total * 4, cudaMemcpyDeviceToHost));
-  return GEM_OK;
+  const bool fits = w.cand_total <= cand_cap;
+  if (fits && w.cand_total && cand_out)
+    CU(cudaMemcpyAsync(cand_out, w.d_cand, w.cand_total * 4, cudaMemcpyDeviceToHost, ctx->s));
+  CU(cudaStreamSynchronize(ctx->s));
+  return fits ? GEM_OK : GEM_ERR_OVERFLOW;
 }
 
 extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t u, uint32_t wv,
