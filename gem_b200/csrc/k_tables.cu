@@ -418,11 +418,15 @@ uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t 
   return nlab == 0 || (W <= 8 && vtiles >= vunits + vunits / 4) ? TAB_WGROUP : 1u;
 }
 
+// Dynamic shared memory of a count block, at most (count_warps keeps to it: a
+// warp's stage is 16 KB for the widest columns).
+constexpr uint32_t COUNT_SMEM = 96u << 10;
+
 // Warps per block of the count pass: each warp stages 32 columns of W words
-// per tile; blocks stay within 96 KB of shared memory so that two fit an SM.
+// per tile; blocks stay within COUNT_SMEM so that two fit an SM.
 static uint32_t count_warps(uint32_t W, uint32_t G) {
   const uint64_t per_warp = 32ull * G * W * 4;
-  const uint64_t w = (96ull << 10) / per_warp;
+  const uint64_t w = COUNT_SMEM / per_warp;
   return w > 8 ? 8u : w < 1 ? 1u : (uint32_t)w;
 }
 
@@ -447,7 +451,11 @@ static uint32_t resident_blocks(const void *fn, int threads, size_t smem, uint64
 template <bool WRITE, bool ONE, uint32_t G>
 static void launch_vtx(const VPass &P, uint32_t warps, size_t smem, cudaStream_t s) {
   const void *fn = (const void *)table_vtx_kernel<WRITE, ONE, G>;
-  if (smem) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // A limit above the default (48 KB with the static part) belongs to the
+  // kernel, not to the launch, and lanes launch from threads of their own: always
+  // the most that any wave takes (the wave's own size let one lane lower it
+  // between another lane's two calls, whose launch then failed).
+  if (smem > 32u << 10) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COUNT_SMEM);
   const uint32_t blocks = resident_blocks(fn, (int)warps * 32, smem, (P.t1 - P.t0 + warps - 1) / warps);
   table_vtx_kernel<WRITE, ONE, G><<<blocks, warps * 32, smem, s>>>(P);
 }

@@ -4,6 +4,7 @@ labels than the resident label counts cover, membership columns of every
 width, hash buckets that overflow, pair items and pair pools of odd lengths,
 scans on both sides of the one-block limit."""
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -157,3 +158,30 @@ def test_out_of_core_partitions_kept_or_streamed_twice():
             assert s["waves_in_place"] == 0
             streamed.append(s["bytes_streamed"])
     assert streamed[1] == 2 * streamed[0]
+
+
+def test_lanes_of_different_column_widths():
+    """The count pass of wide columns (44 words: 1,300 filter rows of one label) takes more shared memory than a kernel
+    may by default: that limit is the kernel's, so waves of another width on another thread must leave it."""
+    g = cut(gem.HostGraph.rmat(10, 6, seed=29), 1000).set_labels(51, 0.0, seed=3)
+    stars = [gem.Query([0, i, j], [(0, 1), (0, 2)]) for i in range(51) for j in range(i + 1)][:1300]
+    widths = [stars, stars[:45]]
+    with gem.Context(time_cap_ms=20000) as a, gem.Context(time_cap_ms=20000) as b:
+        exp, bad = [], []
+        for c, qs in zip((a, b), widths):
+            c.load_graph(g)
+            exp.append(c.batch_counts(qs)[1].tolist())
+        assert sum(exp[0]) > 0 and exp[1] == exp[0][:45]
+
+        def lane(i, c):
+            for _ in range(200):
+                st, counts, status = c.batch_counts(widths[i])
+                if st != 0 or status.any() or counts.tolist() != exp[i]:
+                    bad.append((i, st))
+
+        lanes = [threading.Thread(target=lane, args=x) for x in ((0, a), (1, b))]
+        for t in lanes:
+            t.start()
+        for t in lanes:
+            t.join()
+        assert not bad, (len(bad), bad[0])
