@@ -907,6 +907,18 @@ static void *stage(gem_ctx *ctx, size_t bytes) {
   return static_cast<char *>(ctx->h_small) + at;
 }
 
+// Starts a call's use of the staging buffer.  A call ends with a
+// synchronisation and stage_done(); one that failed half way has left copies
+// in flight, which read the buffer or (table sizes) are still to be written to
+// it, so the next call waits for them first.
+static gem_status stage_begin(gem_ctx *ctx) {
+  if (ctx->h_busy) CU(cudaStreamSynchronize(ctx->s));
+  ctx->h_used = 0;
+  ctx->h_busy = true;
+  return GEM_OK;
+}
+static void stage_done(gem_ctx *ctx) { ctx->h_busy = false; }
+
 // Host-to-device copy on the context's stream through pinned staging: the
 // source may be reused as soon as this returns.
 static cudaError_t h2d(gem_ctx *ctx, void *dst, const void *src, size_t bytes) {
@@ -1836,13 +1848,13 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
 }
 
 gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_t *emb_dev, uint64_t emb_cap) {
-  ctx->h_used = 0;  // the previous wave's copies have completed (it ended with a synchronising readback)
-  ctx->keep_live = false;
   if (!ctx->loaded) {
     ctx->err = "no data graph loaded";
     return GEM_ERR_STATE;
   }
   CU(cudaSetDevice(ctx->opts.device));
+  ST(stage_begin(ctx));
+  ctx->keep_live = false;
   const uint64_t launches0 = g_launches.load();
   const size_t nq = w.q.size();
   w.row_of.assign(nq, {});
@@ -1905,6 +1917,7 @@ gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_
   ST(phase_sync("join"));
   CU(cudaEventRecord(ctx->ev[4], ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
+  stage_done(ctx);
   w.filter_ms = ev_ms(ctx->ev[0], ctx->ev[1]);
   w.tables_ms = ev_ms(ctx->ev[1], ctx->ev[2]);
   w.index_ms = ev_ms(ctx->ev[2], ctx->ev[3]);
@@ -2199,7 +2212,7 @@ extern "C" gem_status gem_filter(gem_ctx *ctx, const gem_query *q, uint32_t thre
   w.q.resize(1);
   ST(make_host_query(q, w.q[0], ctx->err));
   ctx->arena.reset();
-  ctx->h_used = 0;  // the previous call ended with a synchronisation
+  ST(stage_begin(ctx));
   w.share_rows = false;  // rows in query-vertex order, one each
   ST(wave_filter(ctx, w, threshold, false));
   for (uint32_t u = 0; u < q->nv; ++u) counts[u] = w.cnt[u];
@@ -2207,6 +2220,7 @@ extern "C" gem_status gem_filter(gem_ctx *ctx, const gem_query *q, uint32_t thre
   if (fits && w.cand_total && cand_out)
     CU(cudaMemcpyAsync(cand_out, w.d_cand, w.cand_total * 4, cudaMemcpyDeviceToHost, ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
+  stage_done(ctx);
   return fits ? GEM_OK : GEM_ERR_OVERFLOW;
 }
 
@@ -2221,7 +2235,7 @@ extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t 
   const HostQuery &hq = w.q[0];
   if (u >= hq.nv || wv >= hq.nv || !(hq.adj[u] & (1u << wv))) return GEM_ERR_ARG;
   ctx->arena.reset();
-  ctx->h_used = 0;  // the previous call ended with a synchronisation
+  ST(stage_begin(ctx));
   w.share_rows = false;  // rows in query-vertex order, one each
   w.active.assign(1, 1);
   ST(wave_filter(ctx, w, 0, true));
@@ -2235,6 +2249,7 @@ extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t 
   w.plan.assign(1, p);
   ST(wave_tables(ctx, w));
   CU(cudaStreamSynchronize(ctx->s));
+  stage_done(ctx);
   const TabEdge &e = w.edges[0];
   const uint64_t nk = w.cnt[u];
   *n_keys = nk;
@@ -2258,7 +2273,7 @@ extern "C" gem_status gem_index_probe(gem_ctx *ctx, const gem_query *q, uint32_t
   ST(make_host_query(q, w.q[0], ctx->err));
   if (u >= w.q[0].nv) return GEM_ERR_ARG;
   ctx->arena.reset();
-  ctx->h_used = 0;  // the previous call ended with a synchronisation
+  ST(stage_begin(ctx));
   w.share_rows = false;  // rows in query-vertex order, one each
   w.active.assign(1, 1);
   w.idx_kind.assign(1, std::vector<uint32_t>(QV, 0));
@@ -2288,6 +2303,7 @@ extern "C" gem_status gem_index_probe(gem_ctx *ctx, const gem_query *q, uint32_t
   CU(cudaGetLastError());
   if (n_keys) CU(cudaMemcpyAsync(pos_out, d_out, 4ull * n_keys, cudaMemcpyDeviceToHost, ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
+  stage_done(ctx);
   return GEM_OK;
 }
 

@@ -195,6 +195,7 @@ struct gem_ctx {
   uint32_t *d_err = nullptr;
   void *h_small = nullptr;           // pinned staging for a wave's small copies (H_SMALL_BYTES)
   size_t h_used = 0;                 // bytes of h_small handed out in the current wave
+  bool h_busy = false;               // a call that has not synchronised since its first copy
   // join schedule: CUDA graph and per-size-bucket tuning (gem_autotune)
   gem::JoinGraph jgraph;
   Tune tune[6];

@@ -189,3 +189,39 @@ def test_lanes_of_different_column_widths():
         for t in lanes:
             t.join()
         assert not bad, (len(bad), bad[0])
+
+
+@pytest.mark.parametrize("kind", ["auto", "cuckoo"])
+def test_calls_after_a_failed_one(kind):
+    """Calls that run out of budget at every phase (budgets in small steps) leave copies in flight; the calls right
+    after them, which use the same staging buffer, are exact."""
+    g = gem.HostGraph.rmat(13, 8, seed=41).set_labels(5, 0.0, seed=2)
+    opts = dict(time_cap_ms=20000, index_kind=gem.IDX_CUCKOO if kind == "cuckoo" else gem.IDX_AUTO)
+    big = gem.gen_queries(g, 20, gem.ANY, 1, seed=3)[0]
+    small = gem.gen_queries(g, 3, gem.ANY, 3, seed=8)
+    with gem.Context(**opts) as c:
+        c.load_graph(g)
+        exp = [(c.run(q)["count"], [x.tolist() for x in c.filter(q)]) for q in small]
+    failed = 0
+    for kib in range(6 << 10, 64 << 10, 32):
+        try:
+            c = gem.Context(budget_bytes=kib << 10, **{**opts, "time_cap_ms": 100})
+            c.load_graph(g)
+        except gem.GemError:
+            continue
+        ran = 0
+        with c:
+            for q, e in zip(small, exp):
+                r = c.run(big, raise_on_error=False)
+                assert r["status"] in ("OK", "ERR_OOM", "ERR_TIMEOUT"), r
+                ran += r["status"] != "ERR_OOM"
+                failed += r["status"] == "ERR_OOM"
+                try:
+                    got = (c.run(q)["count"], [x.tolist() for x in c.filter(q)])
+                except gem.GemError as x:
+                    assert x.status == 2, x
+                    continue
+                assert got == e
+        if ran == len(small):
+            break
+    assert failed > 30
