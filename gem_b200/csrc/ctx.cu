@@ -1260,7 +1260,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   };
   const uint64_t all_tiles = nv + ctx->g.narcs / 32;
   uint64_t tiles = 0, value_cap = 0;
-  bool bounded = !ctx->opts.ooc && !ctx->label_pair_arcs.empty() && w.q.size() <= BOUNDED_QUERIES;
+  bool bounded = !w.frugal && !ctx->opts.ooc && !ctx->label_pair_arcs.empty() && w.q.size() <= BOUNDED_QUERIES;
   if (bounded) {
     for (const TabEdge &e : edge) {
       tiles += tile_bound(e);
@@ -1271,6 +1271,8 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     for (const auto &ch : ctx->arena.chunks) free_bytes += ch.size - ch.used;
     bounded = need <= BOUNDED_BYTES && need <= free_bytes / 4;
   }
+  const bool map_needed = key_map && std::find(w.pair.begin(), w.pair.end(), PAIR_POOL) != w.pair.end();
+  w.optional = bounded || (key_map && !map_needed);
   std::vector<uint32_t> smask(w.pos_words, 0);
   for (uint32_t r : src_row) smask[w.row_pos[r] >> 5] |= 1u << (w.row_pos[r] & 31u);
   uint64_t *d_offs;
@@ -1502,11 +1504,10 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   // single query whose tables do not fit the device budget keeps them in
   // mapped pinned host memory, which the write pass and the join reach over
   // the host link; a batch wave that does not fit is split instead.
-  // Key positions that only spread the ordinary pool's items (pair 2) are left
-  // out when they do not fit.
+  // Key positions that only spread the ordinary pool's items (PAIR_ITEMS) are
+  // left out when they do not fit.
   w.d_vkey = nullptr;
   const uint64_t nv_alloc = nvals ? nvals : 1;
-  const bool map_needed = key_map && std::find(w.pair.begin(), w.pair.end(), PAIR_POOL) != w.pair.end();
   gem_status vst = aalloc(ctx, nv_alloc, &w.d_values);
   if (vst == GEM_ERR_OOM && ctx->keep_live) {  // the values before the partitions: the write pass streams again
     release_keep(ctx);  // the count pass has completed (its sizes were read back)
@@ -1899,22 +1900,36 @@ gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_
       return GEM_ERR_INTERNAL;
     }
   }
-  w.pair.assign(nq, 0);
-  for (size_t qi = 0; qi < nq; ++qi)
-    if (w.active[qi])
-      // (out of core the key positions' memory is better left to the values)
-      w.pair[qi] = pair_pool(ctx, w.plan[qi], mode)                    ? PAIR_POOL
-                   : w.plan[qi].n_enum >= 3 && !ctx->opts.ooc ? PAIR_ITEMS
-                                                                       : 0;
   w.plan_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - h0).count();
-  ST(wave_tables(ctx, w));
-  ST(phase_sync("edge tables"));
-  CU(cudaEventRecord(ctx->ev[2], ctx->s));
-  ST(wave_index(ctx, w));
-  ST(phase_sync("index"));
-  CU(cudaEventRecord(ctx->ev[3], ctx->s));
-  ST(wave_join(ctx, w, mode, emb_dev, emb_cap));
-  ST(phase_sync("join"));
+  auto tables_to_join = [&]() -> gem_status {
+    w.pair.assign(nq, 0);
+    for (size_t qi = 0; qi < nq; ++qi)
+      if (w.active[qi])
+        // (out of core the key positions' memory is better left to the values)
+        w.pair[qi] = pair_pool(ctx, w.plan[qi], mode)                             ? PAIR_POOL
+                     : w.plan[qi].n_enum >= 3 && !ctx->opts.ooc && !w.frugal ? PAIR_ITEMS
+                                                                              : 0;
+    ST(wave_tables(ctx, w));
+    ST(phase_sync("edge tables"));
+    CU(cudaEventRecord(ctx->ev[2], ctx->s));
+    ST(wave_index(ctx, w));
+    ST(phase_sync("index"));
+    CU(cudaEventRecord(ctx->ev[3], ctx->s));
+    ST(wave_join(ctx, w, mode, emb_dev, emb_cap));
+    return phase_sync("join");
+  };
+  // Near the budget the tables' optional memory may leave too little for what
+  // is required after it: the wave then takes only what it must.  (The stream
+  // orders the second build behind the first one's kernels.)
+  const Arena::Mark filtered = ctx->arena.mark();
+  gem_status st = tables_to_join();
+  if (st == GEM_ERR_OOM && w.optional) {
+    ctx->err.clear();
+    ctx->arena.rewind(filtered);
+    w.frugal = true;
+    st = tables_to_join();
+  }
+  ST(st);
   CU(cudaEventRecord(ctx->ev[4], ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
   stage_done(ctx);

@@ -121,6 +121,8 @@ struct Wave {
   float table_pass_ms[2] = {0, 0};  // the table kernels' count and write passes
   float t_begin_ms = 0, t_end_ms = 0;  // first and last event of the wave against the context's ev_ref
   uint64_t arena_bytes = 0;            // arena bytes the wave used
+  bool frugal = false;              // no optional memory: exact table sizes, key positions for the pair pool only
+  bool optional = false;            // the tables asked for some
   bool table_passes = false;        // the passes ran (their events were recorded)
   double plan_ms = 0;
   uint64_t bytes_filter = 0, bytes_tables = 0, bytes_index = 0, bytes_join = 0;

@@ -225,3 +225,25 @@ def test_calls_after_a_failed_one(kind):
         if ran == len(small):
             break
     assert failed > 30
+
+
+@pytest.mark.parametrize("kind", ["auto", "cuckoo"])
+def test_optional_memory_gives_way(kind):
+    """Key positions that only spread the join's items are optional: budgets that hold everything else run the batch
+    in one wave, whether the positions or what is allocated after them would not have fitted."""
+    g = gem.HostGraph.rmat(14, 8, seed=51).set_labels(8, 0.0, seed=2)
+    qs = gem.gen_queries(g, 4, gem.ANY, 12, seed=4)
+    opts = dict(time_cap_ms=20000, index_kind=gem.IDX_CUCKOO if kind == "cuckoo" else gem.IDX_AUTO)
+    with gem.Context(**opts) as c:
+        c.load_graph(g)
+        rs = c.batch(qs, mode=gem.MODE_HASH)[1]
+        exp = [(r["count"], r["emb_hash"]) for r in rs]
+        whole = c.ooc_stats()["resident_bytes"] + rs[0]["arena_bytes"]
+        optional = 4 * rs[0]["table_total"]
+    assert optional > 400_000
+    for less in (0, 256, 4096, 65536, optional // 4, optional // 2, optional - 4096):
+        with gem.Context(budget_bytes=whole - less, **opts) as c:
+            c.load_graph(g)
+            st, rs = c.batch(qs, mode=gem.MODE_HASH)
+            assert st == 0 and len({r["wave"] for r in rs}) == 1, (less, st)
+            assert [(r["count"], r["emb_hash"]) for r in rs] == exp
