@@ -1326,14 +1326,22 @@ __device__ __forceinline__ uint32_t find_query(const uint64_t *__restrict__ rp, 
   return lo;
 }
 
-// Marks query q incomplete and, once, withdraws every unclaimed root so the
-// grid drains quickly; the queries owning withdrawn roots are marked too.
+// Marks the queries [k0, k1) incomplete that have items in the ordinary pool.
+// The others lie in between with no item of it: the lane-parallel pools, which
+// are over by then or mark their own, have counted them whole.
+__device__ void mark_cut(const JoinArgs &a, uint32_t k0, uint32_t k1) {
+  for (uint32_t k = k0; k < k1; ++k)
+    if (a.queries[k].pool) atomicOr(&a.out[k].pad[0], 1ull);
+}
+
+// Marks query q incomplete and, once, withdraws every unclaimed item of the
+// ordinary pool so the grid drains quickly; the queries owning withdrawn items
+// are marked too.
 __device__ void abandon(const JoinArgs &a, uint32_t q) {
   if (q < a.nquery) atomicOr(&a.out[q].pad[0], 1ull);
   const unsigned long long items = __ldg(a.root_prefix + a.nquery);
   const unsigned long long r0 = atomicExch(&a.ctl->root_next, items);
-  if (r0 < items)
-    for (uint32_t k = find_query(a.root_prefix, a.nquery, r0); k < a.nquery; ++k) atomicOr(&a.out[k].pad[0], 1ull);
+  if (r0 < items) mark_cut(a, find_query(a.root_prefix, a.nquery, r0), a.nquery);
 }
 
 // Item r of the ordinary pool: a root of its query, or (JQuery::pairs) an
@@ -1684,7 +1692,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
           if (lane == 0) {
             const uint32_t q0 = find_query(a.root_prefix, a.nquery, rb_cur);
             const uint32_t q1 = find_query(a.root_prefix, a.nquery, rb_end - 1);
-            for (uint32_t k = q0; k <= q1; ++k) atomicOr(&a.out[k].pad[0], 1ull);
+            mark_cut(a, q0, q1 + 1);
             abandon(a, q0);
             if (pushed) __threadfence();
             atomicSub(&ctl->busy, 1u);
@@ -2030,7 +2038,7 @@ __global__ void __launch_bounds__(256, PART == PART_POOLS ? POOL_BLOCKS : PART &
         abandon(a, q);
         if (from_root && rb_cur < rb_end) {
           const uint32_t q1 = find_query(a.root_prefix, a.nquery, rb_end - 1);
-          for (uint32_t k = q; k <= q1; ++k) atomicOr(&a.out[k].pad[0], 1ull);
+          mark_cut(a, q, q1 + 1);
         }
       }
       if (tc) atomicAdd(&a.out[q].count, (unsigned long long)tc << Q->mirror);

@@ -247,3 +247,21 @@ def test_optional_memory_gives_way(kind):
             st, rs = c.batch(qs, mode=gem.MODE_HASH)
             assert st == 0 and len({r["wave"] for r in rs}) == 1, (less, st)
             assert [(r["count"], r["emb_hash"]) for r in rs] == exp
+
+
+def test_pool_counts_survive_the_cap():
+    """The depth-first part runs out of time: queries of the pools, counted whole before it, keep their counts, also
+    the ones that come after its queries in the join's order."""
+    g = gem.HostGraph.rmat(18, 16, seed=61).set_labels(8, 1.0, seed=2)
+    # three vertices of one label next to both ends of an edge: seven subsets, too many for the pair pool
+    slow = gem.Query([0] * 5, [(0, 1)] + [(e, i) for e in (0, 1) for i in (2, 3, 4)])
+    fast = [gem.Query([7, 6, 6, 7], [(0, 1), (1, 2), (2, 3)]),  # two levels like it, and fewer vertices
+            gem.Query([7, 7, 3, 4, 5, 6], [(0, 1), (0, 2), (0, 3), (1, 4), (1, 5)])]  # two levels, and more
+    with gem.Context(time_cap_ms=60000) as c:
+        c.load_graph(g)
+        exp = [c.run(q)["count"] for q in fast]
+    with gem.Context(time_cap_ms=3) as c:
+        c.load_graph(g)
+        rs = c.batch([slow] + fast)[1]
+    assert rs[0]["status"] == "ERR_TIMEOUT"
+    assert [(r["status"], r["count"]) for r in rs[1:]] == [("OK", e) for e in exp]
