@@ -997,73 +997,91 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   }
   const uint32_t rows = (uint32_t)row_sig.size();
   w.nrows = rows;
-  // the label counts the rows need: the graph's own table, or (above
-  // NLC_MAX_LABELS labels) one of the wave's neighbour labels alone
-  const uint8_t *nlc = ctx->g.nlc;
-  uint32_t stride = ctx->g.nlc_stride;
-  std::vector<uint32_t> wl;
-  if (!stride) {
-    for (const auto &sg : row_sig)
-      for (size_t i = 2; i < sg.size(); ++i)
-        if (sg[i] < ctx->g.nlabels) wl.push_back(sg[i]);
-    std::sort(wl.begin(), wl.end());
-    wl.erase(std::unique(wl.begin(), wl.end()), wl.end());
-  }
   // rows in order of their label (a warp tests rows of one label together)
   std::vector<uint32_t> ord(rows);
   for (uint32_t r = 0; r < rows; ++r) ord[r] = r;
   std::stable_sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) { return row_sig[x][0] < row_sig[y][0]; });
-  std::vector<FilterRow> fr(rows);
-  std::vector<uint32_t> more;
-  for (uint32_t k = 0; k < rows; ++k) {
-    const std::vector<uint32_t> &sg = row_sig[ord[k]];
-    FilterRow &f = fr[k];
-    std::memset(&f, 0, sizeof f);
-    f.row = ord[k];
-    if (sg[0] >= ctx->g.nlabels) f.need = UINT32_MAX;  // no vertex has the label
-    f.more = (uint32_t)more.size();
-    uint32_t n = 0;
-    for (size_t i = 2, j; i < sg.size(); i = j) {  // runs of one neighbour label
-      for (j = i; j < sg.size() && sg[j] == sg[i];) ++j;
-      const uint32_t want = (uint32_t)(j - i);
-      if (sg[i] >= ctx->g.nlabels) {
-        if (f.need != UINT32_MAX) f.need += want;
-        continue;
-      }
-      const uint32_t col =
-          stride ? sg[i] : (uint32_t)(std::lower_bound(wl.begin(), wl.end(), sg[i]) - wl.begin());
-      if (n < FILTER_NEEDS) f.needs[n++] = col << 8 | want;
-      else more.push_back(col << 8 | want);
-    }
-    f.n_more = (uint32_t)more.size() - f.more;
-  }
   // groups of up to 32 rows of one label; a label's rows are consecutive bit
   // positions from a multiple of 32 on (waves of at most 32 rows: all rows
-  // share one column word, and no label list is needed to find their bits)
+  // share one column word, and no label list is needed to find their bits).
+  // Without resident label counts a group also ends where its rows' neighbour
+  // labels would be more than the filter counts at once; waves of at most 32
+  // rows have no such group, since each of those labels has a row.
+  const bool resident = ctx->g.nlc_stride != 0, one = rows <= 32;
   std::vector<FilterGroup> groups;
-  const bool one = rows <= 32;
+  std::vector<FilterRow> fr(rows);
+  std::vector<FilterLabel> glabels;
+  std::vector<uint32_t> more;
   w.labels.clear();
   w.row_pos.assign(rows, 0);
   w.row_lab.resize(rows);
   w.pos_words = one ? 1 : 0;
   uint32_t widest = 1;  // column words of a label
-  for (uint32_t k = 0, e; k < rows; k = e) {
+  uint64_t label_bytes = 0;  // of the label counts of the vertices of every label that some row has
+  for (uint32_t k = 0; k < rows;) {
     const uint32_t lab = row_sig[ord[k]][0];
-    for (e = k; e < rows && row_sig[ord[e]][0] == lab; ++e) {
-      w.row_pos[ord[e]] = one ? e : 32 * w.pos_words + (e - k);
-      w.row_lab[ord[e]] = lab;
+    uint32_t words = 0;
+    while (k < rows && row_sig[ord[k]][0] == lab) {
+      FilterGroup g{lab, k, 0, words, one ? k : 0u, (uint32_t)glabels.size(), 0, UINT32_MAX};
+      std::map<uint32_t, uint32_t> most;  // neighbour label -> most neighbours of it wanted
+      for (; k < rows && g.n < 32 && row_sig[ord[k]][0] == lab; ++k, ++g.n) {
+        const std::vector<uint32_t> &sg = row_sig[ord[k]];
+        if (!resident) {
+          uint32_t more_labels = 0;
+          for (size_t i = 2; i < sg.size(); ++i)
+            more_labels += sg[i] < ctx->g.nlabels && (i == 2 || sg[i] != sg[i - 1]) && !most.count(sg[i]);
+          if (g.n && most.size() + more_labels > FILTER_LABELS) break;
+          for (size_t i = 2, j; i < sg.size(); i = j) {
+            for (j = i; j < sg.size() && sg[j] == sg[i];) ++j;
+            if (sg[i] < ctx->g.nlabels) most[sg[i]] = std::max(most[sg[i]], (uint32_t)(j - i));
+          }
+        }
+        g.min_deg = std::min(g.min_deg, sg[1]);
+        w.row_pos[ord[k]] = one ? k : 32 * (w.pos_words + words) + g.n;
+        w.row_lab[ord[k]] = lab;
+      }
+      for (const auto &x : most) glabels.push_back(FilterLabel{x.first, x.second});
+      g.nlab = (uint32_t)most.size();
+      groups.push_back(g);
+      ++words;
     }
-    const uint32_t words = (e - k + 31) / 32;
-    for (uint32_t c = 0; c < words; ++c)
-      groups.push_back(FilterGroup{lab, k + 32 * c, std::min(32u, e - k - 32 * c), c, one ? k : 0u});
     if (one) continue;
+    if (lab < ctx->label_freq.size())
+      label_bytes += resident ? ctx->g.nlc_stride * ctx->label_freq[lab] : 8 * words * ctx->label_arcs[lab];
     widest = std::max(widest, words);
     w.labels.push_back(RowLabel{lab, w.pos_words, words, 0});
     w.pos_words += words;
   }
+  for (const FilterGroup &g : groups)
+    for (uint32_t k = g.row0; k < g.row0 + g.n; ++k) {
+      const std::vector<uint32_t> &sg = row_sig[ord[k]];
+      FilterRow &f = fr[k];
+      std::memset(&f, 0, sizeof f);
+      f.row = ord[k];
+      if (sg[0] >= ctx->g.nlabels) f.need = UINT32_MAX;  // no vertex has the label
+      f.more = (uint32_t)more.size();
+      uint32_t n = 0;
+      for (size_t i = 2, j; i < sg.size(); i = j) {  // runs of one neighbour label
+        for (j = i; j < sg.size() && sg[j] == sg[i];) ++j;
+        const uint32_t want = (uint32_t)(j - i);
+        if (sg[i] >= ctx->g.nlabels) {
+          if (f.need != UINT32_MAX) f.need += want;
+          continue;
+        }
+        uint32_t at = sg[i];
+        if (!resident)
+          at = (uint32_t)(std::lower_bound(glabels.begin() + g.lab0, glabels.begin() + g.lab0 + g.nlab, sg[i],
+                                           [](const FilterLabel &x, uint32_t l) { return x.lab < l; }) -
+                          (glabels.begin() + g.lab0));
+        if (n < FILTER_NEEDS) f.needs[n++] = at << 8 | want;
+        else more.push_back(at << 8 | want);
+      }
+      f.n_more = (uint32_t)more.size() - f.more;
+    }
   w.W = widest <= 2 ? widest : (widest + 3) / 4 * 4;
   Upload up;
-  const size_t o_fr = up.add(fr), o_more = up.add(more), o_groups = up.add(groups), o_wl = up.add(wl);
+  const size_t o_fr = up.add(fr), o_more = up.add(more), o_groups = up.add(groups),
+               o_glabels = up.add(glabels);
   ST(up.send(ctx));
   const uint64_t nbits = (uint64_t)rows * nwords;
   w.d_cols = nullptr;
@@ -1082,19 +1100,9 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   ST(aalloc(ctx, nsc + 1, &d_ex));
   ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
-  // the wave's own label counts: read by the filter alone, so what is allocated
-  // next may lie over them (the stream orders both)
-  const Arena::Mark before_counts = ctx->arena.mark();
-  if (!stride && !wl.empty()) {
-    stride = (uint32_t)((wl.size() + 15) / 16) * 16;
-    uint8_t *d_nlc;
-    ST(aalloc(ctx, (uint64_t)ctx->g.nv * stride, &d_nlc));
-    launch_nlc_labels(ctx->g, up.at<uint32_t>(o_wl), (uint32_t)wl.size(), d_nlc, stride, ctx->s);
-    nlc = d_nlc;
-  }
-  launch_filter(ctx->g, nlc, stride, up.at<FilterRow>(o_fr), up.at<uint32_t>(o_more), up.at<FilterGroup>(o_groups),
-                (uint32_t)groups.size(), ts, threshold, d_bits, d_cnt, w.d_cols, w.W, nwords, ctx->s);
-  ctx->arena.rewind(before_counts);
+  launch_filter(ctx->g, up.at<FilterRow>(o_fr), up.at<uint32_t>(o_more), up.at<FilterGroup>(o_groups),
+                (uint32_t)groups.size(), up.at<FilterLabel>(o_glabels), ts, threshold, d_bits, d_cnt, w.d_cols, w.W,
+                nwords, ctx->s);
   launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
   launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
   std::vector<uint64_t> rs(rows + 1);
@@ -1110,12 +1118,10 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   CU(cudaGetLastError());
   w.cand_total = total;
   // algorithmic bytes: the labels of every vertex, the label counts of the
-  // vertices of every label that some row has, the rows' words (written,
-  // read and rewritten as rank words), the candidate lists
-  uint64_t b = 4ull * ctx->g.nv + 16 * nbits + 4 * total;
-  for (const RowLabel &l : w.labels)
-    if (l.lab < ctx->label_freq.size()) b += (uint64_t)stride * ctx->label_freq[l.lab];
-  w.bytes_filter = b;
+  // vertices of every label that some row has (their lists and the neighbours'
+  // labels where the counts are not resident), the rows' words (written, read
+  // and rewritten as rank words), the candidate lists
+  w.bytes_filter = 4ull * ctx->g.nv + label_bytes + 16 * nbits + 4 * total;
   return GEM_OK;
 }
 

@@ -64,53 +64,6 @@ void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s
   nlc_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.lab, g.nv, g.nlabels, nlc, stride);
 }
 
-// As nlc_kernel for n chosen labels, found by binary search (at most
-// NLC_MAX_LABELS of them per launch, columns c0 .. c0 + n - 1).
-__global__ void __launch_bounds__(256) nlc_labels_kernel(const uint64_t *__restrict__ off,
-                                                         const uint32_t *__restrict__ nbr,
-                                                         const uint32_t *__restrict__ lab, uint32_t nv,
-                                                         const uint32_t *__restrict__ labels, uint32_t n,
-                                                         uint8_t *__restrict__ nlc, uint32_t stride) {
-  __shared__ uint32_t hist[8][NLC_MAX_LABELS];
-  __shared__ uint32_t want[NLC_MAX_LABELS];
-  const uint32_t lane = dev::lane_id(), w = threadIdx.x >> 5;
-  if (threadIdx.x < n) want[threadIdx.x] = labels[threadIdx.x];
-  __syncthreads();
-  const uint64_t nwarps = (uint64_t)gridDim.x * 8;
-  for (uint64_t v = blockIdx.x * 8ull + w; v < nv; v += nwarps) {
-    for (uint32_t l = lane; l < n; l += 32) hist[w][l] = 0;
-    __syncwarp();
-    for (uint64_t i = off[v] + lane, e = off[v + 1]; i < e; i += 32) {
-      const uint32_t l = __ldg(lab + __ldg(nbr + i));
-      uint32_t lo = 0, hi = n;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (want[mid] < l) lo = mid + 1; else hi = mid;
-      }
-      if (lo < n && want[lo] == l) atomicAdd(&hist[w][lo], 1u);
-    }
-    __syncwarp();
-    for (uint32_t l = lane; l < n; l += 32) {
-      const uint32_t c = hist[w][l];
-      nlc[v * stride + l] = (uint8_t)(c > 255u ? 255u : c);
-    }
-    __syncwarp();
-  }
-}
-
-void launch_nlc_labels(const DevGraph &g, const uint32_t *labels, uint32_t n, uint8_t *nlc, uint32_t stride,
-                       cudaStream_t s) {
-  if (g.nv == 0) return;
-  uint64_t blocks = ((uint64_t)g.nv + 7) / 8;
-  if (blocks > 148ull * 64) blocks = 148ull * 64;
-  for (uint32_t c = 0; c < n; c += NLC_MAX_LABELS) {
-    count_launch();
-    nlc_labels_kernel<<<(uint32_t)blocks, 256, 0, s>>>(g.off, g.nbr, g.lab, g.nv, labels + c,
-                                                       n - c < NLC_MAX_LABELS ? n - c : NLC_MAX_LABELS, nlc + c,
-                                                       stride);
-  }
-}
-
 // One warp per vertex inserts its neighbours into the vertex's table; the
 // buckets that some neighbour had to move on from are marked in `moved`.
 __global__ void __launch_bounds__(256) vnh_build_kernel(const uint64_t *__restrict__ off,

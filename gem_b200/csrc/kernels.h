@@ -36,10 +36,6 @@ struct DevGraph {
 // Per-graph derived data, built once at load time.
 void launch_degrees(const DevGraph &g, uint32_t *deg, cudaStream_t s);
 void launch_nlc(const DevGraph &g, uint8_t *nlc, uint32_t stride, cudaStream_t s);
-// Neighbour counts of `n` chosen labels (sorted ascending), stride bytes per
-// vertex: what a wave needs on a graph of more than NLC_MAX_LABELS labels.
-void launch_nlc_labels(const DevGraph &g, const uint32_t *labels, uint32_t n, uint8_t *nlc, uint32_t stride,
-                       cudaStream_t s);
 
 // Neighbourhood hash: per vertex u a table of its neighbours (u32, empty =
 // VNH_EMPTY) in 8-byte buckets of two slots, three buckets for two arcs: u's
@@ -98,8 +94,8 @@ struct FilterDesc {          // one query (gem_filter_static)
 };
 
 // A row of a wave's filter: candidates have the row's label and, over the
-// needs (label-count column << 8 | neighbours wanted, 0 = unused), a deficit
-// of at most the threshold; `need` is the deficit that no vertex can make up
+// needs (count << 8 | neighbours wanted, 0 = unused; count = the label, or its
+// place in the group's list of labels), a deficit of at most the threshold; `need` is the deficit that no vertex can make up
 // (neighbour labels that the graph lacks; above the threshold: no candidates).
 constexpr uint32_t FILTER_NEEDS = 4;
 struct FilterRow {
@@ -115,17 +111,25 @@ struct FilterGroup {
   uint32_t lab;
   uint32_t row0, n;
   uint32_t word, shift;      // the group's column word, and its first bit there
+  // graphs without resident label counts: the rows' neighbour labels (at most
+  // FILTER_LABELS, from entry lab0 of the wave's list), and the fewest
+  // neighbours that one of the rows has
+  uint32_t lab0, nlab, min_deg;
+};
+constexpr uint32_t FILTER_LABELS = 64;
+struct FilterLabel {
+  uint32_t lab, most;        // a neighbour label, and the most neighbours of it that a row wants
 };
 // Vertex tiles per filter item (the granularity of its counts).
 uint32_t filter_set_tiles(uint32_t ngroups, uint32_t nwords);
 // Candidate words of every row, bits[row * nwords + word]; the candidates of
 // every set of TS (8 or 32) words, cnt[row * sets + set]; and (optional) the
 // membership columns, cols[v * W + word], of every vertex with a row's label.
-// nlc: label counts of every vertex, stride bytes each.
-void launch_filter(const DevGraph &g, const uint8_t *nlc, uint32_t stride, const FilterRow *rows,
-                   const uint32_t *more, const FilterGroup *groups, uint32_t ngroups, uint32_t TS, uint32_t threshold,
-                   uint32_t *bits, uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords,
-                   cudaStream_t s);
+// Label counts come from the graph's resident table, or (nlc_stride = 0) are
+// made on the way, for the vertices of the groups' labels; glabels: the groups'.
+void launch_filter(const DevGraph &g, const FilterRow *rows, const uint32_t *more, const FilterGroup *groups,
+                   uint32_t ngroups, const FilterLabel *glabels, uint32_t TS, uint32_t threshold, uint32_t *bits,
+                   uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords, cudaStream_t s);
 // Rank words (members before the word << 32 | the word) and the sorted
 // candidate lists back to back, given ex = exclusive scan of cnt.
 void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint32_t TS,

@@ -96,15 +96,6 @@ static uint64_t estimate_bytes(const gem_ctx *ctx, const HostQuery &q, uint64_t 
     }
     b += most;
   }
-  if (!ctx->g.nlc_stride) {  // the wave's own label counts (at most its neighbour labels)
-    uint32_t n = 0;
-    for (uint32_t u = 0; u < q.nv; ++u) {
-      uint32_t w = 0;
-      while (w < u && q.lab[w] != q.lab[u]) ++w;
-      n += w == u;
-    }
-    b += al((uint64_t)nv * ((n + 15) / 16 * 16)) + al(4 * n);
-  }
   const uint64_t parts = ctx->part_v.empty() ? 0 : ctx->part_v.size();
   *per_wave = 2 * al(4 * nv) + 2 * (al(4 * nv + 4) + al(8 * (nv + 1)) + al(4 * (nv + ctx->g.narcs / 32 + 1))) +
               al(8 * (nv / 2048 + 2)) + al(16 * parts + 16) + (1ull << 20);

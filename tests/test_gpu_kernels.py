@@ -265,3 +265,50 @@ def test_pool_counts_survive_the_cap():
         rs = c.batch([slow] + fast)[1]
     assert rs[0]["status"] == "ERR_TIMEOUT"
     assert [(r["status"], r["count"]) for r in rs[1:]] == [("OK", e) for e in exp]
+
+
+@pytest.mark.parametrize("ooc", [False, True])
+def test_more_labels_than_resident_counts(ooc):
+    """Above 64 labels the filter counts neighbour labels on the way: rows of one label whose neighbours have more
+    labels than a group counts, lists of up to 1,500 arcs read in part or whole, batches against single runs."""
+    g = cut(gem.HostGraph.rmat(13, 16, seed=71), 8000).set_labels(300, 1.0, seed=5)
+    off, nbr, lab = g.arrays()
+    off = off.astype(np.int64)
+    rng = np.random.default_rng(9)
+    centres = np.flatnonzero((lab == 0) & (np.diff(off) > 8))
+    assert np.diff(off)[centres].max() > 1000
+    stars = []
+    for v in rng.choice(centres, 150):
+        leaf = lab[rng.choice(nbr[off[v]:off[v + 1]], rng.integers(2, 6), replace=False)]
+        stars.append(gem.Query([0] + leaf.tolist(), [(0, 1 + i) for i in range(len(leaf))]))
+    hub = centres[np.argmax(np.diff(off)[centres])]
+    wide = gem.Query([0] + lab[rng.choice(nbr[off[hub]:off[hub + 1]], 31, replace=False)].tolist(),
+                     [(0, 1 + i) for i in range(31)])
+    with gem.Context(time_cap_ms=20000, ooc=ooc) as c:
+        c.load_graph(g)
+        for q in stars[:4] + [wide, gem.Query([0, 299, 0, 301], [(0, 1), (1, 2), (2, 3)])]:
+            for t in (0, 1, 3):
+                for a, b in zip(c.filter(q, threshold=t), oracle.filter(g, q, threshold=t)):
+                    assert np.array_equal(a, b), t
+        st, counts, status = c.batch_counts(stars)
+        assert st == 0 and len({tuple(q.labels) for q in stars}) > 100
+        assert counts.tolist() == [c.run(q)["count"] for q in stars]
+        for q, n in list(zip(stars, counts))[:20]:
+            exp, _, ok = oracle.count(g, q, want_hash=False, work_cap=20_000_000)
+            assert not ok or exp == n
+
+
+def test_many_labels_take_no_memory():
+    """A batch on a graph of many labels runs in one wave on the bytes that it holds at its end."""
+    g = gem.HostGraph.rmat(18, 4, 0.25, 0.25, 0.25, seed=73).set_labels(300, 0.0, seed=5)
+    qs = gem.gen_queries(g, 5, gem.ANY, 60, seed=6)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        rs = c.batch(qs)[1]
+        exp = [r["count"] for r in rs]
+        whole = c.ooc_stats()["resident_bytes"] + rs[0]["arena_bytes"]
+    with gem.Context(time_cap_ms=20000, budget_bytes=whole) as c:
+        c.load_graph(g)
+        st, rs = c.batch(qs)
+        assert st == 0 and len({r["wave"] for r in rs}) == 1
+        assert [r["count"] for r in rs] == exp
