@@ -1045,9 +1045,9 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
       groups.push_back(g);
       ++words;
     }
-    if (one) continue;
     if (lab < ctx->label_freq.size())
       label_bytes += resident ? ctx->g.nlc_stride * ctx->label_freq[lab] : 8 * words * ctx->label_arcs[lab];
+    if (one) continue;
     widest = std::max(widest, words);
     w.labels.push_back(RowLabel{lab, w.pos_words, words, 0});
     w.pos_words += words;

@@ -312,3 +312,29 @@ def test_many_labels_take_no_memory():
         st, rs = c.batch(qs)
         assert st == 0 and len({r["wave"] for r in rs}) == 1
         assert [r["count"] for r in rs] == exp
+
+
+# waves of one column word for all rows, and of one per label
+@pytest.mark.parametrize("n", [1, 30])
+def test_filter_bytes(n):
+    """The filter's algorithmic bytes: labels, label counts of the rows' labels (16 a vertex), three passes of words,
+    candidate lists."""
+    g = gem.HostGraph.rmat(10, 6, seed=81).set_labels(7, 0.0, seed=5)
+    qs = gem.gen_queries(g, 5, gem.ANY, n, seed=6)
+
+    def row(q, u):
+        return q.labels[u], tuple(sorted(q.labels[a + b - u] for a, b in q.edges.astype(int).tolist() if u in (a, b)))
+
+    sigs = {row(q, u) for q in qs for u in range(q.nv)}
+    assert (len(sigs) <= 32) == (n == 1)
+    freq = np.bincount(g.arrays()[2], minlength=7)
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        cand = {}
+        for q in qs:
+            for u, x in enumerate(c.filter(q)):
+                cand[row(q, u)] = len(x)
+        got = c.batch(qs)[1][0]["bytes_alg"][0]
+    words = g.nv // 32
+    assert got == (4 * g.nv + 16 * sum(int(freq[x]) for x in {s[0] for s in sigs}) + 16 * words * len(sigs)
+                   + 4 * sum(cand.values()))
