@@ -823,7 +823,6 @@ static float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// Runs the filter for every query of the wave; fills w.rows / counts / lists.
 // Balanced lane-level counting code of a plan (JQuery::flat): the subset
 // values per prefix match (at most FLAT_MAX_VALUES, each an intersection of
 // at most three lists) and those needing a scan, or 0 when not eligible.
@@ -964,7 +963,8 @@ static cudaError_t d2h_sync(gem_ctx *ctx, void *dst, const void *src, size_t byt
   return e;
 }
 
-// columns: also the membership columns the table passes read.
+// Runs the filter for every query of the wave: rows, candidate counts, rank
+// bitmaps and lists; columns: also the membership columns the table passes read.
 static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool columns) {
   const uint32_t nwords = (ctx->g.nv + 31) / 32;
   w.nwords = nwords;
@@ -1778,7 +1778,7 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   a.donate_max_level = tu.donate_max_level ? tu.donate_max_level : ctx->donate_max_level;
   a.donate_min_lane = tu.donate_min_lane ? tu.donate_min_lane : 32;
   a.donate_min_desc = tu.donate_min_desc ? tu.donate_min_desc : 1;
-// pairs are ten to a hundred times as many as roots: a warp may take 32, one
+  // pairs are ten to a hundred times as many as roots: a warp may take 32, one
   // per lane to look up (fewer once a quarter of an even share is less)
   a.root_batch_max = pair_items ? 32u : std::min(32u, tu.root_batch_max ? tu.root_batch_max : 1u);
   a.lane_scan_max = tu.lane_scan_max ? tu.lane_scan_max : 48;
@@ -1854,6 +1854,21 @@ static gem_status wave_join(gem_ctx *ctx, Wave &w, int mode, uint32_t *emb_dev, 
   return GEM_OK;
 }
 
+// Runs `build` (the tables and what follows them).  Near the budget the tables'
+// optional memory may leave too little for what is required after it: the wave
+// then builds once more with only what it must take.  (The stream orders the
+// second build behind the first one's kernels.)
+template <class F>
+static gem_status with_fallback(gem_ctx *ctx, Wave &w, F build) {
+  const Arena::Mark before = ctx->arena.mark();
+  const gem_status st = build();
+  if (st != GEM_ERR_OOM || !w.optional) return st;
+  ctx->err.clear();
+  ctx->arena.rewind(before);
+  w.frugal = true;
+  return build();
+}
+
 gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_t *emb_dev, uint64_t emb_cap) {
   if (!ctx->loaded) {
     ctx->err = "no data graph loaded";
@@ -1924,18 +1939,7 @@ gem_status run_wave(gem_ctx *ctx, Wave &w, uint32_t threshold, int mode, uint32_
     ST(wave_join(ctx, w, mode, emb_dev, emb_cap));
     return phase_sync("join");
   };
-  // Near the budget the tables' optional memory may leave too little for what
-  // is required after it: the wave then takes only what it must.  (The stream
-  // orders the second build behind the first one's kernels.)
-  const Arena::Mark filtered = ctx->arena.mark();
-  gem_status st = tables_to_join();
-  if (st == GEM_ERR_OOM && w.optional) {
-    ctx->err.clear();
-    ctx->arena.rewind(filtered);
-    w.frugal = true;
-    st = tables_to_join();
-  }
-  ST(st);
+  ST(with_fallback(ctx, w, tables_to_join));
   CU(cudaEventRecord(ctx->ev[4], ctx->s));
   CU(cudaStreamSynchronize(ctx->s));
   stage_done(ctx);
@@ -2268,7 +2272,7 @@ extern "C" gem_status gem_edge_table(gem_ctx *ctx, const gem_query *q, uint32_t 
   p.order[1] = wv;
   p.back[1] = {0};
   w.plan.assign(1, p);
-  ST(wave_tables(ctx, w));
+  ST(with_fallback(ctx, w, [&] { return wave_tables(ctx, w); }));
   CU(cudaStreamSynchronize(ctx->s));
   stage_done(ctx);
   const TabEdge &e = w.edges[0];
