@@ -55,6 +55,11 @@ def test_batch_columns(labels, n, k):
         c.load_graph(g)
         rs = c.batch(qs)[1]
         rh = c.batch(qs, mode=gem.MODE_HASH)[1] if labels > 10 else None
+        # every query alone: waves of few rows, whose table passes are another kernel
+        assert [(r["status"], r["count"]) for r in rs] == [("OK", c.run(q)["count"]) for q in qs]
+        if rh is not None:
+            alone = [c.run(q, mode=gem.MODE_HASH) for q in qs]
+            assert [(r["count"], r["emb_hash"]) for r in rh] == [(r["count"], r["emb_hash"]) for r in alone]
         for q, r in list(zip(qs, rs))[:2]:
             cand = oracle.filter(g, q)
             for a, b in q.edges.tolist():
