@@ -324,15 +324,6 @@ void launch_gather_strided(const uint64_t *in, uint64_t stride, uint32_t n, uint
   gather_strided_kernel<<<(n + 255) / 256, 256, 0, s>>>(in, stride, n, out);
 }
 
-__global__ void set_deadline_kernel(unsigned long long *deadline, unsigned long long cap_ns) {
-  *deadline = dev::globaltimer_ns() + cap_ns;
-}
-
-void launch_set_deadline(unsigned long long *deadline, uint64_t cap_ns, cudaStream_t s) {
-  count_launch();
-  set_deadline_kernel<<<1, 1, 0, s>>>(deadline, cap_ns);
-}
-
 uint64_t scan_tmp_words(uint64_t n) { return (n + SCAN_B - 1) / SCAN_B + 2; }
 
 template <ScanInput K>

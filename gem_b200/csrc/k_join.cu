@@ -195,9 +195,11 @@ __device__ __forceinline__ bool vnh_has(const VnhRow &r, uint32_t v) { return vn
 // unconditional and independent (four in flight per lane), with no branch
 // per key, and the rest are followed one by one (eight in flight measured
 // the same).  Random loads bound it: on the scale-22 graph the path
-// [0,0,0,0] (2.26 G keys) takes 22.6 ms, 2.6 TB/s of DRAM.  It took 60.5 ms
-// at 200 instructions per key when every key was probed slot by slot, eight
-// side by side until the longest of the warp's 256 chains had ended.
+// [0,0,0,0] takes 8.5 ms, 2.3 TB/s of DRAM, of which a quarter of each sector
+// is used.  Its 2.26 G tests took 60.5 ms at 200 instructions per key when every
+// key was probed slot by slot, eight side by side until the longest of the
+// warp's 256 chains had ended, and 22.6 ms so; 17.9 in the pools' own kernel,
+// and half of that since one of the path's two mirrored halves is counted.
 __device__ __forceinline__ uint32_t vnh_has8(const VnhRow &r, const uint32_t (&v)[8], uint32_t want) {
   if (!r.nb) return 0;
   uint32_t hit = 0, more = 0;
@@ -286,9 +288,12 @@ __device__ __forceinline__ uint32_t index_of(const JoinArgs &a, const JLevel *__
 // What a counter finds in the warp's shared memory: nothing (the
 // lane-parallel pools, whose prefixes are the lanes' own), the ranges of the
 // lists keyed by the shared prefix, or those and copies of the two longest
-// lists.  Copies serve contexts without a neighbourhood hash only: against
-// the hash, the nine steps of a shared-memory search lose (path [5,1,2,1,5]
-// at scale 22: 491 ms searching copies, 351 ms probing the hash).
+// lists.  Copies serve contexts without a neighbourhood hash only: with the
+// hash, probing it beats the nine steps of a shared-memory search (path
+// [5,1,2,1,5] at scale 22: 491 ms searching copies, 351 ms probing).  No plan
+// was found on which copies win: 110 queries of 5 to 16 vertices, sparse and
+// dense, that ran to the end at scales 12 to 22 take 1/16 to 0.88 of the time
+// that they took with copies and the slot-by-slot hash before.
 enum : int { LC_NONE = 0, LC_RANGES = 1, LC_COPIES = 2 };
 template <int C>
 struct ListCacheT {

@@ -72,8 +72,6 @@ enum ScanInput : uint32_t {
 };
 // out[i] = in[i * stride] for i < n.
 void launch_gather_strided(const uint64_t *in, uint64_t stride, uint32_t n, uint64_t *out, cudaStream_t s);
-// *deadline = device global timer + cap_ns.
-void launch_set_deadline(unsigned long long *deadline, uint64_t cap_ns, cudaStream_t s);
 // tmp needs scan_tmp_words(n) u64 words.
 uint64_t scan_tmp_words(uint64_t n);
 void launch_scan(const void *in, ScanInput kind, uint64_t n, uint64_t *out, uint64_t *tmp,

@@ -293,8 +293,9 @@ gem_status gem_autotune(gem_ctx *ctx, const gem_query *qs, uint32_t n, int mode,
  * persistent grid; donate_max_level is the deepest level that hands work to
  * idle warps; donate_min_lane / donate_min_desc are the smallest halves of a
  * level's unread candidates worth handing over (last enumerated level /
- * other levels); root_batch_max caps the roots a warp takes at once;
- * lane_scan_max is the longest intersection a single lane works through
+ * other levels); root_batch_max (at most 32) caps the roots a warp takes at
+ * once; waves whose items are (root, first level) pairs take up to 32 of
+ * those, a quarter of an even share at most; lane_scan_max is the longest intersection a single lane works through
  * before the whole warp takes it over; split_blocks is the work (in blocks
  * of 8 scanned entries) above which a warp's chunk of last-level matches is
  * split with idle warps. */
