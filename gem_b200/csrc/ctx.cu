@@ -1054,6 +1054,14 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   }
   for (const FilterGroup &g : groups)
     for (uint32_t k = g.row0; k < g.row0 + g.n; ++k) {
+  if (!one && resident) {  // every label of the graph, so that the table passes index the list
+    std::vector<RowLabel> all(ctx->g.nlabels);
+    for (uint32_t l = 0; l < ctx->g.nlabels; ++l) all[l] = RowLabel{l, 0, 0, 0};
+    for (const RowLabel &x : w.labels)
+      if (x.lab < ctx->g.nlabels) all[x.lab] = x;
+      else all.push_back(x);
+    w.labels.swap(all);
+  }
       const std::vector<uint32_t> &sg = row_sig[ord[k]];
       FilterRow &f = fr[k];
       std::memset(&f, 0, sizeof f);
@@ -1078,7 +1086,8 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
       }
       f.n_more = (uint32_t)more.size() - f.more;
     }
-  w.W = widest <= 2 ? widest : (widest + 3) / 4 * 4;
+  w.W = table_col_words(widest);
+  w.WT = 1;
   Upload up;
   const size_t o_fr = up.add(fr), o_more = up.add(more), o_groups = up.add(groups),
                o_glabels = up.add(glabels);
@@ -1160,7 +1169,7 @@ static gem_status spill_buffer(gem_ctx *ctx, uint64_t bytes) {
 // per key its tile count and scan.
 static void wave_table_sizes(Wave &w, uint64_t src_tiles, uint64_t vtiles, uint64_t nvals) {
   w.table_values = nvals;
-  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * w.W) + vtiles * 32ull * 4 * (w.W + 1) + 2 * src_tiles * 16 +
+  w.bytes_tables = 2 * vtiles * (16 + 32ull * 4 + 4ull * w.W) + vtiles * 32ull * 4 * (w.WT + 1) + 2 * src_tiles * 16 +
                    w.table_tiles * (4 + 4 + 8) + nvals * (w.d_vkey ? 8 : 4) + w.n_offs * 8 + w.nkeys * (4 + 8 + 4);
 }
 
@@ -1188,7 +1197,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
           TabSource s;
           s.keys = w.d_cand + w.c_base[r];
           s.nkeys = w.cnt[r];
-          s.pad = 0;
+          s.pos = w.row_pos[r];
           s.key_base = nkeys;
           nkeys += w.cnt[r];
           src.push_back(s);
@@ -1236,11 +1245,13 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     e.flags = flags;
     e.tlab = w.row_lab[tgt];
     e.tcol = w.row_pos[tgt];  // all rows in one column word, else the position within its label
-    if (!w.labels.empty())
+    if (!w.labels.empty()) {
       e.tcol -= 32 * std::lower_bound(w.labels.begin(), w.labels.end(), e.tlab,
                                       [](const RowLabel &x, uint32_t l) { return x.lab < l; })->word0;
     e.tile_base = e.ntiles = 0;  // below
     e.off_base = offs;
+      w.WT = std::max(w.WT, table_col_words(e.tcol / 32 + 1));
+    }
     e.offsets = nullptr;
     offs += (uint64_t)src[rq.s].nkeys + 1;
     if (sedge[2 * rq.s + 1] == 0) sedge[2 * rq.s] = (uint32_t)edge.size();
@@ -1288,7 +1299,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   std::vector<VSrc> vs(32 * (size_t)w.pos_words);
   for (size_t i = 0; i < src.size(); ++i)
     vs[w.row_pos[src_row[i]]] =
-        VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, sedge[2 * i], sedge[2 * i + 1]};
+        VSrc{w.d_rb + (uint64_t)src_row[i] * w.nwords, src[i].key_base, 0, sedge[2 * i], sedge[2 * i + 1]};
   std::vector<VEdge> ve(edge.size());
   // stb: the sources' first tiles (exact sizes only)
   std::vector<uint64_t> stb(src.size() + 2, 0);
@@ -1337,7 +1348,8 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
   ST(aalloc(ctx, 2, &d_next));
   launch_vertex_tiles(ctx->g, d_labels, (uint32_t)w.labels.size(), w.d_cols, w.W, d_smask, d_vtiles, ctx->s);
   launch_scan(d_vtiles, SCAN_TILES, nv, d_vtg, d_tmp3, ctx->s);
-  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_vtg, nv, d_stb, d_next, ctx->s);
+  launch_source_tile_bases(d_src, (uint32_t)src.size(), nkeys, d_tp, d_vtg, nv, d_stb, up.at<VSrc>(o_vs),
+                           d_next, ctx->s);
   uint64_t vtiles = all_tiles, vunits = all_tiles;
   if (!bounded) {
     CU(d2h_sync(ctx, stb.data(), d_stb, 8 * stb.size()));
@@ -1439,6 +1451,7 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.W = w.W;
     P.cols = w.d_cols;
     P.smask = d_smask;
+    P.WT = w.WT;
     P.vsrc = up.at<VSrc>(o_vs);
     P.vedge = ue.at<VEdge>(o_ve);
     P.tp = d_tp;

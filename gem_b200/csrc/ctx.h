@@ -93,7 +93,7 @@ struct Wave {
   // (rows of one label are consecutive positions); unset for vertices whose
   // label no row has.
   uint32_t *d_cols = nullptr;
-  uint32_t W = 1;
+  uint32_t W = 1, WT = 1;
   std::vector<gem::RowLabel> labels;  // the rows' labels, sorted
   std::vector<uint32_t> row_pos;      // position per row
   std::vector<uint32_t> row_lab;      // label per row

@@ -46,23 +46,30 @@ void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, 
 
 __global__ void source_tile_bases_kernel(const TabSource *__restrict__ src, uint32_t nsrc, uint64_t nkeys,
                                          const uint64_t *__restrict__ tp, const uint64_t *__restrict__ vtg,
-                                         uint32_t nv, uint64_t *__restrict__ out,
+                                         uint32_t nv, uint64_t *__restrict__ out, VSrc *__restrict__ vsrc,
                                          unsigned long long *__restrict__ counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 2) counters[i] = 0;
   if (i <= nsrc) out[i] = tp[i < nsrc ? src[i].key_base : nkeys];
+  if (i < nsrc) vsrc[src[i].pos].stb = out[i];
   if (i == nsrc + 1) out[i] = vtg[nv];
 }
 
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
-                              const uint64_t *vtg, uint32_t nv, uint64_t *out, unsigned long long *counters,
-                              cudaStream_t s) {
+                              const uint64_t *vtg, uint32_t nv, uint64_t *out, VSrc *vsrc,
+                              unsigned long long *counters, cudaStream_t s) {
   count_launch();
-  source_tile_bases_kernel<<<(nsrc + 2 + 255) / 256, 256, 0, s>>>(d_src, nsrc, nkeys, tp, vtg, nv, out, counters);
+  source_tile_bases_kernel<<<(nsrc + 2 + 255) / 256, 256, 0, s>>>(d_src, nsrc, nkeys, tp, vtg, nv, out, vsrc, counters);
 }
 
-// The wave's label that v has (binary search), or none (words = 0).
-__device__ __forceinline__ RowLabel find_label(const RowLabel *__restrict__ labels, uint32_t n, uint32_t lab) {
+// The entry of a vertex's label: its own index in a list of all the graph's
+// labels, else found by binary search, or none (words = 0).
+__device__ __forceinline__ RowLabel find_label(const RowLabel *__restrict__ labels, uint32_t n, uint32_t nlabels,
+                                               uint32_t lab) {
+  if (n == nlabels) {
+    const uint4 r = __ldg(reinterpret_cast<const uint4 *>(labels + lab));
+    return RowLabel{r.x, r.y, r.z, 0};
+  }
   uint32_t lo = 0, hi = n;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -79,7 +86,7 @@ __global__ void vertex_tiles_kernel(DevGraph g, const RowLabel *__restrict__ lab
                                     const uint32_t *__restrict__ cols, uint32_t W,
                                     const uint32_t *__restrict__ smask, uint32_t *__restrict__ vtiles) {
   for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.nv; v += (uint64_t)gridDim.x * blockDim.x) {
-    const RowLabel l = nlab ? find_label(labels, nlab, __ldg(g.lab + v)) : RowLabel{0, 0, 1, 0};
+    const RowLabel l = nlab ? find_label(labels, nlab, g.nlabels, __ldg(g.lab + v)) : RowLabel{0, 0, 1, 0};
     uint32_t any = 0;
     for (uint32_t c = 0; c < l.words && !any; ++c) any = __ldg(cols + v * W + c) & __ldg(smask + l.word0 + c);
     vtiles[v] = any ? (__ldg(g.deg + v) + 31u) >> 5 : 0u;
@@ -150,6 +157,11 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
+// The same for one word.
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // The table passes over vertex tiles.  One warp per unit (G tiles of 32 arcs of one
@@ -183,13 +195,19 @@ struct VRec {
 //
 // A unit is a chain of dependent loads (counter, vertex, offsets, arcs,
 // columns, rank word, tile base), which bounds the passes of few rows; the
-// next unit's counter, vertex and offsets are fetched while this one's are
-// used (the count passes of four plain queries on the scale-22 graph: 2.55 ms
-// staged and without the prefetch, 2.10 ms).
+// count pass fetches the next unit's counter, vertex and offsets while this
+// one's are used (the count passes of four plain queries on the scale-22 graph:
+// 2.55 ms staged and without the prefetch, 2.10 ms).  The write pass does not: a
+// unit held ahead by every warp doubles the window of vertices in flight, whose
+// partly written value sectors L2 must then hold (993 rows on 524,288 vertices
+// of 5 labels: 29.4 ms with, 24.2 without).
 //
 // Columns hold a vertex's bits for the rows of its own label only: a few
 // words per vertex where one bit per target row of the wave was 80 words (320
 // bytes staged per arc) for 180 mixed-size queries, count pass 4.2 -> 1.0 ms.
+// The count pass stages them up to the word of the last row that some table
+// targets (WT): rows that only key tables, as the centres of stars do, cost
+// nothing there (720 star centres of one label: staged whole 4.4 ms, 3.8).
 template <bool WRITE, bool ONE, uint32_t G>
 __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   extern __shared__ uint32_t stage[];  // count: 32 columns per tile and warp
@@ -197,6 +215,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   __shared__ uint32_t larcs[WRITE || ONE ? 1 : 8][G][NLC_MAX_LABELS];  // count: a tile's arcs to each label
   const uint32_t lane = dev::lane_id(), warp = threadIdx.x >> 5;
   const uint32_t *vmap = G > 1 ? P.vg : P.vt;
+  constexpr bool AHEAD = !WRITE;
   constexpr uint32_t half = G > 1 ? 32 : 0;  // a vertex's first unit in its word of vtg
   // units are taken in order from one counter, so the units in flight
   // stay a narrow window of consecutive vertices
@@ -209,7 +228,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
   uint64_t a0 = __ldg(P.off + v), a1 = __ldg(P.off + v + 1);
   uint64_t c = (t - (uint32_t)(__ldg(P.vtg + v) >> half)) * G;  // the unit: tiles c .. c + nt - 1 of vertex v
   for (;;) {
-    if (lane == 0) got = atomicAdd(P.next, 1ull);  // the next unit's number, looked at below
+    if (AHEAD && lane == 0) got = atomicAdd(P.next, 1ull);  // the next unit's number, looked at below
     const uint64_t tiles = (a1 - a0 + 31) >> 5;
     const uint32_t nt = tiles - c < G ? (uint32_t)(tiles - c) : G;
     uint32_t xs[G];
@@ -223,15 +242,15 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
     auto nvalid = [&](uint32_t i) -> uint32_t {
       return left <= i * 32u ? 0u : left - i * 32u < 32u ? (uint32_t)(left - i * 32u) : 32u;
     };
-    const RowLabel vl = ONE ? RowLabel{0, 0, 1, 0} : find_label(P.labels, P.nlab, __ldg(P.lab + v));
-    uint32_t *wst = stage + (uint64_t)warp * G * 32u * P.W;
+    const RowLabel vl = ONE ? RowLabel{0, 0, 1, 0} : find_label(P.labels, P.nlab, P.nlabels, __ldg(P.lab + v));
+    uint32_t *wst = stage + (uint64_t)warp * G * 32u * P.WT;
     uint32_t xl[G], xc[G];
     if (!WRITE && ONE) {
 #pragma unroll
       for (uint32_t i = 0; i < G; ++i) xc[i] = lane < nvalid(i) ? __ldg(P.cols + xs[i]) : 0u;
     } else if (!WRITE) {
-      // stage the columns of the tiles' arcs, with asynchronous 16-byte copies
-      // (all in flight at once) when they are whole 16-byte chunks
+      // stage the columns of the tiles' arcs with asynchronous copies, all in
+      // flight at once: of 16 bytes when they are whole 16-byte chunks
 #pragma unroll
       for (uint32_t i = 0; i < G; ++i) xl[i] = lane < nvalid(i) ? __ldg(P.lab + xs[i]) : 0xFFFFFFFFu;
       __syncwarp();  // the previous unit's reads of the stage are done
@@ -239,16 +258,16 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
       for (uint32_t i = 0; i < G; ++i) {
         const uint32_t nv = nvalid(i), x = xs[i];
         if (nv == 0) break;
-        uint32_t *st = wst + i * 32u * P.W;
-        if (P.W >= 4) {
-          const uint32_t ch = P.W >> 2;  // chunks per column
+        uint32_t *st = wst + i * 32u * P.WT;
+        if (P.WT >= 4) {
+          const uint32_t ch = P.WT >> 2;  // chunks per column
           for (uint32_t g = lane; g < ((nv * ch + 31u) & ~31u); g += 32) {
             const uint32_t l = g / ch, q = g - l * ch;
             const uint32_t xa = __shfl_sync(dev::FULL, x, l & 31u);
-            if (l < nv) cp_async16(st + l * P.W + q * 4u, P.cols + (uint64_t)xa * P.W + q * 4u);
+            if (l < nv) cp_async16(st + l * P.WT + q * 4u, P.cols + (uint64_t)xa * P.W + q * 4u);
           }
         } else if (lane < nv) {
-          for (uint32_t q = 0; q < P.W; ++q) st[lane * P.W + q] = __ldg(P.cols + (uint64_t)x * P.W + q);
+          for (uint32_t q = 0; q < P.WT; ++q) cp_async4(st + lane * P.WT + q, P.cols + (uint64_t)x * P.W + q);
         }
         if (P.nlabels <= NLC_MAX_LABELS) {
 #pragma unroll
@@ -261,9 +280,12 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
       cp_async_wait_all();
       __syncwarp();
     }
-    const uint64_t tn = P.t0 + __shfl_sync(dev::FULL, got, 0);
+    uint64_t tn = 0;
     uint32_t vn = 0;
-    if (tn < t1) vn = __ldg(vmap + tn);
+    if (AHEAD) {
+      tn = P.t0 + __shfl_sync(dev::FULL, got, 0);
+      if (tn < t1) vn = __ldg(vmap + tn);
+    }
     const uint32_t *sv = P.cols + (uint64_t)v * P.W;
     for (uint32_t wb = 0; wb < vl.words; wb += 32) {
       const uint32_t word = wb + lane < vl.words ? __ldg(sv + wb + lane) & __ldg(P.smask + vl.word0 + wb + lane) : 0u;
@@ -291,7 +313,7 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
           const VSrc &src = P.vsrc[(vl.word0 + wb + j) * 32u + dev::nth_set_bit(wj, q - exj)];
           const uint64_t rw = __ldg(src.rb + (v >> 5));
           k = (uint32_t)(rw >> 32) + __popc((uint32_t)rw & ((1u << (v & 31u)) - 1u));
-          lt = __ldg(P.tp + src.key_base + k) - __ldg(P.tp + src.key_base) + c;
+          lt = __ldg(P.tp + src.key_base + k) - src.stb + c;
           e0 = src.e0;
           ne = src.ne;
         }
@@ -348,13 +370,13 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
                     rest &= ~bal;
                   }
                 }
-                const uint32_t *col = wst + g * 32u * P.W + ((E.tcol & 0x7FFFFFFFu) >> 5);
+                const uint32_t *col = wst + g * 32u * P.WT + ((E.tcol & 0x7FFFFFFFu) >> 5);
                 while (am) {  // two arcs a step
                   const uint32_t l0 = __ffs(am) - 1;
                   am &= am - 1;
                   const uint32_t l1 = am ? __ffs(am) - 1 : l0;
                   am &= am - 1;
-                  m[g] |= ((col[l0 * P.W] >> sh) & 1u) << l0 | ((col[l1 * P.W] >> sh) & 1u) << l1;
+                  m[g] |= ((col[l0 * P.WT] >> sh) & 1u) << l0 | ((col[l1 * P.WT] >> sh) & 1u) << l1;
                 }
               }
             }
@@ -401,6 +423,11 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
         }
       }
     }
+    if (!AHEAD) {
+      if (lane == 0) got = atomicAdd(P.next, 1ull);
+      tn = P.t0 + __shfl_sync(dev::FULL, got, 0);
+      if (tn < t1) vn = __ldg(vmap + tn);
+    }
     if (tn >= t1) return;
     v = vn;
     a0 = __ldg(P.off + v);
@@ -413,7 +440,11 @@ __global__ void __launch_bounds__(256) table_vtx_kernel(VPass P) {
 // chain of loads serve four tiles: four plain queries on the scale-22 graph
 // 2.09 -> 0.81 ms, 100 at once 5.4 -> 3.7 ms.  With few hubs the units hold
 // one tile and only the larger kernel shows (mixed sizes on equal degrees 1.01
-// -> 1.12 ms), so there, and for wide columns (the stage grows with both), one.
+// -> 1.12 ms), so there one.  For wide columns one too: where a vertex is in
+// hundreds of rows the pairs bound the pass, and more resident warps win (720
+// star centres, W = 24: 3.8 ms, in units of four 4.5), though queries whose rows
+// are targets as well would gain (140 mixed-size queries at scale 22, W = 16: 40.6
+// and 23.4 ms).
 uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits) {
   return nlab == 0 || (W <= 8 && vtiles >= vunits + vunits / 4) ? TAB_WGROUP : 1u;
 }
@@ -422,12 +453,16 @@ uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t 
 // warp's stage is 16 KB for the widest columns).
 constexpr uint32_t COUNT_SMEM = 96u << 10;
 
-// Warps per block of the count pass: each warp stages 32 columns of W words
+// Warps per block of the count pass: each warp stages 32 columns of WT words
 // per tile; blocks stay within COUNT_SMEM so that two fit an SM.
-static uint32_t count_warps(uint32_t W, uint32_t G) {
-  const uint64_t per_warp = 32ull * G * W * 4;
+static uint32_t count_warps(uint32_t WT, uint32_t G) {
+  const uint64_t per_warp = 32ull * G * WT * 4;
   const uint64_t w = COUNT_SMEM / per_warp;
   return w > 8 ? 8u : w < 1 ? 1u : (uint32_t)w;
+}
+
+uint32_t table_col_words(uint32_t words) {
+  return words <= 1 ? 1u : words == 2 ? 2u : (words + 3) / 4 * 4;
 }
 
 bool table_vtx_fits(uint32_t W) { return W == 1 || W == 2 || (W % 4 == 0 && W <= 128); }
@@ -466,8 +501,8 @@ void launch_table_vtx(const VPass &P, bool write, cudaStream_t s) {
   if (write && P.nlab == 0) return launch_vtx<true, true, TAB_WGROUP>(P, 8, 0, s);
   if (write) return launch_vtx<true, false, TAB_WGROUP>(P, 8, 0, s);
   if (P.nlab == 0) return launch_vtx<false, true, TAB_WGROUP>(P, 8, 0, s);
-  const uint32_t G = P.units ? TAB_WGROUP : 1u, warps = count_warps(P.W, G);
-  const size_t smem = (size_t)warps * 32 * G * P.W * 4;
+  const uint32_t G = P.units ? TAB_WGROUP : 1u, warps = count_warps(P.WT, G);
+  const size_t smem = (size_t)warps * 32 * G * P.WT * 4;
   if (G > 1) launch_vtx<false, false, TAB_WGROUP>(P, warps, smem, s);
   else launch_vtx<false, false, 1>(P, warps, smem, s);
 }

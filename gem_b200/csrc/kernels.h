@@ -144,7 +144,7 @@ void launch_compact(uint64_t *rb, const uint64_t *ex, uint32_t nrows, uint32_t n
 struct TabSource {           // a (query, query vertex) whose candidates are table keys
   const uint32_t *keys;      // C(u), sorted
   uint32_t nkeys;
-  uint32_t pad;
+  uint32_t pos;              // its row's position (VSrc index)
   uint64_t key_base;         // first index of this source in the flattened key space
 };
 struct TabEdge {             // a directed table T(u -> w)
@@ -163,11 +163,13 @@ void launch_key_tiles(const DevGraph &g, const TabSource *d_src, uint32_t nsrc, 
                       uint32_t *tiles, cudaStream_t s);
 // A label of the wave's rows: its rows are the column bits 32 word0 .. of the
 // wave's row positions, `words` column words per vertex of the label.
-struct RowLabel {
+// (16 bytes: one load.)  Graphs of up to NLC_MAX_LABELS labels list them all, so
+// that a label is its own index.
+struct __attribute__((aligned(16))) RowLabel {
   uint32_t lab, word0, words, pad;
 };
 // vtiles[v] = ceil(deg(v) / 32) for a vertex that some source holds (columns
-// & source masks), else 0.  labels: the wave's labels, sorted, or none (nlab
+// & source masks), else 0.  labels: sorted, or none (nlab
 // = 0): one column word for all rows, zero for vertices of other labels.
 // smask: bit b of word w = the row at position 32 w + b is a source.
 void launch_vertex_tiles(const DevGraph &g, const RowLabel *labels, uint32_t nlab, const uint32_t *cols, uint32_t W,
@@ -183,6 +185,7 @@ struct VSrc {                // a table source as the vertex-tile passes see it
   const uint64_t *rb;        // rank bitmap row of its candidates
   uint64_t key_base;         // first key in the flattened key space
   uint32_t e0, ne;           // its tables: edges [e0, e0 + ne)
+  uint64_t stb;              // tp[key_base], its first tile (launch_source_tile_bases)
 };
 struct VEdge {
   uint64_t tile_base;
@@ -213,6 +216,7 @@ struct VPass {
   uint32_t nlab;
   uint32_t W;
   const uint32_t *cols;
+  uint32_t WT;               // words per column that the count pass stages: up to the last table target's
   const uint32_t *smask;
   const VSrc *vsrc;
   const VEdge *vedge;
@@ -228,11 +232,13 @@ void launch_table_vtx(const VPass &P, bool write, cudaStream_t s);
 // words, at most 128: 4,096 rows of one label).
 bool table_vtx_fits(uint32_t W);
 uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits);
+// Words per column, rounded up to such a width.
+uint32_t table_col_words(uint32_t words);
 // out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys],
-// out[nsrc + 1] = vtg[nv]; zeroes the two counters.
+// out[nsrc + 1] = vtg[nv]; fills the sources' VSrc::stb; zeroes the two counters.
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
-                              const uint64_t *vtg, uint32_t nv, uint64_t *out, unsigned long long *counters,
-                              cudaStream_t s);
+                              const uint64_t *vtg, uint32_t nv, uint64_t *out, VSrc *vsrc,
+                              unsigned long long *counters, cudaStream_t s);
 // out[e] = vp[edges[e].tile_base] for e < nedge and out[nedge] = vp[tiles]:
 // the first value position of every table (and the total), so that table e
 // holds out[e + 1] - out[e] values.

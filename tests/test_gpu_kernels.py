@@ -343,3 +343,21 @@ def test_filter_bytes(n):
     words = g.nv // 32
     assert got == (4 * g.nv + 16 * sum(int(freq[x]) for x in {s[0] for s in sigs}) + 16 * words * len(sigs)
                    + 4 * sum(cand.values()))
+
+
+# hubs (units of four tiles where columns are narrow) and equal degrees; targets in one, two and more words of columns
+# that are up to 24 words wide for the rows that key tables
+@pytest.mark.parametrize("skew", [True, False])
+@pytest.mark.parametrize("leaf,n", [(6, 60), (6, 240), (12, 700)])
+def test_sources_wider_than_targets(skew, leaf, n):
+    p = (0.57, 0.19, 0.19) if skew else (0.25, 0.25, 0.25)
+    g = gem.HostGraph.rmat(12, 12, *p, seed=91).set_labels(14, 0.5, seed=4)
+    rng = np.random.default_rng(n)
+    qs = [gem.Query([0] + np.sort(rng.integers(1, 1 + leaf, 4)).tolist(), [(0, i) for i in range(1, 5)]) for _ in range(n)]
+    # leaves with leaves of their own: rows of label 1 that tables target, some of them beyond the first words
+    qs += [gem.Query([0, 1, a, b], [(0, 1), (1, 2), (1, 3)]) for a in range(1, leaf) for b in range(a + 1)][:n // 4]
+    with gem.Context(time_cap_ms=20000) as c:
+        c.load_graph(g)
+        st, counts, status = c.batch_counts(qs)
+        assert st == 0 and int(counts.sum()) > 0
+        assert counts.tolist() == [c.run(q)["count"] for q in qs]
