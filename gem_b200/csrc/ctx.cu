@@ -1017,6 +1017,7 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   w.row_lab.resize(rows);
   w.pos_words = one ? 1 : 0;
   uint32_t widest = 1;  // column words of a label
+  uint64_t held = 0;         // vertices of the groups' labels
   uint64_t label_bytes = 0;  // of the label counts of the vertices of every label that some row has
   for (uint32_t k = 0; k < rows;) {
     const uint32_t lab = row_sig[ord[k]][0];
@@ -1045,6 +1046,7 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
       groups.push_back(g);
       ++words;
     }
+    if (lab < ctx->label_freq.size()) held += words * ctx->label_freq[lab];
     if (lab < ctx->label_freq.size())
       label_bytes += resident ? ctx->g.nlc_stride * ctx->label_freq[lab] : 8 * words * ctx->label_arcs[lab];
     if (one) continue;
@@ -1052,8 +1054,6 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
     w.labels.push_back(RowLabel{lab, w.pos_words, words, 0});
     w.pos_words += words;
   }
-  for (const FilterGroup &g : groups)
-    for (uint32_t k = g.row0; k < g.row0 + g.n; ++k) {
   if (!one && resident) {  // every label of the graph, so that the table passes index the list
     std::vector<RowLabel> all(ctx->g.nlabels);
     for (uint32_t l = 0; l < ctx->g.nlabels; ++l) all[l] = RowLabel{l, 0, 0, 0};
@@ -1062,6 +1062,8 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
       else all.push_back(x);
     w.labels.swap(all);
   }
+  for (const FilterGroup &g : groups)
+    for (uint32_t k = g.row0; k < g.row0 + g.n; ++k) {
       const std::vector<uint32_t> &sg = row_sig[ord[k]];
       FilterRow &f = fr[k];
       std::memset(&f, 0, sizeof f);
@@ -1110,7 +1112,7 @@ static gem_status wave_filter(gem_ctx *ctx, Wave &w, uint32_t threshold, bool co
   ST(aalloc(ctx, scan_tmp_words(nsc), &d_tmp));
   ST(aalloc(ctx, rows + 1, &d_rows));
   launch_filter(ctx->g, up.at<FilterRow>(o_fr), up.at<uint32_t>(o_more), up.at<FilterGroup>(o_groups),
-                (uint32_t)groups.size(), up.at<FilterLabel>(o_glabels), ts, threshold, d_bits, d_cnt, w.d_cols, w.W,
+                (uint32_t)groups.size(), up.at<FilterLabel>(o_glabels), held, ts, threshold, d_bits, d_cnt, w.d_cols, w.W,
                 nwords, ctx->s);
   launch_scan(d_cnt, SCAN_U32, nsc, d_ex, d_tmp, ctx->s);
   launch_gather_strided(d_ex, nsets, rows + 1, d_rows, ctx->s);
@@ -1248,10 +1250,10 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     if (!w.labels.empty()) {
       e.tcol -= 32 * std::lower_bound(w.labels.begin(), w.labels.end(), e.tlab,
                                       [](const RowLabel &x, uint32_t l) { return x.lab < l; })->word0;
-    e.tile_base = e.ntiles = 0;  // below
-    e.off_base = offs;
       w.WT = std::max(w.WT, table_col_words(e.tcol / 32 + 1));
     }
+    e.tile_base = e.ntiles = 0;  // below
+    e.off_base = offs;
     e.offsets = nullptr;
     offs += (uint64_t)src[rq.s].nkeys + 1;
     if (sedge[2 * rq.s + 1] == 0) sedge[2 * rq.s] = (uint32_t)edge.size();
@@ -1449,9 +1451,9 @@ static gem_status wave_tables(gem_ctx *ctx, Wave &w) {
     P.nlab = (uint32_t)w.labels.size();
     P.nlabels = ctx->g.nlabels;
     P.W = w.W;
+    P.WT = w.WT;
     P.cols = w.d_cols;
     P.smask = d_smask;
-    P.WT = w.WT;
     P.vsrc = up.at<VSrc>(o_vs);
     P.vedge = ue.at<VEdge>(o_ve);
     P.tp = d_tp;

@@ -124,10 +124,11 @@ uint32_t filter_set_tiles(uint32_t ngroups, uint32_t nwords);
 // every set of TS (8 or 32) words, cnt[row * sets + set]; and (optional) the
 // membership columns, cols[v * W + word], of every vertex with a row's label.
 // Label counts come from the graph's resident table, or (nlc_stride = 0) are
-// made on the way, for the vertices of the groups' labels; glabels: the groups'.
+// made on the way, for the vertices of the groups' labels; glabels: the groups',
+// held: those vertices, summed over the groups.
 void launch_filter(const DevGraph &g, const FilterRow *rows, const uint32_t *more, const FilterGroup *groups,
-                   uint32_t ngroups, const FilterLabel *glabels, uint32_t TS, uint32_t threshold, uint32_t *bits,
-                   uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords, cudaStream_t s);
+                   uint32_t ngroups, const FilterLabel *glabels, uint64_t held, uint32_t TS, uint32_t threshold,
+                   uint32_t *bits, uint32_t *cnt, uint32_t *cols, uint32_t W, uint32_t nwords, cudaStream_t s);
 // Rank words (members before the word << 32 | the word) and the sorted
 // candidate lists back to back, given ex = exclusive scan of cnt.
 void launch_rank_rows(const uint32_t *bits, uint32_t nrows, uint32_t nwords, const uint64_t *ex, uint32_t TS,
@@ -184,8 +185,8 @@ void launch_gather_u64(const uint64_t *a, const uint32_t *idx, uint32_t n, uint6
 struct VSrc {                // a table source as the vertex-tile passes see it
   const uint64_t *rb;        // rank bitmap row of its candidates
   uint64_t key_base;         // first key in the flattened key space
-  uint32_t e0, ne;           // its tables: edges [e0, e0 + ne)
   uint64_t stb;              // tp[key_base], its first tile (launch_source_tile_bases)
+  uint32_t e0, ne;           // its tables: edges [e0, e0 + ne)
 };
 struct VEdge {
   uint64_t tile_base;
@@ -215,8 +216,8 @@ struct VPass {
   uint32_t nlabels;          // the graph's
   uint32_t nlab;
   uint32_t W;
-  const uint32_t *cols;
   uint32_t WT;               // words per column that the count pass stages: up to the last table target's
+  const uint32_t *cols;
   const uint32_t *smask;
   const VSrc *vsrc;
   const VEdge *vedge;
@@ -231,9 +232,9 @@ void launch_table_vtx(const VPass &P, bool write, cudaStream_t s);
 // Whether the count pass can stage W-word columns (1, 2 or a multiple of 4
 // words, at most 128: 4,096 rows of one label).
 bool table_vtx_fits(uint32_t W);
-uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits);
 // Words per column, rounded up to such a width.
 uint32_t table_col_words(uint32_t words);
+uint32_t table_count_tiles(uint32_t W, uint32_t nlab, uint64_t vtiles, uint64_t vunits);
 // out[i] = tp[d_src[i].key_base] for i < nsrc, out[nsrc] = tp[nkeys],
 // out[nsrc + 1] = vtg[nv]; fills the sources' VSrc::stb; zeroes the two counters.
 void launch_source_tile_bases(const TabSource *d_src, uint32_t nsrc, uint64_t nkeys, const uint64_t *tp,
