@@ -403,8 +403,8 @@ def profiled_traffic(kind, workload, batch=None):
     """DRAM bytes (read + write) per algorithmic byte of `kind` ("join" or
     "tables") on `workload`, from the committed ncu capture summary whose
     `workload_key` line is "<kind> <workload>" and which states
-    `dram_per_alg_byte` (the ratio does not depend on the wave's size, so a
-    capture of a smaller wave scales to the bench's launches), or (None, None)."""
+    `dram_per_alg_byte` (of a wave like the bench's: smaller waves have
+    smaller ratios), or (None, None)."""
     import glob
     import re
     key = f"{kind} {workload}"

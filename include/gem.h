@@ -176,7 +176,8 @@ typedef struct gem_ooc_stats {
                                    budget and were kept in mapped pinned host memory */
   uint64_t bytes_spilled;       /* bytes of those values (and key positions) */
   uint64_t resident_bytes;      /* device bytes the context holds outside its wave scratch (graph,
-                                   partitions, join queue), counted against its device budget */
+                                   staging, partitions kept for a build's second pass, join
+                                   queue), counted against its device budget */
 } gem_ooc_stats;
 /* GEM_ERR_STATE while the context serves (gem_submit): its waves update the counters. */
 gem_status gem_ctx_ooc_stats(const gem_ctx *ctx, gem_ooc_stats *out);
